@@ -12,6 +12,7 @@
 #include <thrust/iterator/counting_iterator.h>
 
 #include "scene.h"
+#include "wide.cuh"
 
 namespace xyzgpu {
 
@@ -87,7 +88,7 @@ void free_scene(SceneImpl *s) {
   cudaDeviceSynchronize();
   render_workspace_free(s->ws);
   void *bufs[] = {s->d_tri, s->d_ng, s->d_sn, s->d_mat, s->d_shininess, s->d_emission, s->d_lights, s->d_cdf, s->d_spd,
-                  s->d_nodes, s->d_refs, s->d_fetch, s->d_trace_counts};
+                  s->d_nodes, s->d_refs, s->d_wide, s->d_wide_tri, s->d_fetch, s->d_trace_counts};
   for (void *b : bufs)
     if (b) cudaFreeAsync(b, nullptr);
   cudaStreamSynchronize(nullptr);
@@ -570,6 +571,7 @@ int xyzgpu_scene_create(const xyzgpu_scene_desc *d, const xyzgpu_build_params *b
     return set_error(XYZGPU_E_INVALID, "scene_create: unknown builder %d", bp.builder);
   }
   s->build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+  if (s->d_wide) bytes += s->n_wide * kWideWords * 4 + static_cast<int64_t>(nt) * kWideTriVec * 16;
   s->device_bytes = bytes;
 
   DevScene &v = s->dev;
@@ -587,6 +589,8 @@ int xyzgpu_scene_create(const xyzgpu_scene_desc *d, const xyzgpu_build_params *b
   v.cdf = s->d_cdf;
   v.nodes = s->d_nodes;
   v.refs = s->d_refs;
+  v.wide = s->d_wide;
+  v.wide_tri = s->d_wide_tri;
   // Lights of zero total area cannot be sampled: next-event estimation is off
   // (the reference would divide by that area, xyz/core/scene.cpp:65).
   v.n_lights = cdf.back() > 0.0f ? s->n_lights : 0;

@@ -42,6 +42,7 @@ XYZ_DEV f3 normalize3(f3 a) {
   float const r = 1.0f / sqrtf(dot3(a, a));
   return scl3(a, r);
 }
+XYZ_HD float norm1(f3 a) { return fabsf(a.x) + fabsf(a.y) + fabsf(a.z); }
 XYZ_HD f3 xyz3(float4 v) { return f3{v.x, v.y, v.z}; }
 
 // ---------------------------------------------------------------- random
@@ -117,6 +118,9 @@ struct DevScene {
   const float *cdf;       // n_lights + 1 prefix sums of light areas, cdf[0] = 0
   const uint2 *nodes;
   const int32_t *refs;
+  const uint32_t *wide;     // wide tree (wide.cuh) and its triangle records, or null
+  const float4 *wide_tri;
+  float wide_reach;         // largest origin coordinate of the rays it serves
   int n_lights;
   float light_area;
   f3 power;

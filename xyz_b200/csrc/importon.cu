@@ -142,12 +142,12 @@ __global__ void k_particles_start(DevScene S, int particles, uint64_t seed, Part
   if (blockIdx.x == 0 && threadIdx.x == 0) *count = particles;
 }
 
-__global__ void __launch_bounds__(kThreads, 10)
+__global__ void __launch_bounds__(kThreads, 8)
     k_particles_trace(DevScene S, const float4 *qo, const float4 *qd, float4 *hits, const int32_t *count,
                       int32_t *fetch) {
   ExtSink<false> sink{qo, qd, hits, nullptr};
-  TraceCount tc{};
-  trace_persistent<false>(S, *count, fetch, sink, tc);
+  __shared__ WideList s_list;
+  trace_closest_hits(S, *count, fetch, sink, s_list);
 }
 
 // One bounce of every live particle: the importon of a Lambert hit from bounce

@@ -29,10 +29,16 @@
 // same 32-byte sector, and rays working in one region of space read one
 // region of the array.  Node words keep their format; only child indices
 // change.
+//
+// The same two sweeps over the levels give the wide tree (wide.cuh) its
+// triangle sets: boxes and counts of the kd nodes from the deepest level up,
+// positions in depth-first order from the root down; k_wide_nodes then builds
+// the wide nodes level by level and k_wide_tris writes the triangle records.
 #include <algorithm>
 #include <vector>
 
 #include "scene.h"
+#include "wide.cuh"
 
 namespace xyzgpu {
 namespace {
@@ -777,41 +783,81 @@ int grid_for(int64_t work, int threads, int device) {
 }
 
 // ---- depth-first layout
-// Descendant counts of the nodes [begin, end) of one level (their children
-// lie in deeper levels, counted before).
-__global__ void k_layout_desc(const uint2 *__restrict__ nodes, int64_t begin, int64_t end, int32_t *desc) {
-  for (int64_t i = begin + blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < end;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    uint2 const nd = nodes[i];
-    if ((nd.y & 3u) == kKdLeafTag) {
-      desc[i] = 0;
-    } else {
-      uint32_t const c = nd.y >> 2;
-      desc[i] = 2 + desc[c] + desc[c + 1];
-    }
+// Descendant count of node i (its children lie in deeper levels, counted
+// before) and, with sets, the box and triangle count of what lies below it.
+XYZ_DEV void layout_up(const uint2 *__restrict__ nodes, int64_t i, int32_t *desc, const WideSets &T) {
+  uint2 const nd = nodes[i];
+  if ((nd.y & 3u) == kKdLeafTag) {
+    desc[i] = 0;
+    return;
+  }
+  uint32_t const c = nd.y >> 2;
+  desc[i] = 2 + desc[c] + desc[c + 1];
+  if (T.lo) {
+    uint4 const a = T.lo[c], b = T.lo[c + 1], p = T.hi[c], q = T.hi[c + 1];
+    T.lo[i] = make_uint4(min(a.x, b.x), min(a.y, b.y), min(a.z, b.z), 0u);
+    T.hi[i] = make_uint4(max(p.x, q.x), max(p.y, q.y), max(p.z, q.z), p.w + q.w);
   }
 }
 
-__global__ void k_layout_root(int32_t *pos, int32_t *base) {
-  pos[0] = 0;
-  base[0] = 1;
+// New positions of node i's children: the pair at base(parent); the first
+// child's descendants from base + 2, the second's after them.  With sets, the
+// positions of their triangles: the first child's, then the second's.
+XYZ_DEV void layout_down(const uint2 *__restrict__ nodes, int64_t i, const int32_t *__restrict__ desc, int32_t *pos,
+                         int32_t *base, const WideSets &T) {
+  uint2 const nd = nodes[i];
+  if ((nd.y & 3u) == kKdLeafTag) return;
+  uint32_t const c = nd.y >> 2;
+  int32_t const b = base[i];
+  pos[c] = b;
+  pos[c + 1] = b + 1;
+  base[c] = b + 2;
+  base[c + 1] = b + 2 + desc[c];
+  if (T.lo) {
+    int32_t const f = T.first[i];
+    T.first[c] = f;
+    T.first[c + 1] = f + static_cast<int32_t>(T.hi[c].w);
+  }
 }
 
-// New positions of the children of the nodes [begin, end): the pair at
-// base(parent); the first child's descendants from base + 2, the second's
-// after them.
-__global__ void k_layout_place(const uint2 *__restrict__ nodes, int64_t begin, int64_t end,
-                               const int32_t *__restrict__ desc, int32_t *pos, int32_t *base) {
+__global__ void k_layout_desc(const uint2 *__restrict__ nodes, int64_t begin, int64_t end, int32_t *desc, WideSets T) {
   for (int64_t i = begin + blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < end;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    uint2 const nd = nodes[i];
-    if ((nd.y & 3u) == kKdLeafTag) continue;
-    uint32_t const c = nd.y >> 2;
-    int32_t const b = base[i];
-    pos[c] = b;
-    pos[c + 1] = b + 1;
-    base[c] = b + 2;
-    base[c + 1] = b + 2 + desc[c];
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    layout_up(nodes, i, desc, T);
+}
+
+__global__ void k_layout_place(const uint2 *__restrict__ nodes, int64_t begin, int64_t end,
+                               const int32_t *__restrict__ desc, int32_t *pos, int32_t *base, WideSets T) {
+  for (int64_t i = begin + blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < end;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    layout_down(nodes, i, desc, pos, base, T);
+}
+
+// Both sweeps of the top levels in one CTA: a level of at most kTopNodes nodes
+// takes one CTA no longer than a launch of its own takes.
+constexpr int kTopLevels = 16;
+constexpr int64_t kTopNodes = 2048;
+struct TopLevels {
+  int64_t start[kTopLevels + 1];
+  int n;
+};
+
+__global__ void __launch_bounds__(1024)
+    k_layout_top(const uint2 *__restrict__ nodes, TopLevels V, int32_t *desc, int32_t *pos, int32_t *base, WideSets T) {
+  for (int l = V.n - 1; l >= 0; --l) {
+    for (int64_t i = V.start[l] + threadIdx.x; i < V.start[l + 1]; i += blockDim.x) layout_up(nodes, i, desc, T);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    pos[0] = 0;
+    base[0] = 1;
+    if (T.lo) T.first[0] = 0;
+  }
+  __syncthreads();
+  for (int l = 0; l < V.n; ++l) {
+    for (int64_t i = V.start[l] + threadIdx.x; i < V.start[l + 1]; i += blockDim.x)
+      layout_down(nodes, i, desc, pos, base, T);
+    __syncthreads();
   }
 }
 
@@ -822,6 +868,82 @@ __global__ void k_layout_scatter(const uint2 *__restrict__ nodes, int64_t n, con
     uint2 nd = nodes[i];
     if ((nd.y & 3u) != kKdLeafTag) nd.y = (static_cast<uint32_t>(base[i]) << 2) | (nd.y & 3u);
     out[pos[i]] = nd;
+  }
+}
+
+
+// ---- wide tree
+// Each triangle joins the kd leaf that holds its centroid: the leaf's box and
+// count take it in.
+__global__ void k_wide_assign(const float4 *__restrict__ tri, int n, const uint2 *__restrict__ nodes, WideSets T,
+                              int32_t *__restrict__ owner) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    float4 const a = tri[3 * i], b = tri[3 * i + 1], c = tri[3 * i + 2];
+    // vertices as the intersection test sees them: v0, v0 + e1, v0 + e2
+    f3 const v0 = xyz3(a), v1 = add3(v0, xyz3(b)), v2 = add3(v0, xyz3(c));
+    int32_t const leaf = wide_leaf_of(nodes, scl3(add3(add3(v0, v1), v2), 1.0f / 3.0f));
+    owner[i] = leaf;
+    uint32_t *const lo = reinterpret_cast<uint32_t *>(T.lo + leaf);
+    uint32_t *const hi = reinterpret_cast<uint32_t *>(T.hi + leaf);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      float const x = comp3(v0, k), y = comp3(v1, k), z = comp3(v2, k);
+      atomicMin(lo + k, float_key(fminf(fminf(x, y), z)));
+      atomicMax(hi + k, float_key(fmaxf(fmaxf(x, y), z)));
+    }
+    atomicAdd(hi + 3, 1u);
+  }
+}
+
+// State of the level-by-level construction: nodes and records handed out, the
+// node range [level[l], level[l + 1]) of every level, and per level the CTAs
+// that have finished (the last one closes the next level's range).
+struct WideCounters {
+  uint32_t nodes, tris;
+  uint32_t level[kWideStack + 3];
+  uint32_t done[kWideStack + 1];
+};
+
+constexpr int kWideThreads = 64;
+
+__global__ void __launch_bounds__(kWideThreads)
+    k_wide_nodes(const uint2 *__restrict__ kd, WideSets T, float pad, int l, WideCounters *C, WideTask *task,
+                 uint32_t max_nodes, uint32_t *__restrict__ out, int32_t *__restrict__ dst) {
+  uint32_t const b = C->level[l], e = C->level[l + 1];
+  for (uint32_t i = b + blockIdx.x * blockDim.x + threadIdx.x; i < e; i += gridDim.x * blockDim.x) {
+    uint32_t w[kWideWords];
+    wide_make_node(
+        kd, T, task[i], pad, w, [&](int k) { return atomicAdd(&C->nodes, static_cast<uint32_t>(k)); },
+        [&](int k) { return atomicAdd(&C->tris, static_cast<uint32_t>(k)); },
+        [&](uint32_t at, WideTask t) {
+          if (at < max_nodes) task[at] = t;
+        },
+        [&](int32_t at, uint32_t rec) { dst[at] = static_cast<int32_t>(rec); });
+    uint4 *const o = reinterpret_cast<uint4 *>(out + static_cast<size_t>(i) * kWideWords);
+#pragma unroll
+    for (int q = 0; q < kWideWords / 4; ++q) o[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&C->done[l], 1u) == gridDim.x - 1) C->level[l + 2] = min(atomicAdd(&C->nodes, 0u), max_nodes);
+  }
+}
+
+// Triangle records in the order the nodes name them (within a kd leaf of
+// several triangles in arrival order: the closest hit does not depend on it).
+__global__ void k_wide_tris(const float4 *__restrict__ tri, int n, WideSets T, const int32_t *__restrict__ owner,
+                            const int32_t *__restrict__ dst, float4 *__restrict__ out) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    int32_t const leaf = owner[i];
+    // w counts up from the 0xffffffff it was filled with
+    uint32_t const k = atomicAdd(reinterpret_cast<uint32_t *>(T.lo + leaf) + 3, 1u) + 1u;
+    size_t const rec = static_cast<size_t>(dst[T.first[leaf] + static_cast<int32_t>(k)]) * kWideTriVec;
+    float4 const a = tri[3 * i], b = tri[3 * i + 1], c = tri[3 * i + 2];
+    out[rec] = a;
+    out[rec + 1] = b;
+    out[rec + 2] = c;
+    out[rec + 3] = make_float4(__int_as_float(i), norm1(xyz3(b)) + norm1(xyz3(c)), norm1(mk3(a.w, b.w, c.w)), 0.0f);
   }
 }
 
@@ -984,12 +1106,73 @@ int kd_build_device(SceneImpl &s, const float4 *d_tri, int n, const BuildConfig 
   return kd_layout_depth_first(s, level_start, st);
 }
 
+namespace {
+
+// Nodes a wide tree over n triangles may need: a node either has eight
+// children or only leaf children and then at least four triangles, so there
+// are at most n / 4 of the second kind and (n + n / 4) / 7 of the first.
+int64_t wide_max_nodes(int64_t n) { return n / 4 + (n + n / 4) / 7 + 64; }
+
+struct WideBufs {
+  DevBuf<uint4> lo, hi;
+  DevBuf<int32_t> first, owner, dst;
+  DevBuf<uint32_t> nodes;
+  DevBuf<WideTask> task;
+  DevBuf<WideCounters> counters;
+  DevBuf<float4> tris;
+};
+
+// Fills the wide tree from the sets of the breadth-first kd nodes.  A tree
+// deeper than the traversal's stack is dropped (the kd-tree serves alone).
+int wide_build(SceneImpl &s, WideBufs &B, const WideSets &T, float pad, cudaStream_t st) {
+  int const dev = s.device, n = s.n_tris;
+  uint32_t const max_nodes = static_cast<uint32_t>(wide_max_nodes(n));
+  WideCounters h{};
+  h.nodes = 1;
+  h.level[1] = 1;
+  WideTask const root{0, 0, n};
+  XYZ_BUILD_TRY(cudaMemcpyAsync(B.counters.p, &h, sizeof(h), cudaMemcpyHostToDevice, st));
+  XYZ_BUILD_TRY(cudaMemcpyAsync(B.task.p, &root, sizeof(root), cudaMemcpyHostToDevice, st));
+  int const grid = grid_for(n / 8 + 1, kWideThreads, dev);
+  int done = 0;
+  bool more = true;
+  // about log8(n) levels, a few more where the tree is uneven: their launches
+  // are issued ahead and the host looks at the ranges after each group
+  for (int group = n > 4096 ? 10 : 4; more && done < kWideStack; group = 4) {
+    int const upto = std::min(kWideStack, done + group);
+    for (; done < upto; ++done)
+      k_wide_nodes<<<grid, kWideThreads, 0, st>>>(s.d_nodes, T, pad, done, B.counters.p, B.task.p, max_nodes,
+                                                  B.nodes.p, B.dst.p);
+    XYZ_BUILD_TRY(cudaGetLastError());
+    XYZ_BUILD_TRY(cudaMemcpyAsync(&h, B.counters.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+    XYZ_BUILD_TRY(cudaStreamSynchronize(st));
+    more = h.level[done] < h.level[done + 1];
+  }
+  if (more || h.nodes > max_nodes || h.tris != static_cast<uint32_t>(n)) return XYZGPU_OK;
+  k_wide_tris<<<grid_for(n, 256, dev), 256, 0, st>>>(s.d_tri, n, T, B.owner.p, B.dst.p, B.tris.p);
+  XYZ_BUILD_TRY(cudaGetLastError());
+  DevBuf<uint32_t> out;
+  out.st = st;
+  size_t const words = static_cast<size_t>(h.nodes) * kWideWords;
+  if (out.reserve(static_cast<int64_t>(words)) != cudaSuccess) {
+    cudaGetLastError();
+    return XYZGPU_OK;
+  }
+  XYZ_BUILD_TRY(cudaMemcpyAsync(out.p, B.nodes.p, words * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
+  s.n_wide = h.nodes;
+  s.d_wide = out.release();
+  s.d_wide_tri = B.tris.release();
+  return XYZGPU_OK;
+}
+
+}  // namespace
+
 int kd_layout_depth_first(SceneImpl &s, const std::vector<int64_t> &level_start, cudaStream_t st) {
   int64_t const n = s.n_nodes;
-  if (n <= 1) return XYZGPU_OK;
+  if (n < 1 || s.n_tris < 1) return XYZGPU_OK;
   if (level_start.size() < 2 || level_start.front() != 0 || level_start.back() != n)
     return set_error(XYZGPU_E_INVALID, "kd-tree layout: level ranges do not cover the nodes");
-  int const dev = s.device;
+  int const dev = s.device, nt = s.n_tris;
   DevBuf<int32_t> desc, pos, base;
   DevBuf<uint2> out;
   desc.st = pos.st = base.st = out.st = st;
@@ -997,18 +1180,46 @@ int kd_layout_depth_first(SceneImpl &s, const std::vector<int64_t> &level_start,
   XYZ_BUILD_TRY(pos.reserve(n));
   XYZ_BUILD_TRY(base.reserve(n));
   XYZ_BUILD_TRY(out.reserve(n));
-  size_t const levels = level_start.size() - 1;
-  for (size_t l = levels; l-- > 0;) {
-    int64_t const b = level_start[l], e = level_start[l + 1];
-    if (e > b) k_layout_desc<<<grid_for(e - b, 256, dev), 256, 0, st>>>(s.d_nodes, b, e, desc.p);
+  // the wide tree: without room for it (or with coordinates its grid
+  // arithmetic cannot hold) the scene keeps the kd-tree alone
+  float const reach = std::max({std::fabs(s.dev.bmin.x), std::fabs(s.dev.bmin.y), std::fabs(s.dev.bmin.z),
+                                std::fabs(s.dev.bmax.x), std::fabs(s.dev.bmax.y), std::fabs(s.dev.bmax.z)});
+  WideBufs B;
+  B.lo.st = B.hi.st = B.first.st = B.owner.st = B.dst.st = B.nodes.st = B.task.st = B.counters.st = B.tris.st = st;
+  WideSets T;
+  int64_t const max_wide = wide_max_nodes(nt);
+  bool const wide = reach < 1e12f && B.lo.reserve(n) == cudaSuccess && B.hi.reserve(n) == cudaSuccess &&
+                    B.first.reserve(n) == cudaSuccess && B.owner.reserve(nt) == cudaSuccess &&
+                    B.dst.reserve(nt) == cudaSuccess && B.nodes.reserve(max_wide * kWideWords) == cudaSuccess &&
+                    B.task.reserve(max_wide) == cudaSuccess && B.counters.reserve(1) == cudaSuccess &&
+                    B.tris.reserve(int64_t{kWideTriVec} * nt) == cudaSuccess;
+  if (!wide) cudaGetLastError();
+  if (wide) {
+    T = WideSets{B.lo.p, B.hi.p, B.first.p};
+    XYZ_BUILD_TRY(cudaMemsetAsync(B.lo.p, 0xff, n * sizeof(uint4), st));
+    XYZ_BUILD_TRY(cudaMemsetAsync(B.hi.p, 0, n * sizeof(uint4), st));
+    k_wide_assign<<<grid_for(nt, 256, dev), 256, 0, st>>>(s.d_tri, nt, s.d_nodes, T, B.owner.p);
   }
-  k_layout_root<<<1, 1, 0, st>>>(pos.p, base.p);
-  for (size_t l = 0; l < levels; ++l) {
+  int const levels = static_cast<int>(level_start.size()) - 1;
+  TopLevels V{};
+  while (V.n < kTopLevels && V.n < levels && level_start[V.n + 1] - level_start[V.n] <= kTopNodes) ++V.n;
+  for (int l = 0; l <= V.n; ++l) V.start[l] = level_start[l];
+  for (int l = levels; l-- > V.n;) {
     int64_t const b = level_start[l], e = level_start[l + 1];
-    if (e > b) k_layout_place<<<grid_for(e - b, 256, dev), 256, 0, st>>>(s.d_nodes, b, e, desc.p, pos.p, base.p);
+    if (e > b) k_layout_desc<<<grid_for(e - b, 256, dev), 256, 0, st>>>(s.d_nodes, b, e, desc.p, T);
+  }
+  k_layout_top<<<1, 1024, 0, st>>>(s.d_nodes, V, desc.p, pos.p, base.p, T);
+  for (int l = V.n; l < levels; ++l) {
+    int64_t const b = level_start[l], e = level_start[l + 1];
+    if (e > b) k_layout_place<<<grid_for(e - b, 256, dev), 256, 0, st>>>(s.d_nodes, b, e, desc.p, pos.p, base.p, T);
   }
   k_layout_scatter<<<grid_for(n, 256, dev), 256, 0, st>>>(s.d_nodes, n, pos.p, base.p, out.p);
   XYZ_BUILD_TRY(cudaGetLastError());
+  if (wide) {
+    int const rc = wide_build(s, B, T, reach * kWidePad, st);
+    if (rc) return rc;
+    s.dev.wide_reach = reach * kWideReach;
+  }
   XYZ_BUILD_TRY(cudaFreeAsync(s.d_nodes, st));
   s.d_nodes = out.release();
   XYZ_BUILD_TRY(cudaStreamSynchronize(st));

@@ -69,6 +69,9 @@ struct SceneImpl {
   int n_specular = 0;            // materials of kind mirror or metal
   uint2 *d_nodes = nullptr;
   int32_t *d_refs = nullptr;
+  uint32_t *d_wide = nullptr;    // wide tree (wide.cuh)
+  float4 *d_wide_tri = nullptr;  // its triangle records
+  int64_t n_wide = 0;
   int64_t n_nodes = 0, n_refs = 0, n_leaves = 0, n_empty = 0;
   int depth = 0;
   int64_t device_bytes = 0;

@@ -1,9 +1,9 @@
 // Closest-hit entry point (xyzgpu_trace_closest): the batch form of
 // Scene::FindIntersection (xyz/core/scene.hpp:277-295).
 //
-// Persistent warps with per-lane refill (trace_persistent in traverse.cuh):
-// rays are taken from a global counter as lanes free up, so long and short
-// rays balance across lanes and SMs.  Rays are read as two 16-byte vectors and
+// Persistent warps with per-lane refill (trace_wide in traverse.cuh, counting
+// calls walk the kd-tree with trace_persistent): rays are taken from a global
+// counter as lanes free up, so long and short rays balance across lanes and SMs.  Rays are read as two 16-byte vectors and
 // hits written as one.
 #include "scene.h"
 #include "traverse.cuh"
@@ -35,13 +35,18 @@ struct ApiSink {
 };
 
 template <bool kCount>
-__global__ void __launch_bounds__(kTraceThreads)
+__global__ void __launch_bounds__(kTraceThreads, kCount ? 9 : 8)
     k_trace_api(DevScene S, const float4 *__restrict__ rays, int n, float4 *__restrict__ hits,
                 int *__restrict__ fetch, unsigned long long *__restrict__ counts) {
   int const lane = threadIdx.x & 31;
   TraceCount c{0u, 0u, 0u};
   ApiSink sink{rays, hits, 0u, 0u};
-  trace_persistent<kCount>(S, n, fetch, sink, c);
+  if constexpr (kCount) {
+    trace_persistent<true>(S, n, fetch, sink, c);
+  } else {
+    __shared__ WideList s_list;
+    trace_closest_hits(S, n, fetch, sink, s_list);
+  }
   uint32_t const n_rays = sink.n_rays, n_hits = sink.n_hits;
   if (kCount) {
     unsigned long long v[5] = {n_rays, c.nodes, c.leaves, c.tris, n_hits};

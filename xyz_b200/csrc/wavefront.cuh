@@ -565,7 +565,7 @@ struct ShadowSink {
 // than 10 CTAs at 48 registers with ~50 bytes of spills), shadow rays at 10
 // (measured on B200, 1M-triangle scene).
 template <bool kShadow, bool kCount, int kMode = kModePlain>
-__global__ void __launch_bounds__(kThreads, kShadow ? 10 : 9) k_trace_queue(WaveArgs A, int b,
+__global__ void __launch_bounds__(kThreads, kCount ? (kShadow ? 10 : 9) : 8) k_trace_queue(WaveArgs A, int b,
                                                           unsigned long long *prof) {
   constexpr bool kBatch = kMode == kModeBatch;
   if constexpr (kBatch) b = A.cursor->bounce;
@@ -575,24 +575,30 @@ __global__ void __launch_bounds__(kThreads, kShadow ? 10 : 9) k_trace_queue(Wave
   int const qi = b & 1;
   TraceCount tc{0u, 0u, 0u};
   uint32_t visible = 0;
+  // counting renders walk the kd-tree, whose nodes and tests they count
+  auto trace = [&](auto &sink, int *fetch) {
+    if constexpr (kCount) {
+      trace_persistent<true, kBatch>(A.S, n, fetch, sink, tc);
+    } else {
+      __shared__ WideList s_list;
+      trace_closest_hits<kBatch>(A.S, n, fetch, sink, s_list);
+    }
+  };
   if (kShadow && kMode != kModePlain) {
     ShadowSink<false, kMode> sink{&A, 0u, b};
-    trace_persistent<kCount, kBatch>(A.S, n, &cnt[kCFetchSh], sink, tc);
+    trace(sink, &cnt[kCFetchSh]);
     visible = sink.visible;
-  } else if (kBatch) {
-    ExtSink<true> sink{A.q_o[qi], A.q_d[qi], A.hits, &A};
-    trace_persistent<kCount, true>(A.S, n, &cnt[kCFetchExt], sink, tc);
   } else if (kShadow && A.spectral) {
     ShadowSink<true> sink{&A, 0u, b};
-    trace_persistent<kCount>(A.S, n, &cnt[kCFetchSh], sink, tc);
+    trace(sink, &cnt[kCFetchSh]);
     visible = sink.visible;
   } else if (kShadow) {
     ShadowSink<false> sink{&A, 0u, b};
-    trace_persistent<kCount>(A.S, n, &cnt[kCFetchSh], sink, tc);
+    trace(sink, &cnt[kCFetchSh]);
     visible = sink.visible;
   } else {
-    ExtSink<false> sink{A.q_o[qi], A.q_d[qi], A.hits, &A};
-    trace_persistent<kCount>(A.S, n, &cnt[kCFetchExt], sink, tc);
+    ExtSink<kBatch> sink{A.q_o[qi], A.q_d[qi], A.hits, &A};
+    trace(sink, &cnt[kCFetchExt]);
   }
   if (kShadow) {
 #pragma unroll

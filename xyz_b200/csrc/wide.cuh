@@ -1,0 +1,421 @@
+// Eight-wide bounding-box tree over a scene's triangles, derived from its
+// kd-tree: the structure the traversal kernels walk (traverse.cuh).
+//
+// Every triangle belongs to the one kd leaf that holds its centroid, so the
+// kd-tree's split hierarchy becomes a hierarchy of triangle sets (no triangle
+// is referenced twice) with tight boxes.  Groups of its nodes are merged into
+// nodes of up to eight children (the child of largest surface is opened until
+// eight are found), after Ylitie, Karras and Laine, "Efficient Incoherent Ray
+// Traversal on GPUs Through Compressed Wide BVHs" (HPG 2017): child boxes
+// as 8-bit steps of a per-node power-of-two grid, children placed in octant
+// slots so that a ray visits them front to back in the order slot ^ octant.
+//
+// Node: 24 words (96 bytes, three 32-byte loads):
+//   0..2   grid origin          3   index of the first inner child
+//   4..6   grid step (x, y, z)  7   index of the node's first triangle record
+//   8      inner-child slots (8 bits) | triangle bits << 8 (3 per slot, low bits first)
+//   12..17 box minima, 8 bytes per axis (byte s = slot s); 18..23 box maxima
+// Inner children lie consecutively in slot order, triangle records in bit order.
+// Triangle record: 64 bytes, (v0, n.x) (e1, n.y) (e2, n.z) as in DevScene::tri,
+// then the triangle id, |e1| + |e2| and |n| (1-norms, for the error margins).
+//
+// A 1M-triangle mesh: 11 MB of nodes and 63 MB of records, where the kd-tree
+// keeps 38 MB of nodes, 35 MB of references and 47 MB of triangles.
+//
+// The functions are __host__ __device__: the host builds and walks the same
+// tree in the tests' CPU check.
+#pragma once
+
+#include <cmath>
+#include <cstring>
+
+#include "common.cuh"
+
+namespace xyzgpu {
+
+constexpr int kWideWords = 24;       // 32-bit words of a node
+constexpr int kWideLeafTris = 3;     // triangles of a leaf child
+constexpr int kWideStack = 64;       // node groups a ray may hold: the tree is no deeper
+constexpr int kWideTriVec = 4;       // float4 per triangle record
+// Boxes grow by this share of the largest scene coordinate S on every side,
+// and rays whose origin has a coordinate beyond kWideReach * S do not use the
+// tree: the grid arithmetic errs by at most 2^-22 of the largest |box - origin|
+// (9 S * 2^-22 = 2.1e-6 S), the padding is 3.8e-6 S.
+constexpr float kWidePad = 1.0f / 262144.0f;
+constexpr float kWideReach = 8.0f;
+
+// Triangle sets of the kd-tree's (breadth-first) nodes while the tree is built.
+struct WideSets {
+  uint4 *lo = nullptr;       // ordered keys of the box minimum
+  uint4 *hi = nullptr;       // of the maximum; w: triangles below the node
+  int32_t *first = nullptr;  // first triangle of the node in depth-first order
+};
+
+// A wide node to be built: `cnt` triangles from `first` under kd node `node`
+// (all of it, or for a leaf with many triangles a range).
+struct WideTask {
+  int32_t node, first, cnt;
+};
+
+XYZ_HD uint32_t float_key(float f) {
+#ifdef __CUDA_ARCH__
+  uint32_t const u = __float_as_uint(f);
+#else
+  uint32_t u;
+  std::memcpy(&u, &f, 4);
+#endif
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+XYZ_HD float key_float(uint32_t k) {
+  uint32_t const u = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
+#ifdef __CUDA_ARCH__
+  return __uint_as_float(u);
+#else
+  float f;
+  std::memcpy(&f, &u, 4);
+  return f;
+#endif
+}
+XYZ_HD uint32_t wide_bits(float f) {
+#ifdef __CUDA_ARCH__
+  return __float_as_uint(f);
+#else
+  uint32_t u;
+  std::memcpy(&u, &f, 4);
+  return u;
+#endif
+}
+XYZ_HD float wide_float(uint32_t u) {
+#ifdef __CUDA_ARCH__
+  return __uint_as_float(u);
+#else
+  float f;
+  std::memcpy(&f, &u, 4);
+  return f;
+#endif
+}
+
+// The kd leaf that holds the point: at a split plane, the side above.
+XYZ_HD int32_t wide_leaf_of(const uint2 *nodes, f3 p) {
+  uint32_t i = 0;
+  uint2 nd = nodes[0];
+  while ((nd.y & 3u) != kKdLeafTag) {
+    uint32_t const ax = nd.y & 3u;
+    float const v = ax == 0 ? p.x : (ax == 1 ? p.y : p.z);
+    i = (nd.y >> 2) + (v < wide_float(nd.x) ? 0u : 1u);
+    nd = nodes[i];
+  }
+  return static_cast<int32_t>(i);
+}
+
+// Opens a task into two, descending past kd nodes with all triangles on one
+// side; a kd leaf's range is halved.  cnt > kWideLeafTris.
+XYZ_HD void wide_open(const uint2 *nodes, const WideSets &T, WideTask t, WideTask *a, WideTask *b) {
+  for (;;) {
+    uint2 const nd = nodes[t.node];
+    if ((nd.y & 3u) == kKdLeafTag) {
+      int const h = t.cnt >> 1;
+      *a = WideTask{t.node, t.first, h};
+      *b = WideTask{t.node, t.first + h, t.cnt - h};
+      return;
+    }
+    int32_t const c = static_cast<int32_t>(nd.y >> 2);
+    int32_t const nl = static_cast<int32_t>(T.hi[c].w), nr = static_cast<int32_t>(T.hi[c + 1].w);
+    if (nl > 0 && nr > 0) {
+      *a = WideTask{c, t.first, nl};
+      *b = WideTask{c + 1, t.first + nl, nr};
+      return;
+    }
+    t.node = nl > 0 ? c : c + 1;
+  }
+}
+
+struct WideBox {
+  float lo[3], hi[3];
+};
+
+XYZ_HD WideBox wide_box(const WideSets &T, int32_t node) {
+  uint4 const l = T.lo[node], h = T.hi[node];
+  return WideBox{{key_float(l.x), key_float(l.y), key_float(l.z)}, {key_float(h.x), key_float(h.y), key_float(h.z)}};
+}
+
+// The smallest power of two s >= 2^-100 with 252 s >= extent (the grid starts
+// 1/64 step before the boxes and each bound may round one step outwards).
+XYZ_HD float wide_step(float extent) {
+  float const r = extent * (1.0f / 252.0f);
+  uint32_t e = (wide_bits(r) >> 23) & 0xffu;
+  if (wide_bits(r) & 0x7fffffu) ++e;
+  if (e < 27u) e = 27u;
+  return wide_float(e << 23);
+}
+
+// Builds one node of the tree.  alloc_nodes(k) / alloc_tris(k) reserve k
+// consecutive node / record indices; put_task(i, t) names the task of inner
+// node i, put_tri(pos, rec) the record of the triangle at depth-first
+// position pos.
+template <class AllocNodes, class AllocTris, class PutTask, class PutTri>
+XYZ_HD void wide_make_node(const uint2 *nodes, const WideSets &T, WideTask root, float pad, uint32_t *w,
+                           AllocNodes alloc_nodes, AllocTris alloc_tris, PutTask put_task, PutTri put_tri) {
+  WideTask it[8];
+  float area[8];
+  int m = 1;
+  it[0] = root;
+  area[0] = INFINITY;
+  while (m < 8) {
+    // the largest child that cannot be a leaf, then (into slots that would stay
+    // empty) the largest leaf of several triangles
+    int best = -1;
+    for (int i = 0; i < m; ++i)
+      if (it[i].cnt > kWideLeafTris && (best < 0 || area[i] > area[best])) best = i;
+    if (best < 0)
+      for (int i = 0; i < m; ++i)
+        if (it[i].cnt > 1 && (best < 0 || area[i] > area[best])) best = i;
+    if (best < 0) break;
+    WideTask a, b;
+    wide_open(nodes, T, it[best], &a, &b);
+    it[best] = a;
+    it[m] = b;
+    for (int k = 0; k < 2; ++k) {
+      int const i = k == 0 ? best : m;
+      WideBox const x = wide_box(T, it[i].node);
+      float const dx = x.hi[0] - x.lo[0], dy = x.hi[1] - x.lo[1], dz = x.hi[2] - x.lo[2];
+      area[i] = dx * dy + dy * dz + dz * dx;
+    }
+    ++m;
+  }
+  WideBox box[8], all;
+  for (int k = 0; k < 3; ++k) {
+    all.lo[k] = INFINITY;
+    all.hi[k] = -INFINITY;
+  }
+  for (int i = 0; i < m; ++i) {
+    box[i] = wide_box(T, it[i].node);
+    for (int k = 0; k < 3; ++k) {
+      box[i].lo[k] -= pad;
+      box[i].hi[k] += pad;
+      all.lo[k] = fminf(all.lo[k], box[i].lo[k]);
+      all.hi[k] = fmaxf(all.hi[k], box[i].hi[k]);
+    }
+  }
+  // octant slots: the (child, slot) pair that fits best, until all are placed
+  int slot_child[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
+  uint32_t todo = (1u << m) - 1u;
+  while (todo) {
+    float best = -INFINITY;
+    int bc = -1, bs = -1;
+    for (int i = 0; i < m; ++i) {
+      if (!(todo & (1u << i))) continue;
+      float c[3];
+      for (int k = 0; k < 3; ++k) c[k] = (box[i].lo[k] + box[i].hi[k]) - (all.lo[k] + all.hi[k]);
+      for (int s = 0; s < 8; ++s) {
+        if (slot_child[s] >= 0) continue;
+        float const v = ((s & 1) ? c[0] : -c[0]) + ((s & 2) ? c[1] : -c[1]) + ((s & 4) ? c[2] : -c[2]);
+        if (bc < 0 || v > best) {
+          best = v;
+          bc = i;
+          bs = s;
+        }
+      }
+    }
+    slot_child[bs] = bc;
+    todo &= ~(1u << bc);
+  }
+  for (int k = 0; k < kWideWords; ++k) w[k] = 0u;
+  float step[3], org[3];
+  for (int k = 0; k < 3; ++k) {
+    step[k] = wide_step(all.hi[k] - all.lo[k]);
+    org[k] = all.lo[k] - step[k] * (1.0f / 64.0f);
+    w[k] = wide_bits(org[k]);
+    w[4 + k] = wide_bits(step[k]);
+  }
+  int n_inner = 0, n_tris = 0;
+  for (int s = 0; s < 8; ++s) {
+    int const i = slot_child[s];
+    if (i < 0) continue;
+    if (it[i].cnt > kWideLeafTris)
+      ++n_inner;
+    else
+      n_tris += it[i].cnt;
+  }
+  uint32_t const nb = n_inner ? alloc_nodes(n_inner) : 0u;
+  uint32_t const tb = n_tris ? alloc_tris(n_tris) : 0u;
+  w[3] = nb;
+  w[7] = tb;
+  uint32_t meta = 0u;
+  int ni = 0, ti = 0;
+  for (int s = 0; s < 8; ++s) {
+    int const i = slot_child[s];
+    if (i < 0) continue;
+    if (it[i].cnt > kWideLeafTris) {
+      meta |= 1u << s;
+      put_task(nb + ni, it[i]);
+      ++ni;
+    } else {
+      for (int c = 0; c < it[i].cnt; ++c) {
+        meta |= 1u << (8 + 3 * s + c);
+        put_tri(it[i].first + c, tb + ti);
+        ++ti;
+      }
+    }
+    for (int k = 0; k < 3; ++k) {
+      // wide_test places a plane to 1/256 step (its bytes are read as 65536 +
+      // byte): a bound rounds outwards from 1/128 step beyond the box
+      float const ql = floorf((box[i].lo[k] - org[k]) / step[k] - (1.0f / 128.0f));
+      float const qh = ceilf((box[i].hi[k] - org[k]) / step[k] + (1.0f / 128.0f));
+      uint32_t const bl = static_cast<uint32_t>(fminf(fmaxf(ql, 0.0f), 255.0f));
+      uint32_t const bh = static_cast<uint32_t>(fminf(fmaxf(qh, 0.0f), 255.0f));
+      w[12 + 2 * k + (s >> 2)] |= bl << (8 * (s & 3));
+      w[18 + 2 * k + (s >> 2)] |= bh << (8 * (s & 3));
+    }
+  }
+  w[8] = meta;
+}
+
+// ---------------------------------------------------------------- walking
+// What the box tests of a ray need: origin, reciprocal direction (components
+// below 1e-18 replaced by 1e-18 of their sign) and the order its octant gives
+// the slots.
+struct WideRay {
+  f3 o, inv;
+  uint32_t octinv;  // bit k set: the direction's component k is >= 0
+};
+
+XYZ_HD float wide_inv(float d) {
+  float const a = fabsf(d) < 1e-18f ? copysignf(1e-18f, d) : d;
+#ifdef __CUDA_ARCH__
+  return __frcp_rn(a);
+#else
+  return 1.0f / a;
+#endif
+}
+
+XYZ_HD WideRay wide_ray(f3 o, f3 d) {
+  WideRay r;
+  r.o = o;
+  r.inv = mk3(wide_inv(d.x), wide_inv(d.y), wide_inv(d.z));
+  r.octinv = (r.inv.x >= 0.0f ? 1u : 0u) | (r.inv.y >= 0.0f ? 2u : 0u) | (r.inv.z >= 0.0f ? 4u : 0u);
+  return r;
+}
+
+// Rays the tree answers: origin within reach of the scene, direction of
+// about unit length (the margins of wide_margin assume |d| <= 2).
+XYZ_HD bool wide_usable(f3 o, f3 d, float reach) {
+  float const dd = dot3(d, d);
+  return fabsf(o.x) <= reach && fabsf(o.y) <= reach && fabsf(o.z) <= reach && dd <= 4.0f && dd >= 1e-4f;
+}
+
+// Byte j of w as the float 65536 + byte: the byte times 128 added to the bits
+// of 65536 (an integer dot product: it runs on the FMA pipe, where the
+// bit-moving forms would add to the ALU pipe that the comparisons fill).
+template <int J>
+XYZ_HD float wide_byte(uint32_t w) {
+#ifdef __CUDA_ARCH__
+  return __uint_as_float(__dp4a(w, 128u << (8 * J), 0x47800000u));
+#else
+  return 65536.0f + static_cast<float>((w >> (8 * J)) & 0xffu);
+#endif
+}
+
+XYZ_HD float wide_max3(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+#else
+  return fmaxf(fmaxf(a, b), c);
+#endif
+}
+XYZ_HD float wide_min3(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+#else
+  return fminf(fminf(a, b), c);
+#endif
+}
+
+// Two fused multiply-adds q * a + c of one axis (packed FP32 on the device).
+XYZ_HD void wide_fma2(float q0, float q1, float a, float c, float *t0, float *t1) {
+#ifdef __CUDA_ARCH__
+  unsigned long long q, aa, cc, r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(q) : "f"(q0), "f"(q1));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(aa) : "f"(a));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(cc) : "f"(c));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(q), "l"(aa), "l"(cc));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(*t0), "=f"(*t1) : "l"(r));
+#else
+  *t0 = std::fma(q0, a, c);
+  *t1 = std::fma(q1, a, c);
+#endif
+}
+
+// Slots kSlot + J and kSlot + J + 1 of a node (bytes J, J + 1 of the words n, f):
+// 2^slot added to m where the ray's box interval meets [tmin, tlim].
+template <int kSlot, int J>
+XYZ_HD float wide_pair(const uint32_t n[3], const uint32_t f[3], const float a[3], const float c[3], float tmin,
+                       float tlim, float m) {
+  float tn[3][2], tf[3][2];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    wide_fma2(wide_byte<J>(n[k]), wide_byte<J + 1>(n[k]), a[k], c[k], &tn[k][0], &tn[k][1]);
+    wide_fma2(wide_byte<J>(f[k]), wide_byte<J + 1>(f[k]), a[k], c[k], &tf[k][0], &tf[k][1]);
+  }
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    float const t0 = fmaxf(wide_max3(tn[0][s], tn[1][s], tn[2][s]), tmin);
+    float const t1 = fminf(wide_min3(tf[0][s], tf[1][s], tf[2][s]), tlim);
+    if (t0 <= t1) m += static_cast<float>(1 << (kSlot + J + s));
+  }
+  return m;
+}
+
+// Slots of node w whose boxes the ray meets within [tmin, tlim].  Empty slots
+// may report a hit (their box is the grid's first cell): neither an inner bit
+// nor a triangle bit of the node belongs to them.
+XYZ_HD uint32_t wide_test(const uint32_t *w, const WideRay &r, float tmin, float tlim) {
+  float a[3], c[3];
+  float const inv[3] = {r.inv.x, r.inv.y, r.inv.z}, o[3] = {r.o.x, r.o.y, r.o.z};
+  uint32_t near0[3], near1[3], far0[3], far1[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    a[k] = wide_float(w[4 + k]) * inv[k];
+    // (origin - o) * inv - 65536 * a: the bytes are read as 65536 + byte
+    float const po = wide_float(w[k]) - o[k];
+#ifdef __CUDA_ARCH__
+    c[k] = __fmaf_rn(-65536.0f, a[k], po * inv[k]);
+#else
+    c[k] = std::fma(-65536.0f, a[k], po * inv[k]);
+#endif
+    bool const pos = (r.octinv >> k) & 1u;
+    near0[k] = pos ? w[12 + 2 * k] : w[18 + 2 * k];
+    near1[k] = pos ? w[13 + 2 * k] : w[19 + 2 * k];
+    far0[k] = pos ? w[18 + 2 * k] : w[12 + 2 * k];
+    far1[k] = pos ? w[19 + 2 * k] : w[13 + 2 * k];
+  }
+  float m = 8388608.0f;  // 2^23: the sum's low mantissa bits are the slots
+  m = wide_pair<0, 0>(near0, far0, a, c, tmin, tlim, m);
+  m = wide_pair<0, 2>(near0, far0, a, c, tmin, tlim, m);
+  m = wide_pair<4, 0>(near1, far1, a, c, tmin, tlim, m);
+  m = wide_pair<4, 2>(near1, far1, a, c, tmin, tlim, m);
+  return wide_bits(m) & 0xffu;
+}
+
+// Slot bits to visiting order: bit s moves to bit s ^ octinv; the highest bit
+// is visited first.
+XYZ_HD uint32_t wide_order(uint32_t h, uint32_t octinv) {
+  if (octinv & 1u) h = ((h & 0x55u) << 1) | ((h >> 1) & 0x55u);
+  if (octinv & 2u) h = ((h & 0x33u) << 2) | ((h >> 2) & 0x33u);
+  if (octinv & 4u) h = ((h & 0x0fu) << 4) | (h >> 4);
+  return h;
+}
+
+// Slot bits to triangle bits (three per slot).
+XYZ_HD uint32_t wide_spread(uint32_t h) {
+  h = (h | (h << 8)) & 0x00f00fu;
+  h = (h | (h << 4)) & 0x0c30c3u;
+  h = (h | (h << 2)) & 0x249249u;
+  return h * 7u;
+}
+
+}  // namespace xyzgpu
