@@ -45,6 +45,19 @@ XYZ_DEV f3 normalize3(f3 a) {
 XYZ_HD float norm1(f3 a) { return fabsf(a.x) + fabsf(a.y) + fabsf(a.z); }
 XYZ_HD f3 xyz3(float4 v) { return f3{v.x, v.y, v.z}; }
 
+// Octant (eighths of the full turn, 0 .. 7) of the angle of (x, y), or -1 where
+// the point is so close to an octant's border (1e-5 of |x| + |y|, far above the
+// error of an arc tangent) that the rounding of the angle decides.
+XYZ_HD int octant_of(float y, float x) {
+  float const ax = fabsf(x), ay = fabsf(y);
+  float const tol = 1e-5f * (ax + ay);
+  if (!(ax > tol && ay > tol && fabsf(ax - ay) > tol)) return -1;
+  // quadrant, then its half that lies further round
+  int const quad = y > 0.0f ? (x > 0.0f ? 0 : 1) : (x < 0.0f ? 2 : 3);
+  bool const steep = ay > ax;
+  return 2 * quad + (((quad & 1) != 0) != steep ? 1 : 0);
+}
+
 // ---------------------------------------------------------------- random
 // Philox4x32-10 (Salmon et al., SC'11).  Stream layout in include/xyzgpu.h.
 XYZ_HD void philox4x32_10(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, uint32_t k0,

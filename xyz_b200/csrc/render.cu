@@ -396,7 +396,8 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
             int const qi = b & 1;
             XYZ_MARK(5, true);
             int const r = importon_query_launch(*imp->m, A.q_o[qi], A.q_d[qi], A.hits,
-                                                A.counts + b * kCountStride + kCExt, A.S, imp_cdf, st);
+                                                A.counts + b * kCountStride + kCExt,
+                                                A.counts + b * kCountStride + kCFetchQuery, A.S, imp_cdf, st);
             if (r) return r;
             XYZ_MARK(5, false);
             ++launches;

@@ -138,7 +138,7 @@ struct ImportonHooks {
 };
 int importon_wave_prepare(ImportonImpl &m, int64_t capacity, float **cdf);
 int importon_query_launch(ImportonImpl &m, const float4 *qo, const float4 *qd, const float4 *hits,
-                          const int32_t *count, const DevScene &S, float *cdf, cudaStream_t st);
+                          const int32_t *count, int32_t *fetch, const DevScene &S, float *cdf, cudaStream_t st);
 int importon_guide_bounces(const ImportonImpl &m);
 
 int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_params &rp,

@@ -51,6 +51,7 @@ constexpr int kCShadow = 1;     // shadow rays produced in iteration b
 constexpr int kCFetchExt = 2;   // work counter of the extension trace
 constexpr int kCFetchSh = 3;    // work counter of the shadow trace
 constexpr int kCVisible = 4;    // shadow rays that reached their vertex
+constexpr int kCFetchQuery = 5; // work counter of the importon queries
 
 struct CamDev {
   f3 eye, right, up, back;
@@ -699,10 +700,14 @@ XYZ_DEV int importon_bin(f3 dir, f3 sn, f3 tan, f3 bin, bool *above) {
   *above = cs > 0.0f;
   int u = static_cast<int>(cs * cs * 2.0f);
   if (u >= 2) u = 1;
-  float phi = 0.5f * atan2f(-dot3(dir, bin), -dot3(dir, tan));
-  if (phi < 0.0f) phi = static_cast<float>(static_cast<double>(phi) + kPi);
-  int v = static_cast<int>(static_cast<double>(phi) * (8.0 * kInvPi));
-  if (v >= 8) v = 7;
+  float const y = -dot3(dir, bin), x = -dot3(dir, tan);
+  int v = octant_of(y, x);
+  if (v < 0) {
+    float phi = 0.5f * atan2f(y, x);
+    if (phi < 0.0f) phi = static_cast<float>(static_cast<double>(phi) + kPi);
+    v = static_cast<int>(static_cast<double>(phi) * (8.0 * kInvPi));
+    if (v >= 8) v = 7;
+  }
   return u * 8 + v;
 }
 
