@@ -24,12 +24,17 @@ namespace {
 
 constexpr int kFilmThreads = 256;
 
-int film_grid(int64_t n) {
+bool aligned(const void *p, uintptr_t bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; }
+
+int device_sms() {
   int dev = 0;
   cudaGetDevice(&dev);
-  int64_t const want = (n + kFilmThreads - 1) / kFilmThreads;
-  int64_t const cap = static_cast<int64_t>(sm_count(dev)) * 8;
-  return static_cast<int>(std::max<int64_t>(1, std::min(want, cap)));
+  return sm_count(dev);
+}
+
+// One thread per item (a grid-stride loop takes what lies beyond the limit).
+int film_grid(int64_t n) {
+  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((n + kFilmThreads - 1) / kFilmThreads, 1 << 20)));
 }
 
 // static_cast<unsigned char>(float) as the reference's build performs it: the
@@ -38,39 +43,94 @@ int film_grid(int64_t n) {
 // saturate).
 __device__ __forceinline__ uint8_t byte_of(float v) { return static_cast<uint8_t>(static_cast<uint32_t>(__float2int_rz(v))); }
 
-// hdr_encode (imagefilm_hdr.cpp:14-31): mantissa scale frexp(d) * 255.9999 / d
-// in double, rounded to float, times each component.
+// hdr_encode (imagefilm_hdr.cpp:14-31): the scale frexp(d) * 255.9999 / d,
+// in double, rounded to float, times each component.  frexp(d) / d is the power
+// of two 2^-e, so the scale is 255.9999 2^-e up to the two roundings in double
+// (2^-52), and 255.9999 lies far from a float rounding border: the rounded
+// scale is the float nearest 255.9999 with its exponent lowered by e (d is
+// above 1e-32, so e and the scale stay in the normal range).
+__host__ __device__ __forceinline__ float rgbe_scale(int e) {
+  uint32_t const bits = 0x437ffff9u - (static_cast<uint32_t>(e) << 23);  // 255.9999f
+#ifdef __CUDA_ARCH__
+  return __uint_as_float(bits);
+#else
+  float f;
+  std::memcpy(&f, &bits, 4);
+  return f;
+#endif
+}
+
 __device__ __forceinline__ uchar4 rgbe_of(float r, float g, float b) {
   float const d = fmaxf(fmaxf(r, g), b);
   if (static_cast<double>(d) <= 1e-32) return make_uchar4(0, 0, 0, 0);
-  int e = 0;
-  float const m = frexpf(d, &e);
-  float const f = static_cast<float>(static_cast<double>(m) * 255.9999 / static_cast<double>(d));
+  int e = (static_cast<int>(__float_as_uint(d) >> 23) & 0xff) - 126;
+  float f = rgbe_scale(e);
+  if (!isfinite(d)) {  // XYZE keeps such pixels
+    e = 0;
+    float const m = frexpf(d, &e);
+    f = static_cast<float>(static_cast<double>(m) * 255.9999 / static_cast<double>(d));
+  }
   return make_uchar4(byte_of(r * f), byte_of(g * f), byte_of(b * f), static_cast<uint8_t>(e + 128));
 }
 
-// One thread per pixel; output in file order.  RGBE: scanlines from the top
-// image row down ("-Y H +X W"), the film's XYZ / spp converted to CCIR 601-1
-// RGB (CCIR601_1_XYZ2RGB, libhi/hi/image/color_space.hpp:69-79) and a
+// Four film pixels of a row from pixel p (n of them inside the row): 16-byte
+// loads where the film's rows allow it.
+__device__ __forceinline__ void load_pixels(const float *__restrict__ film, int64_t p, int n, bool vec, float v[12]) {
+  if (vec) {
+    const float4 *q = reinterpret_cast<const float4 *>(film + 3 * p);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      float4 const x = __ldcs(q + k);
+      v[4 * k] = x.x, v[4 * k + 1] = x.y, v[4 * k + 2] = x.z, v[4 * k + 3] = x.w;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 12; ++k) v[k] = k < 3 * n ? film[3 * p + k] : 0.0f;
+  }
+}
+
+// Four pixels of a row per thread; output in file order.  RGBE: scanlines from
+// the top image row down ("-Y H +X W"), the film's XYZ / spp converted to CCIR
+// 601-1 RGB (CCIR601_1_XYZ2RGB, libhi/hi/image/color_space.hpp:69-79) and a
 // non-finite pixel written as 0.  XYZE (the reference's CONFIG_HDR_STRICT
 // build): XYZ / spp, scanlines from the bottom row up ("+Y H +X W").
-__global__ void k_film_rgbe(const float *__restrict__ film, int W, int H, float scale, int xyze,
-                            uchar4 *__restrict__ out) {
-  int64_t const n = static_cast<int64_t>(W) * H;
+// Measured at 1920 x 1080: one pixel per thread with the scale in double 13.4
+// us, this form 9.2 (33 MB; 5.1 us at the copy rate).
+__global__ void __launch_bounds__(kFilmThreads)
+    k_film_rgbe(const float *__restrict__ film, int W, int H, float scale, int xyze, int vec, uchar4 *__restrict__ out) {
+  int const quads = (W + 3) >> 2;
+  int64_t const n = static_cast<int64_t>(quads) * H;
   for (int64_t q = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; q < n;
        q += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    int64_t const row = q / W, x = q - row * W;
-    int64_t const p = (xyze ? row : (H - 1 - row)) * W + x;
-    float const X = film[3 * p] * scale, Y = film[3 * p + 1] * scale, Z = film[3 * p + 2] * scale;
-    if (xyze) {
-      out[q] = rgbe_of(X, Y, Z);
-      continue;
+    int64_t const row = q / quads;
+    int const x = static_cast<int>(q - row * quads) * 4, m = min(4, W - x);
+    float v[12];
+    load_pixels(film, (xyze ? row : (H - 1 - row)) * W + x, m, vec != 0, v);
+    uchar4 px[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float const X = v[3 * k] * scale, Y = v[3 * k + 1] * scale, Z = v[3 * k + 2] * scale;
+      if (xyze) {
+        px[k] = rgbe_of(X, Y, Z);
+        continue;
+      }
+      float r = 1.9104f * X - 0.5338f * Y - 0.2891f * Z;
+      float g = -0.9844f * X + 1.9985f * Y - 0.0279f * Z;
+      float b = 0.0585f * X - 0.1187f * Y + 0.9017f * Z;
+      if (!isfinite(r) || !isfinite(g) || !isfinite(b)) r = g = b = 0.0f;
+      px[k] = rgbe_of(r, g, b);
     }
-    float r = 1.9104f * X - 0.5338f * Y - 0.2891f * Z;
-    float g = -0.9844f * X + 1.9985f * Y - 0.0279f * Z;
-    float b = 0.0585f * X - 0.1187f * Y + 0.9017f * Z;
-    if (!isfinite(r) || !isfinite(g) || !isfinite(b)) r = g = b = 0.0f;
-    out[q] = rgbe_of(r, g, b);
+    uchar4 *const o = out + row * W + x;
+    if (vec) {
+      uint32_t w[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) w[k] = *reinterpret_cast<const uint32_t *>(&px[k]);
+      *reinterpret_cast<uint4 *>(o) = make_uint4(w[0], w[1], w[2], w[3]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (k < m) o[k] = px[k];
+    }
   }
 }
 
@@ -78,23 +138,40 @@ __global__ void k_film_rgbe(const float *__restrict__ film, int W, int H, float 
 // maximum over pixels of 0.6069 c0 + 0.1735 c1 + 0.2003 c2 of the values
 // tone-mapped (float2bmp/main.cpp:186-196; the maximum starts at 0, so the
 // non-negative float bits order as integers).
-__global__ void k_film_max_luminance(const float *__restrict__ film, int64_t n, float scale, int rgb,
-                                     unsigned int *out) {
+// Four pixels per thread and step; one atomic per CTA (a CTA of every eighth
+// of an SM's threads would otherwise send 9,472 to one word).
+__global__ void __launch_bounds__(kFilmThreads)
+    k_film_max_luminance(const float *__restrict__ film, int64_t n, float scale, int rgb, int vec, unsigned int *out) {
+  __shared__ float s_best[kFilmThreads / 32];
   float best = 0.0f;
-  for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < n;
-       p += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    float c[3] = {film[3 * p] * scale, film[3 * p + 1] * scale, film[3 * p + 2] * scale};
-    if (rgb) {
-      float const X = c[0], Y = c[1], Z = c[2];
-      c[0] = 1.9104f * X - 0.5338f * Y - 0.2891f * Z;
-      c[1] = -0.9844f * X + 1.9985f * Y - 0.0279f * Z;
-      c[2] = 0.0585f * X - 0.1187f * Y + 0.9017f * Z;
+  int64_t const quads = (n + 3) >> 2;
+  for (int64_t q = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; q < quads;
+       q += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    int const m = static_cast<int>(min(int64_t{4}, n - 4 * q));
+    float v[12];
+    load_pixels(film, 4 * q, m, vec != 0 && m == 4, v);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (k >= m) break;
+      float c[3] = {v[3 * k] * scale, v[3 * k + 1] * scale, v[3 * k + 2] * scale};
+      if (rgb) {
+        float const X = c[0], Y = c[1], Z = c[2];
+        c[0] = 1.9104f * X - 0.5338f * Y - 0.2891f * Z;
+        c[1] = -0.9844f * X + 1.9985f * Y - 0.0279f * Z;
+        c[2] = 0.0585f * X - 0.1187f * Y + 0.9017f * Z;
+      }
+      float const l = 0.6069f * c[0] + 0.1735f * c[1] + 0.2003f * c[2];
+      if (best < l) best = l;
     }
-    float const l = 0.6069f * c[0] + 0.1735f * c[1] + 0.2003f * c[2];
-    if (best < l) best = l;
   }
   for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_down_sync(0xffffffffu, best, o));
-  if ((threadIdx.x & 31) == 0 && best > 0.0f) atomicMax(out, __float_as_uint(best));
+  if ((threadIdx.x & 31) == 0) s_best[threadIdx.x >> 5] = best;
+  __syncthreads();
+  if (threadIdx.x < kFilmThreads / 32) {
+    best = s_best[threadIdx.x];
+    for (int o = kFilmThreads / 64; o > 0; o >>= 1) best = fmaxf(best, __shfl_down_sync(0xffu, best, o));
+    if (threadIdx.x == 0 && best > 0.0f) atomicMax(out, __float_as_uint(best));
+  }
 }
 
 struct ToneArgs {
@@ -104,8 +181,8 @@ struct ToneArgs {
 };
 
 // tonemap() of float2bmp/main.cpp:80-118: operator, gamma src / dst, then the
-// 8-bit quantisation of clamp() (:69-77).
-__device__ __forceinline__ uint8_t tone_one(float light, const ToneArgs &T, float white) {
+// 8-bit quantisation of clamp() (:69-77), in the tool's float arithmetic.
+__device__ __noinline__ uint8_t tone_exact(float light, const ToneArgs &T, float white) {
   if (light <= 0.0f) return 0;
   float v;
   switch (T.op) {
@@ -120,29 +197,123 @@ __device__ __forceinline__ uint8_t tone_one(float light, const ToneArgs &T, floa
   return static_cast<uint8_t>(v * 256.0f);
 }
 
-// One thread per pixel; BMP order (rows from the bottom, as the film) and
-// byte order (blue, green, red = channel 2, 1, 0), rows padded to 4 bytes.
-__global__ void k_film_tonemap(const float *__restrict__ film, int W, int H, ToneArgs T, uint8_t *__restrict__ out) {
+__device__ __forceinline__ float exp2_fast(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float log2_fast(float x) {
+  float r;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rcp_fast(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// The same byte by the fast reciprocal, exponential and logarithm where their
+// result p (in 256ths) lies clear of an integer, or -1 where tone_exact has to
+// be asked.  With L = log2 v and g <= 1, p errs by p (1.7e-7 (1 + |L|) g + 2.4e-7)
+// from the logarithm (2^-22, relative below 1/2) and the power, and by p 1e-6 g
+// from the operator (6 roundings and a reciprocal of 1 ulp): at most 4.5e-4, so
+// 5e-4 is clear.  The film operator 1 - e^-x, used from x = 0.05 on, errs by
+// 256 * 3.6e-6 = 9e-4 (the cancellation, on either side): 2e-3.  Zeros,
+// infinities and NaN (which end at 0 or 1e6 exactly) and other exponents are
+// not clear.
+__device__ __forceinline__ int tone_fast(float light, const ToneArgs &T, float inv_white2) {
+  float v = T.exposure * light;
+  bool fast = T.gamma <= 1.0f;
+  float clear = 5e-4f;
+  if (T.op == XYZGPU_TONEMAP_REINHARD) {
+    v = v * rcp_fast(1.0f + light);
+  } else if (T.op == XYZGPU_TONEMAP_REINHARD_WHITE) {
+    v = v * (1.0f + light * inv_white2) * rcp_fast(1.0f + light);
+  } else if (T.op == XYZGPU_TONEMAP_FILM) {
+    fast = fast && v >= 0.05f;
+    clear = 2e-3f;
+    v = 1.0f - exp2_fast(-1.44269504f * v);
+  }
+  float const p = fminf(exp2_fast(T.gamma * log2_fast(v)) * 256.0f, 1e6f);
+  // nearest integer in the low bits of p + 2^23
+  float const q = p + 8388608.0f, r = q - 8388608.0f;
+  int const byte = min((__float_as_int(q) & 0x7fffff) - (p < r ? 1 : 0), 255);
+  fast = fast && fabsf(p - r) > clear;
+  return light <= 0.0f ? 0 : (fast ? byte : -1);
+}
+
+__device__ __forceinline__ void tone_channels(const ToneArgs &T, float X, float Y, float Z, float c[3]) {
+  c[0] = X * T.scale;
+  c[1] = Y * T.scale;
+  c[2] = Z * T.scale;
+  if (T.rgb) {
+    float const x = c[0], y = c[1], z = c[2];
+    c[0] = 1.9104f * x - 0.5338f * y - 0.2891f * z;
+    c[1] = -0.9844f * x + 1.9985f * y - 0.0279f * z;
+    c[2] = 0.0585f * x - 0.1187f * y + 0.9017f * z;
+  }
+}
+
+// Four pixels of a row per thread: twelve bytes, which are three aligned words
+// of the row (rows are padded to 4 bytes).  BMP order (rows from the bottom, as
+// the film) and byte order (blue, green, red = channel 2, 1, 0); the row's
+// padding bytes are zero (the caller's buffer may hold anything).
+// Measured at 1920 x 1080 (Reinhard with the image's white): a pixel per
+// thread with powf and byte stores 37.0 us, this form 16.3 (issue-bound: 76 % of
+// cycles); the maximum before it 9.5 -> 5.1.
+__global__ void __launch_bounds__(kFilmThreads)
+    k_film_tonemap(const float *__restrict__ film, int W, int H, ToneArgs T, int vec, int words,
+                   uint8_t *__restrict__ out) {
   float const white = T.white_bits ? __uint_as_float(*T.white_bits) : T.white;
+  float const inv_white2 = __fdividef(1.0f, white * white);
   int64_t const stride_b = (3 * static_cast<int64_t>(W) + 3) & ~int64_t{3};
-  int64_t const n = static_cast<int64_t>(W) * H;
-  for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < n;
-       p += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    float c[3] = {film[3 * p] * T.scale, film[3 * p + 1] * T.scale, film[3 * p + 2] * T.scale};
-    if (T.rgb) {
-      float const X = c[0], Y = c[1], Z = c[2];
-      c[0] = 1.9104f * X - 0.5338f * Y - 0.2891f * Z;
-      c[1] = -0.9844f * X + 1.9985f * Y - 0.0279f * Z;
-      c[2] = 0.0585f * X - 0.1187f * Y + 0.9017f * Z;
+  int const quads = (W + 3) >> 2;
+  int64_t const n = static_cast<int64_t>(quads) * H;
+  for (int64_t q = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; q < n;
+       q += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    int64_t const y = q / quads;
+    int const x = static_cast<int>(q - y * quads) * 4, m = min(4, W - x);
+    float v[12];
+    load_pixels(film, y * W + x, m, vec != 0, v);
+    uint32_t w[3] = {0u, 0u, 0u}, ask = 0u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float c[3];
+      tone_channels(T, v[3 * k], v[3 * k + 1], v[3 * k + 2], c);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        int const at = 3 * k + j, byte = tone_fast(c[2 - j], T, inv_white2);
+        w[at >> 2] |= static_cast<uint32_t>(byte & 0xff) << (8 * (at & 3));
+        if (byte < 0 && k < m) ask |= 1u << at;
+        if (k >= m) w[at >> 2] &= ~(0xffu << (8 * (at & 3)));
+      }
     }
-    int64_t const y = p / W, x = p - y * W;
-    uint8_t *o = out + y * stride_b + 3 * x;
-    o[2] = tone_one(c[0], T, white);
-    o[1] = tone_one(c[1], T, white);
-    o[0] = tone_one(c[2], T, white);
-    // the row's padding bytes are zero (the caller's buffer may hold anything)
-    if (x == W - 1)
-      for (int64_t b = 3 * static_cast<int64_t>(W); b < stride_b; ++b) out[y * stride_b + b] = 0;
+    // one copy of the exact form, in a loop: unrolled into the twelve channels
+    // it overflows the instruction cache (22 us)
+    for (; ask; ask &= ask - 1) {
+      int const at = __ffs(static_cast<int>(ask)) - 1, k = at / 3, j = at - 3 * k;
+      const float *f = film + 3 * (y * W + x + k);
+      float c[3];
+      tone_channels(T, f[0], f[1], f[2], c);
+      uint32_t const byte = tone_exact(j == 0 ? c[2] : (j == 1 ? c[1] : c[0]), T, white);
+      uint32_t const shift = 8 * (at & 3);
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        if (q == at >> 2) w[q] = (w[q] & ~(0xffu << shift)) | (byte << shift);
+    }
+    // the group's words: all three, or (the row's end) those that hold its
+    // 3 m bytes, whose rest is the padding
+    uint8_t *const o = out + y * stride_b + 3 * x;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      if (4 * k >= 3 * m) break;
+      if (words) {
+        reinterpret_cast<uint32_t *>(o)[k] = w[k];
+      } else {
+        for (int j = 0; j < 4; ++j) o[4 * k + j] = static_cast<uint8_t>(w[k] >> (8 * j));
+      }
+    }
   }
 }
 
@@ -213,9 +384,10 @@ int xyzgpu_film_encode_rgbe(const float *film, int width, int height, float scal
   clear_error();
   if (!film || !out || width <= 0 || height <= 0 || !std::isfinite(scale))
     return set_error(XYZGPU_E_INVALID, "film_encode_rgbe: bad argument");
-  int64_t const n = static_cast<int64_t>(width) * height;
+  int64_t const n = (static_cast<int64_t>(width) + 3) / 4 * height;
   k_film_rgbe<<<film_grid(n), kFilmThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      film, width, height, scale, xyze != 0, reinterpret_cast<uchar4 *>(out));
+      film, width, height, scale, xyze != 0, aligned(film, 16) && aligned(out, 16) && width % 4 == 0,
+      reinterpret_cast<uchar4 *>(out));
   XYZ_CUDA_TRY(cudaGetLastError());
   return XYZGPU_OK;
 }
@@ -264,10 +436,12 @@ int xyzgpu_film_tonemap(const float *film, int width, int height, const xyzgpu_t
   ToneArgs T{tp->scale, tp->exposure, tp->white, tp->src_gamma / tp->dst_gamma, tp->op, tp->rgb != 0, nullptr};
   if (need_white) {
     XYZ_CUDA_TRY(cudaMemsetAsync(scratch_white, 0, sizeof(unsigned int), st));
-    k_film_max_luminance<<<film_grid(n), kFilmThreads, 0, st>>>(film, n, tp->scale, tp->rgb != 0, scratch_white);
+    k_film_max_luminance<<<std::min(film_grid((n + 3) / 4), 8 * device_sms()), kFilmThreads, 0, st>>>(film, n, tp->scale, tp->rgb != 0,
+                                                                          aligned(film, 16), scratch_white);
     T.white_bits = scratch_white;
   }
-  k_film_tonemap<<<film_grid(n), kFilmThreads, 0, st>>>(film, width, height, T, out);
+  k_film_tonemap<<<film_grid((static_cast<int64_t>(width) + 3) / 4 * height), kFilmThreads, 0, st>>>(
+      film, width, height, T, aligned(film, 16) && width % 4 == 0, aligned(out, 4), out);
   XYZ_CUDA_TRY(cudaGetLastError());
   return XYZGPU_OK;
 }
