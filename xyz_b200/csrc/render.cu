@@ -21,6 +21,20 @@ constexpr int64_t kMaxGuidedWave = int64_t{1} << 23;
 struct Grids {
   int raygen, trace_e, trace_s, trace_s_adj, trace_s_guide, trace_s_imp;
   int shade, shade_adj, shade_guide, shade_sp, shade_imp, film;
+  // No larger than waves of `paths` paths can use: a queue is never longer, and
+  // CTAs without work still cost their launch (a trace of one ray: 5.0 us with
+  // the full grid, 3.8 with one CTA).  Traces get a CTA per 32 rays (8 a warp,
+  // see trace_wide), the shading kernels a thread per path.  A 64 x 64 preview
+  // of 15 bounces: traces 540 -> 414 us, shading 114 -> 110.
+  Grids for_paths(int64_t paths) const {
+    Grids g = *this;
+    auto lower = [paths](int &grid, int per_cta) {
+      grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(grid, (paths + per_cta - 1) / per_cta)));
+    };
+    for (int *t : {&g.trace_e, &g.trace_s, &g.trace_s_adj, &g.trace_s_guide, &g.trace_s_imp}) lower(*t, kRaysPerCta);
+    for (int *t : {&g.shade, &g.shade_adj, &g.shade_guide, &g.shade_sp, &g.shade_imp}) lower(*t, kThreads);
+    return g;
+  }
 };
 
 Grids wave_grids(int device) {
@@ -246,7 +260,7 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
     }
   } ltot_guard{ltot, st}, hit_guard{hit_cache, st}, vis_guard{vis_cache, st};
 
-  Grids const G = wave_grids(s.device);
+  Grids const G = wave_grids(s.device).for_paths(std::min<int64_t>(cap, std::max<int64_t>(1, npix_total * rp.spp)));
   int const prof = rp.profile;
   bool const spectral = rp.spectral != XYZGPU_SPECTRAL_OFF;
   bool const timing = prof == XYZGPU_PROFILE_TIMING;

@@ -5,6 +5,8 @@
 // calls walk the kd-tree with trace_persistent): rays are taken from a global
 // counter as lanes free up, so long and short rays balance across lanes and SMs.  Rays are read as two 16-byte vectors and
 // hits written as one.
+#include <algorithm>
+
 #include "scene.h"
 #include "traverse.cuh"
 
@@ -98,8 +100,8 @@ int trace_api_launch(SceneImpl &s, const float *rays, int n, float *hits, cudaSt
     counters->tri_tests = c[3];
     counters->hits = c[4];
   } else {
-    k_trace_api<false><<<grid_for<false>(s.device), kTraceThreads, 0, st>>>(s.dev, r4, n, h4, s.d_fetch,
-                                                                          nullptr);
+    int const grid = std::min(grid_for<false>(s.device), (n + kRaysPerCta - 1) / kRaysPerCta);
+    k_trace_api<false><<<grid, kTraceThreads, 0, st>>>(s.dev, r4, n, h4, s.d_fetch, nullptr);
     XYZ_CUDA_TRY(cudaGetLastError());
   }
   return XYZGPU_OK;

@@ -333,6 +333,9 @@ constexpr int kWideWait = 12;
 constexpr int kWideStep = 8;
 constexpr int kWideRefill = 12;
 
+// Rays a CTA of four warps needs to be worth launching: eight a warp.
+constexpr int kRaysPerCta = 32;
+
 // A lane holds one ray through three states: under way (live), finished with
 // its answer still in registers, and empty.  Answers are written and new rays
 // taken together, once enough lanes are not under way, so that neither runs
@@ -342,7 +345,12 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
   constexpr bool kTarget = SinkHasTarget<Sink>::value;
   int const lane = threadIdx.x & 31;
   unsigned const lanes_below = (1u << lane) - 1u;
-  bool exhausted = false;
+  // short queues: fewer lanes per warp, so that all warps have a share and a
+  // warp's rays wait for fewer others
+  int const warps = (gridDim.x * blockDim.x) >> 5;
+  int const width = min(32, max(1, (n + warps - 1) / warps));
+  int const refill_at = width < 32 ? 0 : 32 - kWideRefill;
+  bool exhausted = lane >= width;
   const DevScene *lane_scene = &S;
   for (;;) {
     int n_list = 0;  // entries of the warp's list (the same on every lane)
@@ -360,7 +368,7 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
     uint2 stack[kWideStack];
     for (;;) {
       unsigned under_way = __ballot_sync(0xffffffffu, live);
-      if (__popc(under_way) <= 32 - kWideRefill) {
+      if (__popc(under_way) <= refill_at) {
         int retry = -1;
         if (ray >= 0 && !live) {
           if (risky && h.id >= 0)
