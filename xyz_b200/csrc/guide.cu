@@ -91,8 +91,8 @@ struct __align__(128) GuideSmem {
   uint8_t x[kRows * kIn * 2];
   uint8_t h[4][kRows * kW * 2];
   uint8_t d[2][kRows * kW * 2];
-  float db[kLayers][kW];
-  uint64_t mbar;
+  float db[kGuideThreads / 32][kLayers][kW];  // bias gradients, one copy per warp
+  uint64_t mbar[2];
   uint32_t tmem;
   int abort;
 };
@@ -103,6 +103,14 @@ struct GuideDev {
   float lo[3], inv_ext[3];  // position normalisation: s = (p - lo) * inv_ext
   int *err;
 };
+
+// A wait that gave up is reported in a word of page-locked host memory, which
+// the host reads after the stream has finished: no copy and no clearing
+// launch per call (a cleared word stays clear until an error sets it).
+__device__ __forceinline__ void raise_error(const GuideDev &G) {
+  *const_cast<volatile int *>(G.err) = 1;
+  __threadfence_system();
+}
 
 // ---------------------------------------------------------------- encoding
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
@@ -392,24 +400,30 @@ __device__ __forceinline__ bool grad_rows(const GradArgs &A, const float *&rec, 
 }
 
 // ------------------------------------------------------------- kernels
-// Copies the packed weight image (weights, ones tile, bias tiles) into shared
-// memory: 4,480 independent 16-byte loads, several in flight per thread.
-__device__ void load_weights(WeightsSmem &wt, const GuideDev &G) {
-  const uint4 *src = reinterpret_cast<const uint4 *>(G.wblk);
-  uint4 *dst = reinterpret_cast<uint4 *>(&wt);
-#pragma unroll 4
-  for (int i = threadIdx.x; i < static_cast<int>(kWImageBytes / 16); i += blockDim.x) dst[i] = __ldg(&src[i]);
-}
-
-// mbarriers (count 1) and `ncols` TMEM columns for the CTA.
-__device__ void setup(uint64_t *mbar, int nbar, uint32_t *tmem_slot, uint32_t ncols) {
-  if (threadIdx.x == 0)
-    for (int i = 0; i < nbar; ++i) tc::mbar_init(tc::smem_addr(&mbar[i]), 1);
+// mbarriers (count 1; mbar[nbar] is the weights') and `ncols` TMEM columns for
+// the CTA, and the copy of the packed weight image (weights, ones tile, bias
+// tiles: 71,680 bytes) into shared memory.  The copy is one asynchronous bulk
+// load that runs while the rows are read and encoded; await_weights before the
+// first MMA.  (Loaded by the threads it took 5 us before any row.)
+__device__ void setup(WeightsSmem &wt, const GuideDev &G, uint64_t *mbar, int nbar, uint32_t *tmem_slot, uint32_t ncols) {
+  if (threadIdx.x == 0) {
+    for (int i = 0; i <= nbar; ++i) tc::mbar_init(tc::smem_addr(&mbar[i]), 1);
+    tc::fence_smem_to_async();  // the initialised barriers, for the copy
+    tc::bulk_load(tc::smem_addr(&wt), G.wblk, kWImageBytes, tc::smem_addr(&mbar[nbar]));
+  }
   if (threadIdx.x < 32) tc::tmem_alloc(tmem_slot, ncols);
-  tc::fence_smem_to_async();  // the weights every thread stored, for every group's MMAs
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
+}
+
+// Every thread waits for the weights; false (uniformly over the CTA) if any
+// gave up.  Each kernel calls it once before it ends: the copy must not outlive
+// its shared memory (after a timeout it gets one more bounded wait).
+__device__ bool await_weights(uint64_t *mbar) {
+  bool const ok = tc::mbar_wait(tc::smem_addr(mbar), 0, kWaitLimit);
+  if (!ok) tc::mbar_wait(tc::smem_addr(mbar), 0, kWaitLimit);
+  return __syncthreads_or(ok ? 0 : 1) == 0;
 }
 
 // Frees TMEM.  A group whose wait timed out first gives its MMAs still in
@@ -434,7 +448,7 @@ constexpr int kInferThreads = kGroups * kRows;
 struct __align__(128) InferSmem {
   WeightsSmem wt;
   uint8_t x[kGroups][2 * kHBytes];
-  uint64_t mbar[kGroups];
+  uint64_t mbar[kGroups + 1];
   uint32_t tmem;
 };
 
@@ -506,33 +520,79 @@ __device__ bool forward_infer(const WeightsSmem &wt, const GuideDev &G, Tile &c,
   return true;
 }
 
-// Raw outputs of n points (features: n x 6 = position, normal).
+// Raw outputs of n points (features: n x 6 = position, normal).  Tiles go to
+// the SMs first and to a CTA's groups second, so that up to 148 tiles run side
+// by side; a row's 64 outputs are written in whole 32-byte sectors (wide: the
+// buffer is 32-byte aligned).  16,384 points: four tiles to a CTA and single
+// floats 42 us, this form 9.0.
 __global__ void __launch_bounds__(kInferThreads, 1)
-    k_guide_forward(const __grid_constant__ GuideDev G, const float *__restrict__ feat, int n, float *__restrict__ out) {
+    k_guide_forward(const __grid_constant__ GuideDev G, const float *__restrict__ feat, int n, float *__restrict__ out,
+                    int wide) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   InferSmem &S = *reinterpret_cast<InferSmem *>(smem_raw);
-  load_weights(S.wt, G);
-  setup(S.mbar, kGroups, &S.tmem, 256);
+  setup(S.wt, G, S.mbar, kGroups, &S.tmem, 256);
   int const gi = threadIdx.x >> 7;
   Tile c = infer_tile(S, gi);
   uint32_t phase = 0;
   bool aborted = false;
-  int const ntiles = (n + kRows - 1) / kRows;
-  for (int tile = kGroups * blockIdx.x + gi; tile < ntiles; tile += kGroups * gridDim.x) {
+  bool const loaded = await_weights(&S.mbar[kGroups]);
+  if (!loaded && threadIdx.x == 0) raise_error(G);
+  int const ntiles = loaded ? (n + kRows - 1) / kRows : 0;
+  for (int tile = blockIdx.x + gi * gridDim.x; tile < ntiles; tile += kGroups * gridDim.x) {
     int const row = tile * kRows + c.t;
     float f[6] = {0, 0, 0, 0, 0, 1};
     if (row < n)
       for (int k = 0; k < 6; ++k) f[k] = feat[6 * static_cast<int64_t>(row) + k];
     float o[kW];
     if (!forward_infer(S.wt, G, c, phase, f, o)) {
-      if (c.t == 0) atomicExch(G.err, 1);
+      if (c.t == 0) raise_error(G);
       aborted = true;
       break;
     }
-    if (row < n)
-      for (int j = 0; j < kW; ++j) out[kW * static_cast<int64_t>(row) + j] = o[j];
+    if (row < n) {
+      float *const dst = out + kW * static_cast<int64_t>(row);
+      if (wide) {
+#pragma unroll
+        for (int j = 0; j < kW; j += 8)
+          asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + j), "f"(o[j]), "f"(o[j + 1]),
+                       "f"(o[j + 2]), "f"(o[j + 3]), "f"(o[j + 4]), "f"(o[j + 5]), "f"(o[j + 6]), "f"(o[j + 7])
+                       : "memory");
+      } else {
+#pragma unroll
+        for (int j = 0; j < kW; ++j) dst[j] = o[j];
+      }
+    }
   }
   teardown(S.tmem, 256, aborted, c.mbar, phase);
+}
+
+// Adds the column sums of a blocked bf16 matrix [128][64] to the warp's dst[64]
+// (each warp sums its 32 rows).  A thread reads one core matrix (8 rows of 8
+// columns, 16 bytes a row, starting at a row of its own so that a quarter warp
+// covers all banks); the warp's four row groups meet by shuffles.
+__device__ void add_column_sums(const uint8_t *d, float *dst) {
+  int const t = threadIdx.x, lane = t & 31, cg = t & 7;
+  const uint8_t *const core = d + (t >> 3) * (kW / 8) * 128 + cg * 128;
+  float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    uint4 const q = *reinterpret_cast<const uint4 *>(core + ((j + t) & 7) * 16);
+    uint32_t const w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      s[2 * k] += __uint_as_float(w[k] << 16);
+      s[2 * k + 1] += __uint_as_float(w[k] & 0xffff0000u);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    s[k] += __shfl_xor_sync(0xffffffffu, s[k], 8);
+    s[k] += __shfl_xor_sync(0xffffffffu, s[k], 16);
+  }
+  if (lane < 8) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) dst[cg * 8 + k] += s[k];
+  }
 }
 
 // Gradient of sum over records of -w * log p(dir) * scale, added to grad
@@ -546,14 +606,13 @@ __global__ void __launch_bounds__(kGuideThreads, 1)
   float *__restrict__ grad = A.grad;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   GuideSmem &S = *reinterpret_cast<GuideSmem *>(smem_raw);
-  load_weights(S.wt, G);
-  for (int i = threadIdx.x; i < kLayers * kW; i += blockDim.x) (&S.db[0][0])[i] = 0.0f;
-  setup(&S.mbar, 1, &S.tmem, 512);
+  for (int i = threadIdx.x; i < kGuideThreads / 32 * kLayers * kW; i += blockDim.x) (&S.db[0][0][0])[i] = 0.0f;
+  setup(S.wt, G, S.mbar, 1, &S.tmem, 512);
   Tile c;
   c.x = S.x;
   c.h = S.h[0];
   c.tmem = S.tmem;
-  c.mbar = tc::smem_addr(&S.mbar);
+  c.mbar = tc::smem_addr(&S.mbar[0]);
   c.bar = 0;
   c.t = threadIdx.x;
   uint32_t phase = 0;
@@ -572,6 +631,10 @@ __global__ void __launch_bounds__(kGuideThreads, 1)
       wgt = q[9];
     }
     encode_row(S.x, r, G, f);
+    if (first && !await_weights(&S.mbar[1])) {
+      ok = false;
+      break;
+    }
     float o[kW];
     if (!forward(S.wt, c, phase, true, o)) {
       ok = false;
@@ -589,12 +652,6 @@ __global__ void __launch_bounds__(kGuideThreads, 1)
     int dbuf = 0;
     for (int l = kLayers - 1; l >= 0 && ok; --l) {
       publish(0);
-      if (r < kW) {  // bias gradient: column sums of the (bf16) delta
-        float acc = 0.0f;
-        for (int m = 0; m < kRows; ++m)
-          acc += __bfloat162float(*reinterpret_cast<const __nv_bfloat16 *>(S.d[dbuf] + tc::blocked_offset(m, r, kW)));
-        S.db[l][r] += acc;
-      }
       const uint8_t *act = l == 0 ? S.x : S.h[l - 1];
       int const K = layer_in(l);
       if (threadIdx.x == 0) {
@@ -615,6 +672,7 @@ __global__ void __launch_bounds__(kGuideThreads, 1)
         }
         tc::mma_commit(c.mbar);
       }
+      add_column_sums(S.d[dbuf], S.db[threadIdx.x >> 5][l]);  // bias gradient, while the MMAs run
       if (!await_mma(c, phase)) {
         ok = false;
         break;
@@ -640,27 +698,67 @@ __global__ void __launch_bounds__(kGuideThreads, 1)
     }
     first = false;
   }
-  if (!ok && threadIdx.x == 0) atomicExch(G.err, 1);
-  // weight gradients out of TMEM (M = 64 layout) and bias gradients
+  if (first && ok) ok = await_weights(&S.mbar[1]);  // a CTA without rows
+  if (!ok && threadIdx.x == 0) raise_error(G);
+  // weight gradients out of TMEM (M = 64 layout) into the buffers that are free
+  // now, as [K][64] of floats in the parameters' order: layer 0 fills S.x, layers
+  // 1..4 fill S.h
+  static_assert(sizeof(S.x) == kIn * kW * 4 && sizeof(S.h) == 4 * kW * kW * 4, "gradient staging");
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  if (ok && !first) {
+  bool const add = ok && !first;
+  if (add) {
     int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t const lane_base = static_cast<uint32_t>(warp * 32) << 16;
     int const nrow = warp * 16 + lane;  // output unit of this lane (lanes < 16)
     for (int l = 0; l < kLayers; ++l) {
       int const K = layer_in(l);
-      for (int q = 0; q < K; q += 16) {
-        float v[16];
+      float *const dst = l == 0 ? reinterpret_cast<float *>(S.x) : reinterpret_cast<float *>(S.h[l - 1]);
+#pragma unroll 2
+      for (int q = 0; q < K; q += 32) {
+        float v[32];
         tc::tmem_ld16(S.tmem + lane_base + dw_col(l) + q, v);
+        tc::tmem_ld16(S.tmem + lane_base + dw_col(l) + q + 16, v + 16);
         tc::tmem_wait_ld();
-        if (lane < 16)
-          for (int t = 0; t < 16; ++t) atomicAdd(&grad[param_w(l) + (q + t) * kW + nrow], v[t]);
+        if (lane < 16) {
+#pragma unroll
+          for (int t = 0; t < 32; ++t) dst[(q + t) * kW + nrow] = v[t];
+        }
       }
     }
-    for (int i = threadIdx.x; i < kLayers * kW; i += blockDim.x)
-      atomicAdd(&grad[param_b(i / kW) + i % kW], (&S.db[0][0])[i]);
+  }
+  __syncthreads();
+  if (add) {
+    // one reduction per four parameters where the buffer allows it
+    bool const vec = reinterpret_cast<uintptr_t>(grad) % 16 == 0;
+    auto add4 = [&](float *at, float4 v) {
+      if (vec) {
+        atomicAdd(reinterpret_cast<float4 *>(at), v);
+      } else {
+        atomicAdd(at, v.x);
+        atomicAdd(at + 1, v.y);
+        atomicAdd(at + 2, v.z);
+        atomicAdd(at + 3, v.w);
+      }
+    };
+    // (the order does not matter: every sum meets 128 CTAs' sums to its address,
+    // 8.6 us at 16,384 rows from the same place or from one of its own; single
+    // floats 13.5)
+    for (int l = 0; l < kLayers; ++l) {
+      const float4 *const src = reinterpret_cast<const float4 *>(l == 0 ? S.x : S.h[l - 1]);
+      for (int i = threadIdx.x; i < layer_in(l) * kW / 4; i += kGuideThreads) add4(grad + param_w(l) + 4 * i, src[i]);
+    }
+    for (int i = threadIdx.x; i < kLayers * kW / 4; i += kGuideThreads) {
+      int const l = i / (kW / 4), j = 4 * (i % (kW / 4));
+      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+      for (int w = 0; w < kGuideThreads / 32; ++w) {
+        float4 const x = *reinterpret_cast<const float4 *>(&S.db[w][l][j]);
+        v = make_float4(v.x + x.x, v.y + x.y, v.z + x.z, v.w + x.w);
+      }
+      add4(grad + param_b(l) + j, v);
+    }
   }
   teardown(S.tmem, 512, !ok, c.mbar, phase);
 }
@@ -727,8 +825,7 @@ __device__ void infer_features(const InferArgs &I, const InferRow &r, float f[6]
 __global__ void __launch_bounds__(kInferThreads, 1) k_guide_infer(const __grid_constant__ GuideDev G, InferArgs I) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   InferSmem &S = *reinterpret_cast<InferSmem *>(smem_raw);
-  load_weights(S.wt, G);
-  setup(S.mbar, kGroups, &S.tmem, 256);
+  setup(S.wt, G, S.mbar, kGroups, &S.tmem, 256);
   int const gi = threadIdx.x >> 7;
   Tile c = infer_tile(S, gi);
   uint32_t phase = 0;
@@ -745,7 +842,9 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_guide_infer(const __grid_c
   cur.h = valid(tile) ? I.hits[row_of(tile)] : miss_hit();
   infer_gather(I, row_of(tile), cur);
   nxt.h = valid(tile + step) ? I.hits[row_of(tile + step)] : miss_hit();
-  for (; tile < ntiles; tile += step) {
+  bool const loaded = await_weights(&S.mbar[kGroups]);
+  if (!loaded && threadIdx.x == 0) raise_error(G);
+  for (; loaded && tile < ntiles; tile += step) {
     int const i = row_of(tile);
     float f[6];
     infer_features(I, cur, f);
@@ -753,7 +852,7 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_guide_infer(const __grid_c
     float4 const h2 = valid(tile + 2 * step) ? I.hits[row_of(tile + 2 * step)] : miss_hit();
     float o[kW];
     if (!forward_infer(S.wt, G, c, phase, f, o)) {
-      if (c.t == 0) atomicExch(G.err, 1);
+      if (c.t == 0) raise_error(G);
       aborted = true;
       break;
     }
@@ -937,7 +1036,7 @@ struct GuideImpl {
   SceneImpl *scene = nullptr;
   float *d_params = nullptr, *d_grad = nullptr, *d_m = nullptr, *d_v = nullptr;
   uint8_t *d_wblk = nullptr;
-  int *d_err = nullptr;
+  int *h_err = nullptr;  // page-locked, mapped: set by a kernel whose wait gave up
   TrainState *d_ts = nullptr;  // Adam step, batch offset, row counts (device)
   float lo[3] = {0, 0, 0}, inv_ext[3] = {1, 1, 1};
   // guided-render buffers
@@ -967,7 +1066,7 @@ GuideDev guide_dev(const GuideImpl &g) {
     d.lo[k] = g.lo[k];
     d.inv_ext[k] = g.inv_ext[k];
   }
-  d.err = g.d_err;
+  d.err = g.h_err;
   return d;
 }
 
@@ -992,10 +1091,12 @@ double rand_sym(uint64_t &s) {
 }
 
 int check_err(GuideImpl &g, cudaStream_t st, const char *who) {
-  int e = 0;
-  XYZ_CUDA_TRY(cudaMemcpyAsync(&e, g.d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
   XYZ_CUDA_TRY(cudaStreamSynchronize(st));
-  if (e) return set_error(XYZGPU_E_CUDA, "%s: a tensor-core wait timed out", who);
+  volatile int *const e = g.h_err;
+  if (*e) {
+    *e = 0;
+    return set_error(XYZGPU_E_CUDA, "%s: a tensor-core wait timed out", who);
+  }
   return XYZGPU_OK;
 }
 
@@ -1009,8 +1110,8 @@ int guide_forward_launch(GuideImpl &g, const float *feat, int n, float *out, cud
     attr = true;
   }
   if (n <= 0) return XYZGPU_OK;
-  int const grid = std::max(1, std::min((n + kGroups * kRows - 1) / (kGroups * kRows), sm_count(g.device)));
-  k_guide_forward<<<grid, kInferThreads, sizeof(InferSmem), st>>>(guide_dev(g), feat, n, out);
+  k_guide_forward<<<grid_for(g.device, n), kInferThreads, sizeof(InferSmem), st>>>(
+      guide_dev(g), feat, n, out, reinterpret_cast<uintptr_t>(out) % 32 == 0);
   XYZ_CUDA_TRY(cudaGetLastError());
   return XYZGPU_OK;
 }
@@ -1181,7 +1282,7 @@ void xyzgpu_guide_destroy(xyzgpu_guide h) {
   cudaFree(g.d_m);
   cudaFree(g.d_v);
   cudaFree(g.d_wblk);
-  cudaFree(g.d_err);
+  cudaFreeHost(g.h_err);
   cudaFree(g.d_mix);
   cudaFree(g.d_rec);
   cudaFree(g.d_train);
@@ -1228,9 +1329,10 @@ int xyzgpu_guide_create(xyzgpu_scene scene, const xyzgpu_guide_config *cfg, xyzg
       cudaMalloc(reinterpret_cast<void **>(&g.d_m), kParams * sizeof(float)) != cudaSuccess ||
       cudaMalloc(reinterpret_cast<void **>(&g.d_v), kParams * sizeof(float)) != cudaSuccess ||
       cudaMalloc(reinterpret_cast<void **>(&g.d_wblk), kWImageBytes) != cudaSuccess ||
-      cudaMalloc(reinterpret_cast<void **>(&g.d_err), sizeof(int)) != cudaSuccess ||
+      cudaHostAlloc(reinterpret_cast<void **>(&g.h_err), sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess ||
       cudaMalloc(reinterpret_cast<void **>(&g.d_ts), sizeof(TrainState)) != cudaSuccess)
     return fail(set_error(XYZGPU_E_NOMEM, "guide_create: device allocation failed"));
+  *g.h_err = 0;
   // He-uniform hidden layers, a small output layer (near-uniform mixture at
   // the start), zero biases
   std::vector<float> p(kParams, 0.0f);
@@ -1243,7 +1345,6 @@ int xyzgpu_guide_create(xyzgpu_scene scene, const xyzgpu_guide_config *cfg, xyzg
       cudaMemset(g.d_grad, 0, kParams * sizeof(float)) != cudaSuccess ||
       cudaMemset(g.d_m, 0, kParams * sizeof(float)) != cudaSuccess ||
       cudaMemset(g.d_v, 0, kParams * sizeof(float)) != cudaSuccess ||
-      cudaMemset(g.d_err, 0, sizeof(int)) != cudaSuccess ||
       cudaMemset(g.d_ts, 0, sizeof(TrainState)) != cudaSuccess)
     return fail(set_error(XYZGPU_E_CUDA, "guide_create: initialisation failed"));
   int rc = pack(g, nullptr);
@@ -1284,7 +1385,6 @@ int xyzgpu_guide_forward(xyzgpu_guide h, const float *features, int n, float *ou
   GuideImpl &g = h->g;
   cudaStream_t const st = static_cast<cudaStream_t>(stream);
   XYZ_CUDA_TRY(cudaSetDevice(g.device));
-  XYZ_CUDA_TRY(cudaMemsetAsync(g.d_err, 0, sizeof(int), st));
   int const rc = guide_forward_launch(g, features, n, out, st);
   if (rc) return rc;
   return check_err(g, st, "guide_forward");
@@ -1297,7 +1397,6 @@ int xyzgpu_guide_gradient(xyzgpu_guide h, const float *records, int n, float sca
   GuideImpl &g = h->g;
   cudaStream_t const st = static_cast<cudaStream_t>(stream);
   XYZ_CUDA_TRY(cudaSetDevice(g.device));
-  XYZ_CUDA_TRY(cudaMemsetAsync(g.d_err, 0, sizeof(int), st));
   int const rc = guide_gradient_launch(g, records, n, scale, grad, st);
   if (rc) return rc;
   return check_err(g, st, "guide_gradient");
@@ -1329,7 +1428,6 @@ int xyzgpu_render_guided(xyzgpu_guide h, const xyzgpu_camera *cam, const xyzgpu_
     return set_error(XYZGPU_E_INVALID, "render_guided: scenes with mirror or metal materials are not guided");
   cudaStream_t const st = static_cast<cudaStream_t>(stream);
   XYZ_CUDA_TRY(cudaSetDevice(g.device));
-  XYZ_CUDA_TRY(cudaMemsetAsync(g.d_err, 0, sizeof(int), st));
   GuideHooks hooks{&g, train != 0};
   int const rc = render_launch(*g.scene, *cam, *rp, film, st, nullptr, &hooks);
   if (rc) return rc;
@@ -1354,7 +1452,6 @@ int xyzgpu_guide_train_step(xyzgpu_guide h, const float *records, int n, void *s
   GuideImpl &g = h->g;
   cudaStream_t const st = static_cast<cudaStream_t>(stream);
   XYZ_CUDA_TRY(cudaSetDevice(g.device));
-  XYZ_CUDA_TRY(cudaMemsetAsync(g.d_err, 0, sizeof(int), st));
   int rc = guide_gradient_launch(g, records, n, 1.0f / static_cast<float>(n), g.d_grad, st);
   if (rc) return rc;
   rc = adam_pack_launch(g, guide_dev(g), 0, 0, 0, st);

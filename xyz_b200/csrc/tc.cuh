@@ -103,6 +103,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, uint32
 }
 
 // TMEM allocation: one whole warp; the base address is written to *slot.
+// Asynchronous copy of `bytes` (a multiple of 16, both addresses 16-byte
+// aligned) from global to shared memory, issued by one thread; it completes on
+// the mbarrier, which this call tells to expect the bytes (one arrival).
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t mbar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
+  asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(mbar)
+               : "memory");
+}
+
 __device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(slot)),
                "r"(ncols)
