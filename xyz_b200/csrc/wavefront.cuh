@@ -763,13 +763,52 @@ XYZ_DEV int32_t shading_frame(const DevScene &S, int32_t tri, int back, float f,
   return __float_as_int(g4.w);
 }
 
+// The hits of a queue, 32 at a time: a warp reads the hit codes of its blocks of
+// 32 entries and keeps the indices of the entries that hit in a ring in shared
+// memory, so that the shading code runs with full warps however many rays
+// miss (two of three second rays of an open scene).  next() returns this
+// lane's entry, or -1 beyond the last ones; done when `any` is false.  All lanes
+// of the warp call it.
+struct HitRing {
+  int32_t *ring;  // 64 entries of this warp
+  int n, base, stride, held, head;
+  XYZ_DEV HitRing(int32_t *r, int n_) : ring(r), n(n_), held(0), head(0) {
+    base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32;
+    stride = ((gridDim.x * blockDim.x) >> 5) * 32;
+  }
+  // code_of(i): the hit code of entry i (negative: no hit)
+  template <class CodeOf>
+  XYZ_DEV int next(CodeOf code_of, bool *any) {
+    int const lane = threadIdx.x & 31;
+    while (held < 32 && base < n) {
+      int const i = base + lane;
+      bool const hit = i < n && code_of(i) >= 0;
+      unsigned const m = __ballot_sync(0xffffffffu, hit);
+      if (hit) ring[(head + held + __popc(m & ((1u << lane) - 1u))) & 63] = i;
+      held += __popc(m);
+      base += stride;
+    }
+    __syncwarp();
+    int const take = min(held, 32);
+    int const i = lane < take ? ring[(head + lane) & 63] : -1;
+    __syncwarp();
+    head += take;
+    held -= take;
+    *any = take > 0;
+    return i;
+  }
+};
+
 // kModeAdjoint: the replay pass of xyzgpu_adjoint (same path, plus gradients).
 // kModeBatch: paths of many scenes (xyzgpu_batch_*).
 // kModeGuided: directions from the learned guide mixed with Lambert sampling.
 // kModeImporton: directions from the light-importance histogram of the vertex
 // (the reference's importance-driven tracer).
+// Six CTAs per SM (80 registers): with full warps the kernel waits for its gathers
+// (1M-triangle frame, 10 bounces: 9.34 ms with a warp per 32 queue entries, with
+// the ring 6.78 at five CTAs, 6.62 at six, 6.64 at seven, 7.74 at eight).
 template <int kMode>
-__global__ void __launch_bounds__(kThreads, kMode == kModeGuided ? 5 : 0) k_shade(WaveArgs A, int b) {
+__global__ void __launch_bounds__(kThreads, kMode == kModeGuided ? 5 : 6) k_shade(WaveArgs A, int b) {
   constexpr bool kAdj = kMode == kModeAdjoint;
   constexpr bool kBatch = kMode == kModeBatch;
   constexpr bool kGuide = kMode == kModeGuided;
@@ -780,13 +819,24 @@ __global__ void __launch_bounds__(kThreads, kMode == kModeGuided ? 5 : 0) k_shad
   if constexpr (kBatch) b = A.cursor->bounce;
   int32_t *const cnt = A.counts + b * kCountStride;
   int32_t *const cnt_next = A.counts + (b + 1) * kCountStride;
-  int const n = cnt[kCExt];
-  int const lane = threadIdx.x & 31;
   int const qi = b & 1, qo = qi ^ 1;
-  int const warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  int const nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int base = warp * 32; base < n; base += nwarps * 32) {
-    int const i = base + lane;
+  __shared__ int32_t s_ring[kThreads / 32][64];
+  HitRing hits(s_ring[threadIdx.x >> 5], cnt[kCExt]);
+  // the adjoint's primal pass records every entry's hit, its replay reads it
+  auto code_of = [&](int i) -> int32_t {
+    if (kAdj && A.hit_cache)
+      return __float_as_int(A.hit_cache[static_cast<int64_t>(A.q_slot[qi][i]) * A.cache_stride + b].w);
+    if (kMode == kModePlain && A.hit_cache) {
+      float4 const h = A.hits[i];
+      A.hit_cache[static_cast<int64_t>(A.q_slot[qi][i]) * A.cache_stride + b] = h;
+      return __float_as_int(h.w);
+    }
+    return __float_as_int(A.hits[i].w);
+  };
+  for (;;) {
+    bool any;
+    int const i = hits.next(code_of, &any);
+    if (!any) break;
     bool push_ext = false, push_sh = false;
     int32_t slot = 0, tri = 0;
     f3 pos{}, dir{}, lpos{}, vin{}, pbv{};
@@ -802,14 +852,13 @@ __global__ void __launch_bounds__(kThreads, kMode == kModeGuided ? 5 : 0) k_shad
     // alone, and the mixture buffer is not read
     bool const use_guide = kGuide && A.guide_alpha > 0.0f;
     GuideMix M;
-    if (use_guide && i < n) load_mix(A.mix + 40 * static_cast<int64_t>(i), M);
-    if (i < n) {
+    if (use_guide && i >= 0) load_mix(A.mix + 40 * static_cast<int64_t>(i), M);
+    if (i >= 0) {
       slot = A.q_slot[qi][i];
-      int64_t const cache_at = static_cast<int64_t>(slot) * A.cache_stride + b;
-      float4 const h = (kAdj && A.hit_cache) ? A.hit_cache[cache_at] : A.hits[i];
-      if (kMode == kModePlain && A.hit_cache) A.hit_cache[cache_at] = h;
+      float4 const h =
+          (kAdj && A.hit_cache) ? A.hit_cache[static_cast<int64_t>(slot) * A.cache_stride + b] : A.hits[i];
       int32_t const code = __float_as_int(h.w);
-      if (code >= 0) {
+      {
         tri = code >> 1;
         int const back = code & 1;
         float4 const o4 = A.q_o[qi][i], d4 = A.q_d[qi][i];
@@ -1212,28 +1261,28 @@ XYZ_DEV float4 spd_values(const WaveArgs &A, const float *spd, const HeroSet &hs
 
 XYZ_DEV float4 mul4(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
 
-__global__ void __launch_bounds__(kThreads) k_shade_spectral(WaveArgs A, int b) {
+__global__ void __launch_bounds__(kThreads, 6) k_shade_spectral(WaveArgs A, int b) {
   int32_t *const cnt = A.counts + b * kCountStride;
   int32_t *const cnt_next = A.counts + (b + 1) * kCountStride;
-  int const n = cnt[kCExt];
-  int const lane = threadIdx.x & 31;
   int const qi = b & 1, qo = qi ^ 1;
-  int const warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  int const nwarps = (gridDim.x * blockDim.x) >> 5;
   DevScene const &S = A.S;
-  for (int base = warp * 32; base < n; base += nwarps * 32) {
-    int const i = base + lane;
+  __shared__ int32_t s_ring[kThreads / 32][64];
+  HitRing hits(s_ring[threadIdx.x >> 5], cnt[kCExt]);
+  for (;;) {
+    bool any;
+    int const i = hits.next([&](int j) { return __float_as_int(A.hits[j].w); }, &any);
+    if (!any) break;
     bool push_ext = false, push_sh = false;
     int32_t slot = 0, tri = 0;
     f3 pos{}, dir{}, lpos{}, vin{};
     float4 pb4{}, beta{};
     float nk2nk3 = 0.0f, fsn_out = 0.0f;
     uint32_t misc = 0;
-    if (i < n) {
+    if (i >= 0) {
       slot = A.q_slot[qi][i];
       float4 const h = A.hits[i];
       int32_t const code = __float_as_int(h.w);
-      if (code >= 0) {
+      {
         tri = code >> 1;
         int const back = code & 1;
         float4 const o4 = A.q_o[qi][i], d4 = A.q_d[qi][i];
