@@ -251,6 +251,17 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
       vis_cache = nullptr;
     }
   }
+  // The emission gradient spread over 256 bytes per material, less where that
+  // would take more than 16 MB; the caller's array if there is no room.
+  float *em_spread = nullptr;
+  int em_stride = 64;
+  int const nm = std::max(1, s.n_materials);
+  while (em_stride > 1 && static_cast<int64_t>(em_stride) * nm > (int64_t{1} << 22)) em_stride /= 2;
+  size_t const em_bytes = static_cast<size_t>(em_stride) * nm * sizeof(float);
+  if (adj && em_stride > 1 && cudaMallocAsync(reinterpret_cast<void **>(&em_spread), em_bytes, st) != cudaSuccess) {
+    cudaGetLastError();
+    em_spread = nullptr;
+  }
   // frees the adjoint's buffers on every return below
   struct FreeAsync {
     void *p;
@@ -258,7 +269,8 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
     ~FreeAsync() {
       if (p) cudaFreeAsync(p, st);
     }
-  } ltot_guard{ltot, st}, hit_guard{hit_cache, st}, vis_guard{vis_cache, st};
+  } ltot_guard{ltot, st}, hit_guard{hit_cache, st}, vis_guard{vis_cache, st}, em_guard{em_spread, st};
+  if (em_spread) XYZ_CUDA_TRY(cudaMemsetAsync(em_spread, 0, em_bytes, st));
 
   Grids const G = wave_grids(s.device).for_paths(std::min<int64_t>(cap, std::max<int64_t>(1, npix_total * rp.spp)));
   int const prof = rp.profile;
@@ -317,7 +329,8 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
     A.ltot = ltot;
     A.dfilm = adj->d_film;
     A.g_alb = adj->g_albedo;
-    A.g_em = adj->g_emission;
+    A.g_em = em_spread ? em_spread : adj->g_emission;
+    A.em_stride = em_spread ? em_stride : 1;
   }
   GuideWave gw;
   if (guide) {
@@ -485,6 +498,11 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
       rc_out.paths += static_cast<uint64_t>(A.npaths);
       rc_out.waves += 1;
     }
+  }
+  if (em_spread) {
+    k_adj_gather<<<(nm + kThreads - 1) / kThreads, kThreads, 0, st>>>(em_spread, em_stride, nm, adj->g_emission);
+    ++launches;
+    XYZ_CUDA_TRY(cudaGetLastError());
   }
   XYZ_CUDA_TRY(cudaEventRecord(sw.done, st));
   sw.last = st;
