@@ -591,6 +591,7 @@ int xyzgpu_scene_create(const xyzgpu_scene_desc *d, const xyzgpu_build_params *b
   v.refs = s->d_refs;
   v.wide = s->d_wide;
   v.wide_tri = s->d_wide_tri;
+  v.n_wide = static_cast<int>(s->n_wide);
   // Lights of zero total area cannot be sampled: next-event estimation is off
   // (the reference would divide by that area, xyz/core/scene.cpp:65).
   v.n_lights = cdf.back() > 0.0f ? s->n_lights : 0;

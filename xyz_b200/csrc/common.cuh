@@ -134,6 +134,7 @@ struct DevScene {
   const uint32_t *wide;     // wide tree (wide.cuh) and its triangle records, or null
   const float4 *wide_tri;
   float wide_reach;         // largest origin coordinate of the rays it serves
+  int n_wide;               // its nodes
   int n_lights;
   float light_area;
   f3 power;

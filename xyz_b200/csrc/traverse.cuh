@@ -280,16 +280,20 @@ XYZ_DEV void trace_persistent(const DevScene &S, int n, int *fetch, Sink &sink, 
 // it, or two hits whose distances differ by less than their rounding.  Such
 // rays are recognised while they are traced (wide_margin: the hit is closer
 // to an edge, or a second accepted hit closer in distance, than the error
-// bound of the test), put into a list of the warp in shared memory, and
-// traced through the kd-tree once the list is full or the queue is empty.
-// Everywhere else a correct traversal of either tree finds the same triangle.
-// About 0.1 to 1 % of the rays take that way (edges of a 1M-triangle mesh).
-// Rays the wide tree cannot serve (wide_usable) take it too.
+// bound of the test).  About 0.1 to 1 % of the rays are (edges of a 1M-triangle
+// mesh).  Where no split plane of the kd-tree passes within the error of the hit
+// point (wide_settled), all these hits lie in the one leaf that holds it, whose
+// triangles the kd loop tests in ascending order: it keeps the nearest, and of
+// equal distances the highest id, which is what this loop keeps.  The rest
+// (1 % of the 1 %), and rays the wide tree cannot serve (wide_usable), go into
+// a list of the warp in shared memory and are traced through the kd-tree once
+// the list is full or the queue is empty.  Everywhere else a correct traversal
+// of either tree finds the same triangle.
 //
 // Why: the kd loop runs at 8 of 32 lanes per instruction and 351 warp
 // instructions per ray, 43 dependent node loads and 16 triangle tests a ray;
 // a wide node costs one round of uniform arithmetic on eight boxes for three
-// 32-byte loads, and a ray needs about nine of them.
+// 32-byte loads, and a ray needs about ten of them.
 constexpr int kWideRetry = 128;  // list entries per warp; 64 + one refill + the lanes under way fit
 constexpr int kWideRetryFull = 64;
 
@@ -302,6 +306,22 @@ XYZ_DEV void wide_margin(float t, float e, float n, float inv_det, float *m, flo
   float const r = (fabsf(t) + e) * fabsf(inv_det) * (1.0f / 1048576.0f);
   *m = r * e;
   *dt = r * n;
+}
+
+// Whether the point at distance t lies in one kd leaf together with every hit
+// within `slack` of it: the descent to its leaf meets no split plane closer
+// than twice the error of the hits (along the ray and across it, for |d| <= 2)
+// plus the rounding of the point itself.
+XYZ_DEV bool wide_settled(const uint2 *__restrict__ nodes, f3 o, f3 d, float t, float slack) {
+  f3 const p = add3(o, scl3(d, t));
+  float const eps = 4.0f * slack + (norm1(o) + norm1(p)) * (1.0f / 2097152.0f);
+  uint2 nd = __ldg(&nodes[0]);
+  while ((nd.y & 3u) != kKdLeafTag) {
+    float const off = comp3(p, static_cast<int>(nd.y & 3u)) - __uint_as_float(nd.x);
+    if (!(fabsf(off) > eps)) return false;
+    nd = __ldg(&nodes[(nd.y >> 2) + (off > 0.0f ? 1u : 0u)]);
+  }
+  return true;
 }
 
 template <class Sink>
@@ -327,11 +347,15 @@ XYZ_DEV void wide_load8(const uint32_t *p, uint32_t *w) {
 // bounces of a 1M-triangle mesh / an indoor room / box stacks (ms): tests
 // as they come, two at a time, 1.50 / 1.39 / 1.34; waiting for 8, 10, 14
 // lanes 1.38 / 1.26 / 1.19, 1.35 / 1.23 / 1.17, 1.38 / 1.20 / 1.15; eight
-// tests at a time 1.43 / 1.26 / 1.22; refill at 8 or 16 idle lanes +-2 %.
+// tests at a time 1.43 / 1.26 / 1.22; refill at 8 or 16 idle lanes +-2 %, but in
+// a room of 36 triangles, whose rays take one node step and a dozen tests, 16
+// keeps the warp's rays together: camera rays and two bounces 0.38 / 0.46 / 0.47
+// ms at 12, 0.38 / 0.41 / 0.44 at 16, 0.36 / 0.41 / 0.44 at 20.
 constexpr int kWideTris = 4;
 constexpr int kWideWait = 12;
 constexpr int kWideStep = 8;
-constexpr int kWideRefill = 12;
+constexpr int kWideRefill = 12, kWideRefillTiny = 16;
+constexpr int kWideTinyNodes = 64;
 
 // Rays a CTA of four warps needs to be worth launching: eight a warp.
 constexpr int kRaysPerCta = 32;
@@ -349,8 +373,9 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
   // warp's rays wait for fewer others
   int const warps = (gridDim.x * blockDim.x) >> 5;
   int const width = min(32, max(1, (n + warps - 1) / warps));
-  int const refill_at = width < 32 ? 0 : 32 - kWideRefill;
+  int const refill_at = width < 32 ? 0 : 32 - ((kBatch || S.n_wide > kWideTinyNodes) ? kWideRefill : kWideRefillTiny);
   bool exhausted = lane >= width;
+  bool kd_only = false;  // the same on every lane
   const DevScene *lane_scene = &S;
   for (;;) {
     int n_list = 0;  // entries of the warp's list (the same on every lane)
@@ -360,8 +385,7 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
     WideRay R{};
     float tmin = 0.0f, tlim = 0.0f;
     RayHit h{};
-    int32_t own = -1;    // target queries: the target
-    bool risky = false;
+    float slack = 0.0f;  // > 0: rounding could decide the answer (wide_settled)
     uint32_t base = 0, group = 0;             // node group: first child, hits (visiting order) << 8 | inner slots
     uint32_t tri_base = 0, tri_valid = 0, tri_hits = 0;
     int sp = 0;
@@ -371,7 +395,8 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
       if (__popc(under_way) <= refill_at) {
         int retry = -1;
         if (ray >= 0 && !live) {
-          if (risky && h.id >= 0)
+          const uint2 *const kd = kBatch ? lane_scene->nodes : S.nodes;
+          if (h.id >= 0 && slack > 0.0f && !wide_settled(kd, R.o, d, h.t, slack))
             retry = ray;
           else
             sink.store(ray, h);
@@ -400,7 +425,7 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
               h.id = -1;
               h.back = 0;
               tlim = tmax;
-              risky = false;
+              slack = 0.0f;
               if (!SL.wide || !wide_usable(o, d, SL.wide_reach)) {
                 retry = i;
               } else {
@@ -415,7 +440,7 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
                 if constexpr (kTarget) {
                   // the target's own hit: what could hide it lies before it;
                   // if it is not hit, the answer is "not the target"
-                  own = sink.target(i);
+                  int32_t const own = sink.target(i);
                   float4 const a = __ldg(&SL.tri[3 * own]), b = __ldg(&SL.tri[3 * own + 1]),
                                c = __ldg(&SL.tri[3 * own + 2]);
                   float t, f, g, inv_det;
@@ -424,7 +449,7 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
                   if (live) {
                     float m, dt;
                     wide_margin(t, norm1(xyz3(b)) + norm1(xyz3(c)), norm1(mk3(a.w, b.w, c.w)), inv_det, &m, &dt);
-                    risky = f < m || g < m || 1.0f - (f + g) < m || t < tmin + dt || tmax < t + dt;
+                    if (f < m || g < m || 1.0f - (f + g) < m || t < tmin + dt || tmax < t + dt) slack = dt;
                     h.t = t;
                     h.f = f;
                     h.g = g;
@@ -440,6 +465,12 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
         unsigned const again = __ballot_sync(0xffffffffu, retry >= 0);
         if (retry >= 0) list[n_list + __popc(again & lanes_below)] = retry;
         n_list += __popc(again);
+        // a whole warp of rays that the tree cannot serve: the rest of the queue
+        // is taken to be like them
+        if (again == 0xffffffffu) {
+          kd_only = true;
+          break;
+        }
         under_way = __ballot_sync(0xffffffffu, live);
         // nothing under way: the list is traced and the rest of the queue
         // taken, or (not yet full) more rays are taken first
@@ -496,26 +527,24 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
             float m, dt;
             wide_margin(t, __uint_as_float(w[13]), __uint_as_float(w[14]), inv_det, &m, &dt);
             bool const edge = f < m || g < m || 1.0f - (f + g) < m || t < tmin + dt;
-            if constexpr (kTarget) {
-              if (id != own) {
-                if (!edge && t + dt < h.t) {
-                  // certainly before the target: the ray is answered
-                  h.id = -1;
-                  live = false;
-                } else {
-                  risky = true;
-                }
+            if (kTarget && id != h.id && !edge && t + dt < h.t) {
+              // certainly before the target: the ray is answered
+              h.id = -1;
+              live = false;
+            } else if (id != h.id) {
+              // the largest error among the hits that are too close to tell apart
+              float const both = fmaxf(fmaxf(slack, tlim - h.t), dt);
+              if (t < h.t || (t == h.t && id > h.id)) {
+                slack = h.t <= t + dt ? both : (edge ? dt : 0.0f);
+                h.t = t;
+                h.f = f;
+                h.g = g;
+                h.id = id;
+                h.back = back;
+                tlim = t + dt;
+              } else {
+                slack = both;
               }
-            } else if (t <= h.t) {
-              risky = edge || h.t <= t + dt;
-              h.t = t;
-              h.f = f;
-              h.g = g;
-              h.id = id;
-              h.back = back;
-              tlim = t + dt;
-            } else {
-              risky = true;
             }
           }
         }
@@ -538,6 +567,11 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
       TraceCount tc{};
       trace_persistent<false, kBatch>(S, n_list, list_fetch, again, tc);
       __syncwarp();
+    }
+    if (kd_only) {
+      TraceCount tc{};
+      trace_persistent<false, kBatch>(S, n, fetch, sink, tc);
+      return;
     }
     if (__all_sync(0xffffffffu, exhausted)) return;
   }

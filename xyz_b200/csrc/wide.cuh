@@ -298,10 +298,14 @@ XYZ_HD WideRay wide_ray(f3 o, f3 d) {
 }
 
 // Rays the tree answers: origin within reach of the scene, direction of
-// about unit length (the margins of wide_margin assume |d| <= 2).
+// about unit length (the margins of wide_margin assume |d| <= 2), no component
+// so small that its reciprocal is infinite: such a ray can lie in a split plane
+// of the kd-tree, whose distance is then not a number, and the kd loop's choice
+// of cells is its own.
 XYZ_HD bool wide_usable(f3 o, f3 d, float reach) {
   float const dd = dot3(d, d);
-  return fabsf(o.x) <= reach && fabsf(o.y) <= reach && fabsf(o.z) <= reach && dd <= 4.0f && dd >= 1e-4f;
+  return fabsf(o.x) <= reach && fabsf(o.y) <= reach && fabsf(o.z) <= reach && dd <= 4.0f && dd >= 1e-4f &&
+         fminf(fminf(fabsf(d.x), fabsf(d.y)), fabsf(d.z)) >= 1e-37f;
 }
 
 // Byte j of w as the float 65536 + byte: the byte times 128 added to the bits
