@@ -477,7 +477,8 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
       } else {
         XYZ_MARK(4, true);
         if (spectral)
-          k_film_spectral<<<gf, kThreads, 0, st>>>(A, film_dev);
+          k_film_spectral<<<static_cast<int>(std::min<int64_t>((A.npix + 31) / 32, 1 << 20)), 32 * kFilmSamples, 0,
+                            st>>>(A, film_dev);
         else
           k_film<<<gf, kThreads, 0, st>>>(A, film_dev);
         XYZ_MARK(4, false);
