@@ -20,6 +20,7 @@ constexpr int64_t kMaxGuidedWave = int64_t{1} << 23;
 // devices never see a partly filled entry or another device's grids.
 struct Grids {
   int raygen, trace_e, trace_s, trace_s_adj, trace_s_guide, trace_s_imp;
+  int both[2], both_sp[2], both_adj[2], both_guide[2], both_imp[2];  // [1]: k_trace_both<true>
   int shade, shade_adj, shade_guide, shade_sp, shade_imp, film;
   // No larger than waves of `paths` paths can use: a queue is never longer, and
   // CTAs without work still cost their launch (a trace of one ray: 5.0 us with
@@ -32,6 +33,8 @@ struct Grids {
       grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(grid, (paths + per_cta - 1) / per_cta)));
     };
     for (int *t : {&g.trace_e, &g.trace_s, &g.trace_s_adj, &g.trace_s_guide, &g.trace_s_imp}) lower(*t, kRaysPerCta);
+    for (int *t : {g.both, g.both_sp, g.both_adj, g.both_guide, g.both_imp})
+      for (int k = 0; k < 2; ++k) lower(t[k], kRaysPerCta);
     for (int *t : {&g.shade, &g.shade_adj, &g.shade_guide, &g.shade_sp, &g.shade_imp}) lower(*t, kThreads);
     return g;
   }
@@ -50,6 +53,16 @@ Grids wave_grids(int device) {
     g.trace_s = occupancy_grid(k_trace_queue<true, false>, device);
     g.trace_s_adj = occupancy_grid(k_trace_queue<true, false, kModeAdjoint>, device);
     g.trace_s_guide = occupancy_grid(k_trace_queue<true, false, kModeGuided>, device);
+    g.both[0] = occupancy_grid(k_trace_both<false, kModePlain>, device);
+    g.both[1] = occupancy_grid(k_trace_both<true, kModePlain>, device);
+    g.both_sp[0] = occupancy_grid(k_trace_both<false, kModePlain, true>, device);
+    g.both_sp[1] = occupancy_grid(k_trace_both<true, kModePlain, true>, device);
+    g.both_adj[0] = occupancy_grid(k_trace_both<false, kModeAdjoint>, device);
+    g.both_adj[1] = occupancy_grid(k_trace_both<true, kModeAdjoint>, device);
+    g.both_guide[0] = occupancy_grid(k_trace_both<false, kModeGuided>, device);
+    g.both_guide[1] = occupancy_grid(k_trace_both<true, kModeGuided>, device);
+    g.both_imp[0] = occupancy_grid(k_trace_both<false, kModeImporton>, device);
+    g.both_imp[1] = occupancy_grid(k_trace_both<true, kModeImporton>, device);
     g.shade = occupancy_grid(k_shade<kModePlain>, device);
     g.shade_adj = occupancy_grid(k_shade<kModeAdjoint>, device);
     g.shade_guide = occupancy_grid(k_shade<kModeGuided>, device);
@@ -394,9 +407,12 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
         ++launches;
         // a replay over cached intersections traces no rays
         bool const trace = !(replay && cached);
+        // Shadow rays go with the next bounce's extension rays (k_trace_both);
+        // profiled renders keep the two classes apart.
+        bool const both = prof == XYZGPU_PROFILE_OFF;
         for (int b = 0; b < iters; ++b) {
           XYZ_MARK(1, true);
-          if (!trace)
+          if (!trace || (both && b > 0))
             ;
           else if (counting)
             k_trace_queue<false, true><<<G.trace_e, kThreads, 0, st>>>(A, b, pc);
@@ -444,7 +460,25 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
           XYZ_MARK(3, true);
           if (!trace)
             ;
-          else if (counting)
+          else if (both && b + 1 < iters) {
+            bool const mixed = A.npaths <= kMixedPaths;
+            auto launch = [&](auto long_queue, auto short_queue, const int *grid) {
+              if (mixed)
+                short_queue<<<grid[1], kThreads, 0, st>>>(A, b);
+              else
+                long_queue<<<grid[0], kThreads, 0, st>>>(A, b);
+            };
+            if (spectral)
+              launch(k_trace_both<false, kModePlain, true>, k_trace_both<true, kModePlain, true>, G.both_sp);
+            else if (replay)
+              launch(k_trace_both<false, kModeAdjoint>, k_trace_both<true, kModeAdjoint>, G.both_adj);
+            else if (guide)
+              launch(k_trace_both<false, kModeGuided>, k_trace_both<true, kModeGuided>, G.both_guide);
+            else if (imp)
+              launch(k_trace_both<false, kModeImporton>, k_trace_both<true, kModeImporton>, G.both_imp);
+            else
+              launch(k_trace_both<false, kModePlain>, k_trace_both<true, kModePlain>, G.both);
+          } else if (counting)
             k_trace_queue<true, true><<<G.trace_s, kThreads, 0, st>>>(A, b, pc);
           else if (replay)
             k_trace_queue<true, false, kModeAdjoint><<<G.trace_s_adj, kThreads, 0, st>>>(A, b, pc);
@@ -455,7 +489,7 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
           else
             k_trace_queue<true, false><<<G.trace_s, kThreads, 0, st>>>(A, b, pc);
           XYZ_MARK(3, false);
-          launches += trace ? 3 : 1;
+          launches += !trace ? 1 : (both && b > 0 ? 2 : 3);
         }
         return XYZGPU_OK;
       };
@@ -610,12 +644,12 @@ namespace {
 
 std::mutex g_noalloc_mu;
 
-// Per device: the array's device address and the launch grids of the five
+// Per device: the array's device address and the launch grids of the
 // kernels (occupancy x SM count of that device).  An entry is published, under
 // g_noalloc_mu, only once all of its fields are set.
 struct NoAllocDevice {
   unsigned char *base;
-  int raygen, trace_e, trace_s, shade, film;
+  int raygen, trace_e, trace_s, both[2], shade, film;
 };
 NoAllocDevice g_noalloc_dev[64] = {};
 
@@ -635,6 +669,8 @@ int noalloc_device(int device, NoAllocDevice *out) {
     d.raygen = occupancy_grid(k_raygen<false>, device);
     d.trace_e = occupancy_grid(k_trace_queue<false, false>, device);
     d.trace_s = occupancy_grid(k_trace_queue<true, false>, device);
+    d.both[0] = occupancy_grid(k_trace_both<false, kModePlain>, device);
+    d.both[1] = occupancy_grid(k_trace_both<true, kModePlain>, device);
     d.shade = occupancy_grid(k_shade<kModePlain>, device);
     d.film = occupancy_grid(k_film, device);
     d.base = static_cast<unsigned char *>(p);
@@ -722,9 +758,14 @@ int render_noalloc_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_r
       int const gr = static_cast<int>(std::min<int64_t>(dev.raygen, (A.npaths + kThreads - 1) / kThreads));
       k_raygen<false><<<gr, kThreads, 0, st>>>(A);
       for (int b = 0; b < iters; ++b) {
-        k_trace_queue<false, false><<<dev.trace_e, kThreads, 0, st>>>(A, b, tally + 8);
+        if (b == 0) k_trace_queue<false, false><<<dev.trace_e, kThreads, 0, st>>>(A, b, tally + 8);
         k_shade<kModePlain><<<dev.shade, kThreads, 0, st>>>(A, b);
-        k_trace_queue<true, false><<<dev.trace_s, kThreads, 0, st>>>(A, b, tally + 8);
+        if (b + 1 < iters && A.npaths <= kMixedPaths)
+          k_trace_both<true, kModePlain><<<dev.both[1], kThreads, 0, st>>>(A, b);
+        else if (b + 1 < iters)
+          k_trace_both<false, kModePlain><<<dev.both[0], kThreads, 0, st>>>(A, b);
+        else
+          k_trace_queue<true, false><<<dev.trace_s, kThreads, 0, st>>>(A, b, tally + 8);
       }
       int const gf = static_cast<int>(std::min<int64_t>(dev.film, (A.npix + kThreads - 1) / kThreads));
       k_film<<<gf, kThreads, 0, st>>>(A, film);

@@ -119,6 +119,18 @@ template <class S, class = void>
 struct SinkHasTarget : std::false_type {};
 template <class S>
 struct SinkHasTarget<S, std::void_t<decltype(S::kTarget)>> : std::bool_constant<S::kTarget> {};
+// Sinks with kMixed hold plain rays as well (target(i) is -1, targeted(i) false).
+template <class S, class = void>
+struct SinkIsMixed : std::false_type {};
+template <class S>
+struct SinkIsMixed<S, std::void_t<decltype(S::kMixed)>> : std::bool_constant<S::kMixed> {};
+template <class Sink>
+XYZ_DEV bool sink_targeted(const Sink &s, int i) {
+  if constexpr (SinkIsMixed<Sink>::value)
+    return s.targeted(i);
+  else
+    return SinkHasTarget<Sink>::value;
+}
 // One iteration of the persistent loop descends at most this many nodes; a lane
 // still above its next leaf resumes there in the next iteration, so the warp's
 // leaf tests do not wait for its longest descent (counting renders descend
@@ -172,10 +184,13 @@ XYZ_DEV void trace_persistent(const DevScene &S, int n, int *fetch, Sink &sink, 
           h.back = 0;
           bool skip = false;
           if constexpr (kTarget) {
-            RayHit own = h;
-            skip = !hit_triangle(SL.tri, sink.target(i), o, d, tmin, own);
-            stop_t = own.t;
-            if (kCount) tc.tris++;
+            stop_t = -INFINITY;
+            if (sink_targeted(sink, i)) {
+              RayHit own = h;
+              skip = !hit_triangle(SL.tri, sink.target(i), o, d, tmin, own);
+              stop_t = own.t;
+              if (kCount) tc.tris++;
+            }
           }
           inv[0] = __frcp_rn(d.x);
           inv[1] = __frcp_rn(d.y);
@@ -327,11 +342,13 @@ XYZ_DEV bool wide_settled(const uint2 *__restrict__ nodes, f3 o, f3 d, float t, 
 template <class Sink>
 struct RetrySink {
   static constexpr bool kTarget = SinkHasTarget<Sink>::value;
+  static constexpr bool kMixed = SinkIsMixed<Sink>::value;
   Sink *s;
   const int32_t *list;
   XYZ_DEV void load(int i, f3 &o, f3 &d, float &tmin, float &tmax) const { s->load(list[i], o, d, tmin, tmax); }
   XYZ_DEV const DevScene *scene(int i) const { return s->scene(list[i]); }
   XYZ_DEV int32_t target(int i) const { return s->target(list[i]); }
+  XYZ_DEV bool targeted(int i) const { return sink_targeted(*s, list[i]); }
   XYZ_DEV void store(int i, const RayHit &h) { s->store(list[i], h); }
 };
 
@@ -440,22 +457,24 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
                 if constexpr (kTarget) {
                   // the target's own hit: what could hide it lies before it;
                   // if it is not hit, the answer is "not the target"
-                  int32_t const own = sink.target(i);
-                  float4 const a = __ldg(&SL.tri[3 * own]), b = __ldg(&SL.tri[3 * own + 1]),
-                               c = __ldg(&SL.tri[3 * own + 2]);
-                  float t, f, g, inv_det;
-                  int32_t back;
-                  live = test_triangle(a, b, c, o, d, tmin, tmax, &t, &f, &g, &back, &inv_det);
-                  if (live) {
-                    float m, dt;
-                    wide_margin(t, norm1(xyz3(b)) + norm1(xyz3(c)), norm1(mk3(a.w, b.w, c.w)), inv_det, &m, &dt);
-                    if (f < m || g < m || 1.0f - (f + g) < m || t < tmin + dt || tmax < t + dt) slack = dt;
-                    h.t = t;
-                    h.f = f;
-                    h.g = g;
-                    h.id = own;
-                    h.back = back;
-                    tlim = t + dt;
+                  if (sink_targeted(sink, i)) {
+                    int32_t const own = sink.target(i);
+                    float4 const a = __ldg(&SL.tri[3 * own]), b = __ldg(&SL.tri[3 * own + 1]),
+                                 c = __ldg(&SL.tri[3 * own + 2]);
+                    float t, f, g, inv_det;
+                    int32_t back;
+                    live = test_triangle(a, b, c, o, d, tmin, tmax, &t, &f, &g, &back, &inv_det);
+                    if (live) {
+                      float m, dt;
+                      wide_margin(t, norm1(xyz3(b)) + norm1(xyz3(c)), norm1(mk3(a.w, b.w, c.w)), inv_det, &m, &dt);
+                      if (f < m || g < m || 1.0f - (f + g) < m || t < tmin + dt || tmax < t + dt) slack = dt;
+                      h.t = t;
+                      h.f = f;
+                      h.g = g;
+                      h.id = own;
+                      h.back = back;
+                      tlim = t + dt;
+                    }
                   }
                 }
               }
@@ -527,7 +546,7 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
             float m, dt;
             wide_margin(t, __uint_as_float(w[13]), __uint_as_float(w[14]), inv_det, &m, &dt);
             bool const edge = f < m || g < m || 1.0f - (f + g) < m || t < tmin + dt;
-            if (kTarget && id != h.id && !edge && t + dt < h.t) {
+            if (kTarget && id != h.id && !edge && t + dt < h.t && sink_targeted(sink, ray)) {
               // certainly before the target: the ray is answered
               h.id = -1;
               live = false;
