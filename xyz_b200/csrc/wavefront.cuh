@@ -581,7 +581,10 @@ template <bool kShadow, bool kCount, int kMode = kModePlain>
 __global__ void __launch_bounds__(kThreads, kCount ? (kShadow ? 10 : 9) : 8) k_trace_queue(WaveArgs A, int b,
                                                           unsigned long long *prof) {
   constexpr bool kBatch = kMode == kModeBatch;
-  if constexpr (kBatch) b = A.cursor->bounce;
+  if constexpr (kBatch) {
+    b += A.cursor->bounce;  // b: 0, or -1 for the bounce that has just ended
+    if (b < 0) return;
+  }
   int32_t *const cnt = A.counts + b * kCountStride;
   int const n = kShadow ? cnt[kCShadow] : cnt[kCExt];
   int const lane = threadIdx.x & 31;
@@ -663,10 +666,15 @@ struct BothSink {
   }
 };
 
+// Batched waves: the extension rays of the cursor's bounce and the shadow rays
+// of the one before it (none at bounce 0).
 template <bool kMixed, int kMode, bool kSpec = false>
 __global__ void __launch_bounds__(kThreads, kMixed ? 7 : 8) k_trace_both(WaveArgs A, int b) {
-  int32_t *const cnt = A.counts + b * kCountStride, *const next = cnt + kCountStride;
-  int const qi = (b + 1) & 1, n_ext = next[kCExt], n_shadow = cnt[kCShadow];
+  constexpr bool kBatch = kMode == kModeBatch;
+  static_assert(!(kMixed && kBatch), "a mixed queue holds rays of one scene");
+  if constexpr (kBatch) b = A.cursor->bounce - 1;
+  int32_t *const next = A.counts + (b + 1) * kCountStride, *const cnt = b >= 0 ? next - kCountStride : next;
+  int const qi = (b + 1) & 1, n_ext = next[kCExt], n_shadow = b >= 0 ? cnt[kCShadow] : 0;
   __shared__ WideList s_list;
   uint32_t visible;
   if constexpr (kMixed) {
@@ -675,10 +683,11 @@ __global__ void __launch_bounds__(kThreads, kMixed ? 7 : 8) k_trace_both(WaveArg
     visible = sink.shadow.visible;
   } else {
     ShadowSink<kSpec, kMode> shadow{&A, 0u, b};
-    trace_closest_hits(A.S, n_shadow, &cnt[kCFetchSh], shadow, s_list);
+    // (an empty queue is not entered: at bounce 0 its counters are those of bounce 0 itself)
+    if (!kBatch || n_shadow > 0) trace_closest_hits<kBatch>(A.S, n_shadow, &cnt[kCFetchSh], shadow, s_list);
     visible = shadow.visible;
-    ExtSink<false> ext{A.q_o[qi], A.q_d[qi], A.hits, &A};
-    trace_closest_hits(A.S, n_ext, &next[kCFetchExt], ext, s_list);
+    ExtSink<kBatch> ext{A.q_o[qi], A.q_d[qi], A.hits, &A};
+    trace_closest_hits<kBatch>(A.S, n_ext, &next[kCFetchExt], ext, s_list);
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) visible += __shfl_down_sync(0xffffffffu, visible, off);
