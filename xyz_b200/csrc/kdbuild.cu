@@ -43,7 +43,15 @@
 namespace xyzgpu {
 namespace {
 
-constexpr int kBigRefs = 2048;
+// References from which a node is split by CTAs: a warp needs 30 us for the
+// decision and 65 us for the emit of 2,000 references (9 and 10 us for 500), the
+// CTAs' five launches 20 us in all.  Device time of the build kernels below,
+// 247,042 triangles: 1,200 us at 2,048, 1,060 at 1,024, 920 at 512 (the
+// decision as it was before), at 256 as at 512.
+constexpr int kBigRefs = 512;
+// References a lane of the small nodes' kernels has in flight: both kernels 696
+// us at 2, 725 at 4 (registers).
+constexpr int kRefUnroll = 2;
 constexpr int kBigThreads = 256;
 constexpr int kBigSlicesMax = 128;     // CTAs per big node when emitting
 constexpr int kBigSliceBudget = 1024;  // CTAs per emit launch (about)
@@ -141,9 +149,38 @@ XYZ_DEV int bin_of(float x, float lo, float scale, int B) {
 XYZ_DEV bool better(float c0, int i0, float c1, int i1) { return c0 < c1 || (c0 == c1 && i0 < i1); }
 
 // ---- decide: one warp per small node
+// The cost of candidate i of axis kA: candidate_cost with the axis known.
+template <int kA>
+XYZ_DEV float plane_cost(const BuildArgs &A, int i, int nl, int nr, f3 ext, float lo, float hi, float step, float sa) {
+  float const plane = lo + static_cast<float>(i) * step;
+  float const dl = plane - lo, dr = hi - plane;
+  float const sal = half_area3(kA == 0 ? dl : ext.x, kA == 1 ? dl : ext.y, kA == 2 ? dl : ext.z);
+  float const sar = half_area3(kA == 0 ? dr : ext.x, kA == 1 ? dr : ext.y, kA == 2 ? dr : ext.z);
+  float cost = A.ct + A.ci * (sal * static_cast<float>(nl) + sar * static_cast<float>(nr)) / sa;
+  if (nl == 0 || nr == 0) cost = cost * (1.0f - A.eb);
+  return cost;
+}
+
+// The order of finite costs and infinity as unsigned numbers; a NaN comes last.
+XYZ_DEV uint32_t cost_key(float c) {
+  if (!(c == c)) return 0xffffffffu;
+  uint32_t const u = __float_as_uint(c + 0.0f);
+  return u ^ ((u >> 31) ? 0xffffffffu : 0x80000000u);
+}
+XYZ_DEV float key_cost(uint32_t k) { return __uint_as_float(k ^ ((k >> 31) ? 0x80000000u : 0xffffffffu)); }
+
+// Deep levels hold 100,000 nodes of a few references and are bound by
+// instructions; shallow ones hold a few hundred nodes of up to kBigRefs, whose
+// warps wait for their loads.  So: up to 32 bins, lane i holds plane i + 1 of
+// each axis and the counts before it, starts and ends packed in 16 bits each
+// (three histograms and scans instead of six, nothing written back); the loads
+// of kRefUnroll references are in flight together; up to that many stay in
+// registers for the children's counts.  All 30 levels of a 247,042-triangle
+// build: 618 -> 400 us (843 with nodes of up to 2,047 references).
 __global__ void __launch_bounds__(32 * kWarpsPerBlock)
     k_decide_small(LevelArrays L, int m, RefArrays R, BuildArgs A) {
-  __shared__ uint32_t hist[kWarpsPerBlock][3 * 2 * (kKdMaxBins + 1)];
+  static_assert(kBigRefs <= 0xffff, "packed counts");
+  __shared__ uint32_t hist[kWarpsPerBlock][3 * (kKdMaxBins + 1)];
   int const lane = threadIdx.x & 31;
   int const wib = threadIdx.x >> 5;
   uint32_t *h = hist[wib];
@@ -153,98 +190,123 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
     int const n = L.count[j];
     int const B = kd_node_bins(A.bins, n);
     if (n >= kBigRefs && eligible(A, n)) continue;  // a CTA decides this node
-    if (!eligible(A, n)) {
-      if (lane == 0) {
-        L.axis[j] = -1;
-        L.nl[j] = L.nr[j] = 0;
-      }
-      continue;
-    }
     float4 const lo4 = L.blo[j], hi4 = L.bhi[j];
-    float const ext[3] = {hi4.x - lo4.x, hi4.y - lo4.y, hi4.z - lo4.z};
-    float const sa = half_area3(ext[0], ext[1], ext[2]);
-    if (!(sa > 0.0f)) {
+    int const rb = L.begin[j];
+    f3 const ext = mk3(hi4.x - lo4.x, hi4.y - lo4.y, hi4.z - lo4.z);
+    float const sa = half_area3(ext.x, ext.y, ext.z);
+    if (!eligible(A, n) || !(sa > 0.0f)) {
       if (lane == 0) {
         L.axis[j] = -1;
         L.nl[j] = L.nr[j] = 0;
       }
       continue;
     }
-    // the six rows' first B + 1 entries (the rest is never read)
-    for (int t = lane; t < 6 * (B + 1); t += 32) h[(t / (B + 1)) * (kKdMaxBins + 1) + t % (B + 1)] = 0u;
+    float const bins = static_cast<float>(B);
+    f3 const scale = mk3(bins / ext.x, bins / ext.y, bins / ext.z);
+    f3 const step = mk3(ext.x / bins, ext.y / bins, ext.z / bins);
+    // the three rows' first B entries (the rest is never read)
+    for (int t = lane; t < B; t += 32) h[t] = h[kKdMaxBins + 1 + t] = h[2 * (kKdMaxBins + 1) + t] = 0u;
     __syncwarp();
-    int const rb = L.begin[j];
-    for (int a = 0; a < 3; ++a) {
-      if (!(ext[a] > 0.0f)) continue;
-      float const scale = static_cast<float>(B) / ext[a];
-      float const lo = comp4(lo4, a);
-      for (int r = lane; r < n; r += 32) {
-        int const b0 = bin_of(R.lo[a][rb + r], lo, scale, B);
-        int const b1 = bin_of(R.hi[a][rb + r], lo, scale, B);
-        atomicAdd(&h[(a * 2 + 0) * (kKdMaxBins + 1) + b0], 1u);
-        atomicAdd(&h[(a * 2 + 1) * (kKdMaxBins + 1) + b1], 1u);
-      }
-    }
-    __syncwarp();
-    // exclusive prefix of each of the six rows in place, the whole warp per
-    // row: lane k holds bins 2k and 2k + 1 (B <= 64), an inclusive scan of
-    // the pairs' sums over the lanes; row[B] gets the total
-    for (int q = 0; q < 6; ++q) {
-      uint32_t *row = h + q * (kKdMaxBins + 1);
-      int const b0 = 2 * lane, b1 = 2 * lane + 1;
-      uint32_t const v0 = b0 < B ? row[b0] : 0u, v1 = b1 < B ? row[b1] : 0u;
-      uint32_t const pair = v0 + v1;
-      uint32_t incl = pair;
+    float v[kRefUnroll][6];
+    for (int r0 = 0; r0 < n; r0 += 32 * kRefUnroll) {
 #pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        uint32_t const t = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl += t;
+      for (int u = 0; u < kRefUnroll; ++u) {
+        int const r = rb + min(r0 + 32 * u + lane, n - 1);
+        if (u == 0 || r0 + 32 * u < n) {
+#pragma unroll
+          for (int a = 0; a < 3; ++a) {
+            v[u][2 * a] = R.lo[a][r];
+            v[u][2 * a + 1] = R.hi[a][r];
+          }
+        }
       }
-      __syncwarp();
-      if (b0 < B) row[b0] = incl - pair;
-      if (b1 < B) row[b1] = incl - pair + v0;
-      if (lane == 31) row[B] = incl;
-      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < kRefUnroll; ++u) {
+        if (r0 + 32 * u + lane < n) {
+#pragma unroll
+          for (int a = 0; a < 3; ++a) {
+            float const e = a == 0 ? ext.x : (a == 1 ? ext.y : ext.z);
+            float const o = comp4(lo4, a), sc = a == 0 ? scale.x : (a == 1 ? scale.y : scale.z);
+            if (e > 0.0f) {
+              atomicAdd(&h[a * (kKdMaxBins + 1) + bin_of(v[u][2 * a], o, sc, B)], 1u);
+              atomicAdd(&h[a * (kKdMaxBins + 1) + bin_of(v[u][2 * a + 1], o, sc, B)], 0x10000u);
+            }
+          }
+        }
+      }
     }
+    __syncwarp();
+    // plane i + 1 has the bins up to i on its left: inclusive scans over the
+    // lanes, 32 bins at a time
     float best = INFINITY;
     int best_c = 0x7fffffff;
-    for (int c = lane; c < 3 * (B - 1); c += 32) {
-      float pl;
-      int nl;
-      float const cost = candidate_cost(A, B, h, c, n, ext, lo4, hi4, sa, &pl, &nl);
-      if (better(cost, c, best, best_c)) {
-        best = cost;
-        best_c = c;
-      }
-    }
+    uint32_t carry[3] = {0u, 0u, 0u};
+    for (int base = 0; base < B - 1; base += 32) {
+      int const i = base + lane + 1;
+      uint32_t incl[3];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      float const oc = __shfl_xor_sync(0xffffffffu, best, off);
-      int const oi = __shfl_xor_sync(0xffffffffu, best_c, off);
-      if (better(oc, oi, best, best_c)) {
-        best = oc;
-        best_c = oi;
+      for (int a = 0; a < 3; ++a) incl[a] = i <= B ? h[a * (kKdMaxBins + 1) + i - 1] : 0u;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          uint32_t const t = __shfl_up_sync(0xffffffffu, incl[a], off);
+          if (lane >= off) incl[a] += t;
+        }
+#pragma unroll
+      for (int a = 0; a < 3; ++a) incl[a] += carry[a];
+      if (i < B) {
+        auto consider = [&](float e, float cost, int c) {
+          if (e > 0.0f && better(cost, c, best, best_c)) {
+            best = cost;
+            best_c = c;
+          }
+        };
+        auto left = [&](int a) { return static_cast<int>(incl[a] & 0xffffu); };
+        auto right = [&](int a) { return n - static_cast<int>(incl[a] >> 16); };
+        consider(ext.x, plane_cost<0>(A, i, left(0), right(0), ext, lo4.x, hi4.x, step.x, sa), i - 1);
+        consider(ext.y, plane_cost<1>(A, i, left(1), right(1), ext, lo4.y, hi4.y, step.y, sa), (B - 1) + i - 1);
+        consider(ext.z, plane_cost<2>(A, i, left(2), right(2), ext, lo4.z, hi4.z, step.z, sa), 2 * (B - 1) + i - 1);
       }
+      if (base + 32 < B - 1)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) carry[a] = __shfl_sync(0xffffffffu, incl[a], 31);
     }
+    // smallest cost, then smallest candidate
+    uint32_t const key = cost_key(best);
+    uint32_t const min_key = __reduce_min_sync(0xffffffffu, key);
+    best_c = static_cast<int>(
+        __reduce_min_sync(0xffffffffu, key == min_key ? static_cast<uint32_t>(best_c) : 0x7fffffffu));
     int axis = -1;
     float plane = 0.0f;
-    if (best < A.ci * static_cast<float>(n)) {
-      int nl_bin;
-      candidate_cost(A, B, h, best_c, n, ext, lo4, hi4, sa, &plane, &nl_bin);
-      axis = best_c / (B - 1);
-    }
     int nl = 0, nr = 0;
-    if (axis >= 0) {
-      for (int r = lane; r < n; r += 32) {
-        bool l, rr;
-        classify_ref(R.lo[axis][rb + r], R.hi[axis][rb + r], plane, &l, &rr);
-        nl += l;
-        nr += rr;
-      }
+    if (key_cost(min_key) < A.ci * static_cast<float>(n)) {
+      axis = best_c / (B - 1);
+      int const i = best_c - axis * (B - 1) + 1;
+      float const s = axis == 0 ? step.x : (axis == 1 ? step.y : step.z);
+      plane = comp4(lo4, axis) + static_cast<float>(i) * s;
+      if (n <= 32 * kRefUnroll) {
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        nl += __shfl_xor_sync(0xffffffffu, nl, off);
-        nr += __shfl_xor_sync(0xffffffffu, nr, off);
+        for (int u = 0; u < kRefUnroll; ++u) {
+          float const lo = axis == 0 ? v[u][0] : (axis == 1 ? v[u][2] : v[u][4]);
+          float const hi = axis == 0 ? v[u][1] : (axis == 1 ? v[u][3] : v[u][5]);
+          bool l = false, r = false;
+          if (32 * u + lane < n) classify_ref(lo, hi, plane, &l, &r);
+          nl += __popc(__ballot_sync(0xffffffffu, l));
+          nr += __popc(__ballot_sync(0xffffffffu, r));
+        }
+      } else {
+        const float *const lo = rb + (axis == 0 ? R.lo[0] : (axis == 1 ? R.lo[1] : R.lo[2]));
+        const float *const hi = rb + (axis == 0 ? R.hi[0] : (axis == 1 ? R.hi[1] : R.hi[2]));
+#pragma unroll 4
+        for (int r = lane; r < n; r += 32) {
+          bool l, rr;
+          classify_ref(lo[r], hi[r], plane, &l, &rr);
+          nl += l;
+          nr += rr;
+        }
+        nl = __reduce_add_sync(0xffffffffu, nl);
+        nr = __reduce_add_sync(0xffffffffu, nr);
       }
     }
     if (lane == 0) {
@@ -503,12 +565,12 @@ XYZ_DEV void write_split_node(const EmitArgs &E, int j, int axis, float plane) {
   E.N.count[c + 1] = E.L.nr[j];
 }
 
-XYZ_DEV void write_ref(const RefArrays &D, int dst, const RefArrays &S, int src, int axis, float plane,
-                       bool left) {
-  D.tri[dst] = S.tri[src];
+// One reference of a child: its box (lo, hi per axis) cut at the plane.
+XYZ_DEV void put_ref(const RefArrays &D, int dst, int32_t tri, const float *box, int axis, float plane, bool left) {
+  D.tri[dst] = tri;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    float lo = S.lo[k][src], hi = S.hi[k][src];
+    float lo = box[2 * k], hi = box[2 * k + 1];
     if (k == axis) {
       if (left)
         hi = fminf(hi, plane);
@@ -518,6 +580,17 @@ XYZ_DEV void write_ref(const RefArrays &D, int dst, const RefArrays &S, int src,
     D.lo[k][dst] = lo;
     D.hi[k][dst] = hi;
   }
+}
+
+XYZ_DEV void write_ref(const RefArrays &D, int dst, const RefArrays &S, int src, int axis, float plane,
+                       bool left) {
+  float box[6];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    box[2 * k] = S.lo[k][src];
+    box[2 * k + 1] = S.hi[k][src];
+  }
+  put_ref(D, dst, S.tri[src], box, axis, plane, left);
 }
 
 __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_emit_small(EmitArgs E, BuildArgs A) {
@@ -543,17 +616,36 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_emit_small(EmitArgs E, 
     int const lbase = static_cast<int>(E.L.scan[j].z);
     int const rbase = lbase + E.L.nl[j];
     int nl_run = 0, nr_run = 0;
-    for (int r0 = 0; r0 < n; r0 += 32) {
-      int const r = r0 + lane;
-      bool l = false, rr = false;
-      if (r < n) classify_ref(E.R.lo[axis][rb + r], E.R.hi[axis][rb + r], plane, &l, &rr);
-      unsigned const ml = __ballot_sync(0xffffffffu, l);
-      unsigned const mr = __ballot_sync(0xffffffffu, rr);
-      unsigned const below = (1u << lane) - 1u;
-      if (l) write_ref(E.RN, lbase + nl_run + __popc(ml & below), E.R, rb + r, axis, plane, true);
-      if (rr) write_ref(E.RN, rbase + nr_run + __popc(mr & below), E.R, rb + r, axis, plane, false);
-      nl_run += __popc(ml);
-      nr_run += __popc(mr);
+    unsigned const below = (1u << lane) - 1u;
+    for (int r0 = 0; r0 < n; r0 += 32 * kRefUnroll) {
+      float v[kRefUnroll][6];
+      int32_t tri[kRefUnroll];
+#pragma unroll
+      for (int u = 0; u < kRefUnroll; ++u) {
+        int const r = rb + min(r0 + 32 * u + lane, n - 1);
+        if (u > 0 && r0 + 32 * u >= n) break;  // the same on every lane
+        tri[u] = E.R.tri[r];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          v[u][2 * k] = E.R.lo[k][r];
+          v[u][2 * k + 1] = E.R.hi[k][r];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kRefUnroll; ++u) {
+        if (u > 0 && r0 + 32 * u >= n) break;
+        float const *const w = v[u];
+        float const lo = axis == 0 ? w[0] : (axis == 1 ? w[2] : w[4]);
+        float const hi = axis == 0 ? w[1] : (axis == 1 ? w[3] : w[5]);
+        bool l = false, rr = false;
+        if (r0 + 32 * u + lane < n) classify_ref(lo, hi, plane, &l, &rr);
+        unsigned const ml = __ballot_sync(0xffffffffu, l);
+        unsigned const mr = __ballot_sync(0xffffffffu, rr);
+        if (l) put_ref(E.RN, lbase + nl_run + __popc(ml & below), tri[u], w, axis, plane, true);
+        if (rr) put_ref(E.RN, rbase + nr_run + __popc(mr & below), tri[u], w, axis, plane, false);
+        nl_run += __popc(ml);
+        nr_run += __popc(mr);
+      }
     }
   }
 }
