@@ -18,8 +18,8 @@
 //              scatter of references into the children (ballot / block scans,
 //              and per-slice counts for big nodes, keep the parent's order) or
 //              into the leaf reference array
-// The host reads two small values per level (the big-node count and the scan
-// totals) to size the next level; everything else stays on the device.
+// The host reads once per level (the scan totals and the next level's big-node
+// count) to size the next level; everything else stays on the device.
 //
 // Layout (kd_layout_depth_first, after either builder): the breadth-first
 // array is permuted so that every subtree occupies one contiguous range, in
@@ -57,6 +57,7 @@ constexpr int kBigSlicesMax = 128;     // CTAs per big node when emitting
 constexpr int kBigSliceBudget = 1024;  // CTAs per emit launch (about)
 constexpr int kWarpsPerBlock = 4;
 constexpr int kScanThreads = 256;
+constexpr int kFirstLevelNodes = 8192;  // 0.6 MB a set of level arrays
 constexpr int kScanPerThread = 8;
 constexpr int kScanPerBlock = kScanThreads * kScanPerThread;
 
@@ -73,6 +74,13 @@ struct LevelArrays {
   float *plane;
   int32_t *nl, *nr;
   uint4 *scan;        // in: (split, leaf refs, next refs, empty leaf); out: exclusive prefix
+};
+
+// What the host reads of a level.
+struct LevelTotals {
+  uint4 scan;        // splits, leaf refs, next refs, empty leaves
+  int32_t next_big;  // the next level's big nodes
+  int32_t pad[3];
 };
 
 struct BuildArgs {
@@ -98,7 +106,15 @@ __global__ void k_init_refs(const float4 *__restrict__ tri, int n, RefArrays R) 
   }
 }
 
-XYZ_DEV bool eligible(const BuildArgs &a, int n) { return n > a.leaf_max && a.depth < a.max_depth; }
+__global__ void k_init_root(LevelArrays L, float4 lo, float4 hi, int n, int32_t *big_count) {
+  L.blo[0] = lo;
+  L.bhi[0] = hi;
+  L.begin[0] = 0;
+  L.count[0] = n;
+  *big_count = 0;
+}
+
+__host__ __device__ inline bool eligible(const BuildArgs &a, int n) { return n > a.leaf_max && a.depth < a.max_depth; }
 
 __global__ void k_classify(LevelArrays L, int m, BuildArgs a, int32_t *big_list, int32_t *big_count) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
@@ -178,9 +194,11 @@ XYZ_DEV float key_cost(uint32_t k) { return __uint_as_float(k ^ ((k >> 31) ? 0x8
 // registers for the children's counts.  All 30 levels of a 247,042-triangle
 // build: 618 -> 400 us (843 with nodes of up to 2,047 references).
 __global__ void __launch_bounds__(32 * kWarpsPerBlock)
-    k_decide_small(LevelArrays L, int m, RefArrays R, BuildArgs A) {
+    k_decide_small(LevelArrays L, int m, RefArrays R, BuildArgs A, LevelTotals *totals, int32_t *big_count) {
   static_assert(kBigRefs <= 0xffff, "packed counts");
   __shared__ uint32_t hist[kWarpsPerBlock][3 * (kKdMaxBins + 1)];
+  // counters of the next level (this level's list is complete)
+  if (blockIdx.x == 0 && threadIdx.x == 0) totals->next_big = *big_count = 0;
   int const lane = threadIdx.x & 31;
   int const wib = threadIdx.x >> 5;
   uint32_t *h = hist[wib];
@@ -451,11 +469,16 @@ __global__ void __launch_bounds__(kBigThreads)
   }
 }
 
-__global__ void k_flags(LevelArrays L, int m, int force_leaves) {
+__global__ void k_flags(LevelArrays L, int m, int force_leaves, BuildArgs next, LevelTotals *totals) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
     if (force_leaves) L.axis[j] = -1;
     int const split = L.axis[j] >= 0;
     int const n = L.count[j];
+    if (split) {
+      int const nl = L.nl[j], nr = L.nr[j];
+      int const big = (nl >= kBigRefs && eligible(next, nl)) + (nr >= kBigRefs && eligible(next, nr));
+      if (big) atomicAdd(&totals->next_big, big);
+    }
     L.scan[j] = make_uint4(split, split ? 0u : static_cast<uint32_t>(n),
                            split ? static_cast<uint32_t>(L.nl[j] + L.nr[j]) : 0u, (!split && n == 0) ? 1u : 0u);
   }
@@ -1068,10 +1091,11 @@ int kd_build_device(SceneImpl &s, const float4 *d_tri, int n, const BuildConfig 
   LevelBufs lv[2];
   DevBuf<uint2> nodes;
   DevBuf<int32_t> leaf_refs;
-  DevBuf<int32_t> big_list, small_i32;
+  DevBuf<int32_t> big_list, big_count;
   DevBuf<int2> big_cnt;
   DevBuf<uint32_t> big_hist;
-  DevBuf<uint4> block_sums, grand;
+  DevBuf<uint4> block_sums;
+  DevBuf<LevelTotals> totals;
   for (int q = 0; q < 2; ++q) {
     refs[q].tri.st = st;
     for (auto &c : refs[q].c) c.st = st;
@@ -1082,15 +1106,16 @@ int kd_build_device(SceneImpl &s, const float4 *d_tri, int n, const BuildConfig 
   }
   nodes.st = st;
   leaf_refs.st = st;
-  big_list.st = small_i32.st = st;
+  big_list.st = big_count.st = st;
   big_cnt.st = big_hist.st = st;
-  block_sums.st = grand.st = st;
+  block_sums.st = totals.st = st;
   XYZ_BUILD_TRY(refs[0].reserve(std::max(1, n)));
-  XYZ_BUILD_TRY(lv[0].reserve(1));
+  // (a level may hold twice the nodes of the one before: not from one node up)
+  for (auto &l : lv) XYZ_BUILD_TRY(l.reserve(std::min(std::max(1, n), kFirstLevelNodes)));
   XYZ_BUILD_TRY(nodes.reserve(std::max<int64_t>(64, 2 * static_cast<int64_t>(n) / std::max(1, cfg.leaf_max_tris))));
   XYZ_BUILD_TRY(leaf_refs.reserve(std::max<int64_t>(64, 2 * static_cast<int64_t>(n))));
-  XYZ_BUILD_TRY(small_i32.reserve(8));
-  XYZ_BUILD_TRY(grand.reserve(1));
+  XYZ_BUILD_TRY(big_count.reserve(1));
+  XYZ_BUILD_TRY(totals.reserve(1));
 
   if (n > 0) {
     k_init_refs<<<grid_for(n, 256, dev), 256, 0, st>>>(d_tri, n, refs[0].view());
@@ -1098,28 +1123,25 @@ int kd_build_device(SceneImpl &s, const float4 *d_tri, int n, const BuildConfig 
   }
   float4 const rlo = make_float4(s.dev.bmin.x, s.dev.bmin.y, s.dev.bmin.z, 0.0f);
   float4 const rhi = make_float4(s.dev.bmax.x, s.dev.bmax.y, s.dev.bmax.z, 0.0f);
-  int32_t const zero = 0;
-  XYZ_BUILD_TRY(cudaMemcpyAsync(lv[0].blo.p, &rlo, sizeof(float4), cudaMemcpyHostToDevice, st));
-  XYZ_BUILD_TRY(cudaMemcpyAsync(lv[0].bhi.p, &rhi, sizeof(float4), cudaMemcpyHostToDevice, st));
-  XYZ_BUILD_TRY(cudaMemcpyAsync(lv[0].begin.p, &zero, sizeof(int32_t), cudaMemcpyHostToDevice, st));
-  XYZ_BUILD_TRY(cudaMemcpyAsync(lv[0].count.p, &n, sizeof(int32_t), cudaMemcpyHostToDevice, st));
+  k_init_root<<<1, 1, 0, st>>>(lv[0].view(), rlo, rhi, n, big_count.p);
+  XYZ_BUILD_TRY(cudaGetLastError());
 
   int64_t level_base = 0, leaf_total = 0, leaves = 0, empty = 0;
   int m = 1, depth = 0, cur = 0;
+  A.depth = 0;
+  int n_big = n >= kBigRefs && eligible(A, n) ? 1 : 0;
   std::vector<int64_t> level_start;
   for (depth = 0;; ++depth) {
     level_start.push_back(level_base);
     A.depth = depth;
     LevelArrays L = lv[cur].view();
-    // big nodes
-    XYZ_BUILD_TRY(big_list.reserve(m));
-    XYZ_BUILD_TRY(cudaMemsetAsync(small_i32.p, 0, sizeof(int32_t), st));
-    k_classify<<<grid_for(m, 256, dev), 256, 0, st>>>(L, m, A, big_list.p, small_i32.p);
-    int32_t n_big = 0;
-    XYZ_BUILD_TRY(cudaMemcpyAsync(&n_big, small_i32.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    XYZ_BUILD_TRY(cudaStreamSynchronize(st));
+    if (n_big > 0) {
+      XYZ_BUILD_TRY(big_list.reserve(n_big));
+      k_classify<<<grid_for(m, 256, dev), 256, 0, st>>>(L, m, A, big_list.p, big_count.p);
+    }
     RefArrays const R = refs[cur].view();
-    k_decide_small<<<grid_for(int64_t{m} * 32, 32 * kWarpsPerBlock, dev), 32 * kWarpsPerBlock, 0, st>>>(L, m, R, A);
+    k_decide_small<<<grid_for(int64_t{m} * 32, 32 * kWarpsPerBlock, dev), 32 * kWarpsPerBlock, 0, st>>>(
+        L, m, R, A, totals.p, big_count.p);
     // big nodes: sliced histograms, one CTA per node for the decision, sliced
     // left / right counts (kept for the emit) and their per-node totals;
     // slices per node: up to 128, about 1,024 CTAs per launch in all
@@ -1135,16 +1157,22 @@ int kd_build_device(SceneImpl &s, const float4 *d_tri, int n, const BuildConfig 
     }
     XYZ_BUILD_TRY(cudaGetLastError());
     // flags + scan (twice if the reference budget is exceeded)
-    uint4 tot = make_uint4(0, 0, 0, 0);
+    BuildArgs next = A;
+    next.depth = depth + 1;
+    LevelTotals level{};
+    uint4 &tot = level.scan;
     for (int pass = 0; pass < 2; ++pass) {
-      k_flags<<<grid_for(m, 256, dev), 256, 0, st>>>(L, m, pass);
+      k_flags<<<grid_for(m, 256, dev), 256, 0, st>>>(L, m, pass, next, totals.p);
       int const nb = static_cast<int>((m + kScanPerBlock - 1) / kScanPerBlock);
       XYZ_BUILD_TRY(block_sums.reserve(nb));
-      k_scan_blocks<<<nb, kScanThreads, 0, st>>>(L.scan, m, block_sums.p);
-      k_scan_totals<<<1, kScanThreads, 0, st>>>(block_sums.p, nb, grand.p);
-      k_scan_add<<<(m + 255) / 256, 256, 0, st>>>(L.scan, m, block_sums.p);
+      // one block: its sums are the level's
+      k_scan_blocks<<<nb, kScanThreads, 0, st>>>(L.scan, m, nb == 1 ? &totals.p->scan : block_sums.p);
+      if (nb > 1) {
+        k_scan_totals<<<1, kScanThreads, 0, st>>>(block_sums.p, nb, &totals.p->scan);
+        k_scan_add<<<(m + 255) / 256, 256, 0, st>>>(L.scan, m, block_sums.p);
+      }
       XYZ_BUILD_TRY(cudaGetLastError());
-      XYZ_BUILD_TRY(cudaMemcpyAsync(&tot, grand.p, sizeof(uint4), cudaMemcpyDeviceToHost, st));
+      XYZ_BUILD_TRY(cudaMemcpyAsync(&level, totals.p, sizeof(level), cudaMemcpyDeviceToHost, st));
       XYZ_BUILD_TRY(cudaStreamSynchronize(st));
       if (static_cast<int64_t>(tot.z) <= cfg.max_refs) break;
     }
@@ -1184,6 +1212,7 @@ int kd_build_device(SceneImpl &s, const float4 *d_tri, int n, const BuildConfig 
     level_base = next_base;
     if (next_m == 0) break;
     m = static_cast<int>(next_m);
+    n_big = level.next_big;
     cur ^= 1;
   }
   XYZ_BUILD_TRY(cudaStreamSynchronize(st));

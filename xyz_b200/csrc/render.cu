@@ -189,8 +189,10 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
   int64_t cap = rp.wave_paths;
   if (cap <= 0) {
     cap = std::min<int64_t>(kMaxDefaultWave, std::max<int64_t>(1, npix_total * rp.spp));
+    // (the query takes a third of a millisecond after a scene's allocations:
+    // only when the buffers would grow)
     size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
+    if (cap > sw.ws.capacity && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
       int64_t const afford = static_cast<int64_t>((free_b / 2 + sw.ws.capacity * kBytesPerPath) / kBytesPerPath);
       cap = std::min(cap, std::max<int64_t>(afford, int64_t{1} << 20));
     }
