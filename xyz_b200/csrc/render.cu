@@ -21,7 +21,7 @@ constexpr int64_t kMaxGuidedWave = int64_t{1} << 23;
 struct Grids {
   int raygen, trace_e, trace_s, trace_s_adj, trace_s_guide, trace_s_imp;
   int both[2], both_sp[2], both_adj[2], both_guide[2], both_imp[2];  // [1]: k_trace_both<true>
-  int shade, shade_adj, shade_guide, shade_sp, shade_imp, film;
+  int shade, shade_adj, shade_guide, shade_sp, shade_imp, film, small_wave;
   // No larger than waves of `paths` paths can use: a queue is never longer, and
   // CTAs without work still cost their launch (a trace of one ray: 5.0 us with
   // the full grid, 3.8 with one CTA).  Traces get a CTA per 32 rays (8 a warp,
@@ -39,6 +39,13 @@ struct Grids {
     return g;
   }
 };
+
+// As many paths a CTA as it takes for all CTAs to be resident.
+void launch_small_wave(const WaveArgs &A, int iters, int resident, cudaStream_t st) {
+  int64_t const per_cta = (A.npaths + resident - 1) / resident;
+  k_small_wave<<<static_cast<int>((A.npaths + per_cta - 1) / per_cta), kThreads, 0, st>>>(A, iters,
+                                                                                         static_cast<int>(per_cta));
+}
 
 Grids wave_grids(int device) {
   static std::mutex mu;
@@ -70,6 +77,7 @@ Grids wave_grids(int device) {
     g.trace_s_imp = occupancy_grid(k_trace_queue<true, false, kModeImporton>, device);
     g.shade_imp = occupancy_grid(k_shade<kModeImporton>, device);
     g.film = occupancy_grid(k_film, device);
+    g.small_wave = occupancy_grid(k_small_wave, device);
     table[d] = g;
     ready[d] = true;
   }
@@ -412,6 +420,11 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
         // Shadow rays go with the next bounce's extension rays (k_trace_both);
         // profiled renders keep the two classes apart.
         bool const both = prof == XYZGPU_PROFILE_OFF;
+        if (both && !adj && !guide && !imp && !spectral && A.npaths <= kSmallWave) {
+          launch_small_wave(A, iters, G.small_wave, st);
+          ++launches;
+          return XYZGPU_OK;
+        }
         for (int b = 0; b < iters; ++b) {
           XYZ_MARK(1, true);
           if (!trace || (both && b > 0))
@@ -651,7 +664,7 @@ std::mutex g_noalloc_mu;
 // g_noalloc_mu, only once all of its fields are set.
 struct NoAllocDevice {
   unsigned char *base;
-  int raygen, trace_e, trace_s, both[2], shade, film;
+  int raygen, trace_e, trace_s, both[2], shade, film, small_wave;
 };
 NoAllocDevice g_noalloc_dev[64] = {};
 
@@ -674,6 +687,7 @@ int noalloc_device(int device, NoAllocDevice *out) {
     d.both[0] = occupancy_grid(k_trace_both<false, kModePlain>, device);
     d.both[1] = occupancy_grid(k_trace_both<true, kModePlain>, device);
     d.shade = occupancy_grid(k_shade<kModePlain>, device);
+    d.small_wave = occupancy_grid(k_small_wave, device);
     d.film = occupancy_grid(k_film, device);
     d.base = static_cast<unsigned char *>(p);
     g_noalloc_dev[device] = d;
@@ -759,7 +773,9 @@ int render_noalloc_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_r
       XYZ_CUDA_TRY(cudaMemsetAsync(A.counts, 0, kNoAllocCounts, st));
       int const gr = static_cast<int>(std::min<int64_t>(dev.raygen, (A.npaths + kThreads - 1) / kThreads));
       k_raygen<false><<<gr, kThreads, 0, st>>>(A);
-      for (int b = 0; b < iters; ++b) {
+      bool const small = A.npaths <= kSmallWave;
+      if (small) launch_small_wave(A, iters, dev.small_wave, st);
+      for (int b = 0; b < iters && !small; ++b) {
         if (b == 0) k_trace_queue<false, false><<<dev.trace_e, kThreads, 0, st>>>(A, b, tally + 8);
         k_shade<kModePlain><<<dev.shade, kThreads, 0, st>>>(A, b);
         if (b + 1 < iters && A.npaths <= kMixedPaths)

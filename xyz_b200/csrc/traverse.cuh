@@ -382,13 +382,12 @@ constexpr int kRaysPerCta = 32;
 // taken together, once enough lanes are not under way, so that neither runs
 // for a lane or two at a time.
 template <bool kBatch = false, class Sink>
-XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_t *list, int *list_fetch) {
+XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_t *list, int *list_fetch, int warps) {
   constexpr bool kTarget = SinkHasTarget<Sink>::value;
   int const lane = threadIdx.x & 31;
   unsigned const lanes_below = (1u << lane) - 1u;
   // short queues: fewer lanes per warp, so that all warps have a share and a
   // warp's rays wait for fewer others
-  int const warps = (gridDim.x * blockDim.x) >> 5;
   int const width = min(32, max(1, (n + warps - 1) / warps));
   int const refill_at = width < 32 ? 0 : 32 - ((kBatch || S.n_wide > kWideTinyNodes) ? kWideRefill : kWideRefillTiny);
   bool exhausted = lane >= width;
@@ -603,12 +602,17 @@ struct WideList {
   int fetch[kTraceWarps];
 };
 
-// Closest hits through the wide tree, or the kd-tree of a scene without one.
+// The grid's warps, which share a launch's queues.
+XYZ_DEV int grid_warps() { return static_cast<int>((gridDim.x * blockDim.x) >> 5); }
+
+// Closest hits through the wide tree, or the kd-tree of a scene without one, of
+// a queue that `warps` warps work on.
 template <bool kBatch = false, class Sink>
-XYZ_DEV void trace_closest_hits(const DevScene &S, int n, int *fetch, Sink &sink, WideList &L) {
+XYZ_DEV void trace_closest_hits(const DevScene &S, int n, int *fetch, Sink &sink, WideList &L,
+                                int warps = grid_warps()) {
   if (kBatch || S.wide) {
     int const w = threadIdx.x >> 5;
-    trace_wide<kBatch>(S, n, fetch, sink, L.entry[w], &L.fetch[w]);
+    trace_wide<kBatch>(S, n, fetch, sink, L.entry[w], &L.fetch[w], warps);
   } else {
     TraceCount tc{};
     trace_persistent<false, kBatch>(S, n, fetch, sink, tc);

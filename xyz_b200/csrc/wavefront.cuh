@@ -852,6 +852,11 @@ struct HitRing {
     base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32;
     stride = ((gridDim.x * blockDim.x) >> 5) * 32;
   }
+  // entries [begin, end) by this CTA's warps
+  XYZ_DEV HitRing(int32_t *r, int begin, int end) : ring(r), n(end), held(0), head(0) {
+    base = begin + static_cast<int>(threadIdx.x & ~31u);
+    stride = static_cast<int>(blockDim.x);
+  }
   // code_of(i): the hit code of entry i (negative: no hit)
   template <class CodeOf>
   XYZ_DEV int next(CodeOf code_of, bool *any) {
@@ -880,11 +885,10 @@ struct HitRing {
 // kModeGuided: directions from the learned guide mixed with Lambert sampling.
 // kModeImporton: directions from the light-importance histogram of the vertex
 // (the reference's importance-driven tracer).
-// Six CTAs per SM (80 registers): with full warps the kernel waits for its gathers
-// (1M-triangle frame, 10 bounces: 9.34 ms with a warp per 32 queue entries, with
-// the ring 6.78 at five CTAs, 6.62 at six, 6.64 at seven, 7.74 at eight).
+// The vertices of the hits that `hits` gives out, of bounce b; new queue entries
+// go to positions from q0 on, counted in cnt and cnt_next.
 template <int kMode>
-__global__ void __launch_bounds__(kThreads, kMode == kModeGuided ? 5 : 6) k_shade(WaveArgs A, int b) {
+XYZ_DEV void shade_queue(const WaveArgs &A, int b, HitRing &hits, int32_t *cnt, int32_t *cnt_next, int q0) {
   constexpr bool kAdj = kMode == kModeAdjoint;
   constexpr bool kBatch = kMode == kModeBatch;
   constexpr bool kGuide = kMode == kModeGuided;
@@ -892,12 +896,7 @@ __global__ void __launch_bounds__(kThreads, kMode == kModeGuided ? 5 : 6) k_shad
   // mirror and metal materials exist in plain and batched renders only (the
   // other modes refuse such scenes), so the other variants carry no code for them
   constexpr bool kSpecMat = kMode == kModePlain || kMode == kModeBatch;
-  if constexpr (kBatch) b = A.cursor->bounce;
-  int32_t *const cnt = A.counts + b * kCountStride;
-  int32_t *const cnt_next = A.counts + (b + 1) * kCountStride;
   int const qi = b & 1, qo = qi ^ 1;
-  __shared__ int32_t s_ring[kThreads / 32][64];
-  HitRing hits(s_ring[threadIdx.x >> 5], cnt[kCExt]);
   // the adjoint's primal pass records every entry's hit, its replay reads it
   auto code_of = [&](int i) -> int32_t {
     if (kAdj && A.hit_cache)
@@ -1273,7 +1272,7 @@ __global__ void __launch_bounds__(kThreads, kMode == kModeGuided ? 5 : 6) k_shad
         }
       }
     }
-    int32_t const js = warp_append(&cnt[kCShadow], push_sh);
+    int32_t const js = q0 + warp_append(&cnt[kCShadow], push_sh);
     if (push_sh) {
       A.s_o[js] = make_float4(lpos.x, lpos.y, lpos.z, kBatch ? __int_as_float(block) : __int_as_float(0x7f800000));
       A.s_d[js] = make_float4(vin.x, vin.y, vin.z, nk2nk3);
@@ -1283,7 +1282,7 @@ __global__ void __launch_bounds__(kThreads, kMode == kModeGuided ? 5 : 6) k_shad
       if (kGuide || kImp) A.s_slot[js] = __float_as_int(rho);
       if (sh_metal) A.s_m[js] = sm4;
     }
-    int32_t const je = warp_append(&cnt_next[kCExt], push_ext);
+    int32_t const je = q0 + warp_append(&cnt_next[kCExt], push_ext);
     if (push_ext) {
       A.q_o[qo][je] = make_float4(pos.x, pos.y, pos.z, kBatch ? __int_as_float(block) : kRayTMin);
       A.q_d[qo][je] = make_float4(dir.x, dir.y, dir.z, __int_as_float(0x7f800000));
@@ -1294,6 +1293,94 @@ __global__ void __launch_bounds__(kThreads, kMode == kModeGuided ? 5 : 6) k_shad
   }
 }
 
+
+// Six CTAs per SM (80 registers): with full warps the kernel waits for its gathers
+// (1M-triangle frame, 10 bounces: 9.34 ms with a warp per 32 queue entries, with
+// the ring 6.78 at five CTAs, 6.62 at six, 6.64 at seven, 7.74 at eight).
+template <int kMode>
+__global__ void __launch_bounds__(kThreads, kMode == kModeGuided ? 5 : 6) k_shade(WaveArgs A, int b) {
+  if constexpr (kMode == kModeBatch) b = A.cursor->bounce;
+  int32_t *const cnt = A.counts + b * kCountStride;
+  __shared__ int32_t s_ring[kThreads / 32][64];
+  HitRing hits(s_ring[threadIdx.x >> 5], cnt[kCExt]);
+  shade_queue<kMode>(A, b, hits, cnt, cnt + kCountStride, 0);
+}
+
+// ------------------------------------------------------------ small waves
+// BothSink over the queues of one CTA, whose entries lie from q0 on and were
+// written in this launch (no read-only loads).
+struct LocalSink {
+  static constexpr bool kTarget = true, kMixed = true;
+  ExtSink<false> ext;
+  ShadowSink<false> shadow;
+  int n_ext, q0;
+  XYZ_DEV int at(int i) const { return q0 + (i < n_ext ? i : i - n_ext); }
+  XYZ_DEV bool targeted(int i) const { return i >= n_ext; }
+  XYZ_DEV int32_t target(int i) const { return shadow.A->s_target[at(i)]; }
+  XYZ_DEV void load(int i, f3 &o, f3 &d, float &tmin, float &tmax) const {
+    if (i < n_ext)
+      ext.load(at(i), o, d, tmin, tmax);
+    else
+      shadow.load(at(i), o, d, tmin, tmax);
+  }
+  XYZ_DEV const DevScene *scene(int) const { return nullptr; }
+  XYZ_DEV void store(int i, const RayHit &h) {
+    if (i < n_ext)
+      ext.store(at(i), h);
+    else
+      shadow.store(at(i), h);
+  }
+};
+
+// All bounces of a wave after its camera rays in one launch: CTA c takes
+// paths [c * per_cta, (c + 1) * per_cta) through bounce after bounce with queues
+// and counters of its own, in the same stretch of the wave's buffers.  A launch
+// per bounce ends when the slowest of all rays does, 15 + 8 us a bounce however
+// few paths are left; here a CTA waits for its own rays only, and what a path
+// gets does not depend on who shares its queue.  A 64 x 64 preview of 15
+// bounces 362 -> 169 us.
+// Four CTAs per SM (128 registers: the shading and the traversal in one kernel),
+// half the warps of the kernels apart, which long queues need: renders of depth 10
+// (us), kernels apart / in one: 4,096 paths 301 / 159 (Cornell box), 534 / 184
+// (247,042-triangle mesh), 568 / 264 (room); 65,536 paths 392 / 218, 802 / 422,
+// 816 / 622; 131,072 paths 456 / 282, 970 / 543, 1042 / 1012; 262,144 paths
+// 549 / 414, 1312 / 804, 1430 / 1750.
+constexpr int64_t kSmallWave = int64_t{1} << 17;
+
+__global__ void __launch_bounds__(kThreads, 4) k_small_wave(WaveArgs A, int iters, int per_cta) {
+  __shared__ WideList s_list;
+  __shared__ int32_t s_ring[kThreads / 32][64];
+  __shared__ int32_t s_cnt[2][kCountStride];
+  int const q0 = static_cast<int>(blockIdx.x) * per_cta;
+  int const tid = static_cast<int>(threadIdx.x);
+  if (tid < 2 * kCountStride) s_cnt[tid / kCountStride][tid % kCountStride] = 0;
+  __syncthreads();
+  if (tid == 0) s_cnt[0][kCExt] = static_cast<int32_t>(min(static_cast<int64_t>(per_cta), A.npaths - q0));
+  __syncthreads();
+  for (int b = 0; b <= iters; ++b) {
+    int32_t *const cnt = s_cnt[b & 1], *const other = s_cnt[(b & 1) ^ 1];  // other: bounce b - 1, then b + 1
+    int const n_ext = cnt[kCExt], n_shadow = other[kCShadow];
+    int const qi = b & 1;
+    LocalSink sink{{A.q_o[qi], A.q_d[qi], A.hits, &A}, {&A, 0u, b - 1}, n_ext, q0};
+    if (n_ext + n_shadow > 0)
+      trace_closest_hits(A.S, n_ext + n_shadow, &cnt[kCFetchExt], sink, s_list, kThreads / 32);
+    uint32_t const visible = __reduce_add_sync(0xffffffffu, sink.shadow.visible);
+    if ((tid & 31) == 0 && visible) atomicAdd(&other[kCVisible], static_cast<int32_t>(visible));
+    __syncthreads();
+    if (tid < kCountStride) {
+      // the wave's totals (k_raygen counted its camera rays)
+      int32_t *const total = A.counts + b * kCountStride;
+      if (b > 0 && (tid == kCShadow || tid == kCVisible) && other[tid]) atomicAdd(&total[tid - kCountStride], other[tid]);
+      if (b > 0 && tid == kCExt && n_ext) atomicAdd(&total[tid], n_ext);
+      other[tid] = 0;
+    }
+    __syncthreads();
+    if (n_ext == 0) break;
+    HitRing hits(s_ring[tid >> 5], q0, q0 + n_ext);
+    shade_queue<kModePlain>(A, b, hits, cnt, other, q0);
+    __syncthreads();
+  }
+}
 
 // ------------------------------------------------------------ spectral shade
 // One vertex of the reference's spectral estimator, tgir::Scene::
