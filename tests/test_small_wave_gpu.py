@@ -1,5 +1,6 @@
-"""Waves of at most 2^17 paths run all their bounces in one launch; profiled
-renders launch every bounce's kernels.  Same film, same counters."""
+"""Waves of at most 2^17 paths run all their bounces in one launch, and larger
+ones the bounces after that few rays are left; profiled renders launch every
+bounce's kernels.  Same film, same counters."""
 
 import pytest
 
@@ -7,10 +8,11 @@ pytestmark = pytest.mark.gpu
 
 
 # one path; fewer paths than CTAs, one more, uneven shares; the rule's last size
-# and the first beyond it; several waves in a call
+# and the first beyond it; a wave taken over when it has thinned out; several waves
+# in a call
 @pytest.mark.parametrize("depth", [1, 2, 15])
 @pytest.mark.parametrize("shape", [(1, 1, 1, 0), (37, 16, 1, 0), (593, 1, 1, 0), (97, 61, 3, 0), (512, 256, 1, 0),
-                                   (43691, 3, 1, 0), (97, 61, 3, 5000)])
+                                   (43691, 3, 1, 0), (640, 480, 2, 0), (97, 61, 3, 5000)])
 @pytest.mark.parametrize("kind", ["box", "specular", "mesh"])
 def test_one_launch_gives_the_film_and_counters_of_many(kind, shape, depth):
     import torch

@@ -40,13 +40,6 @@ struct Grids {
   }
 };
 
-// As many paths a CTA as it takes for all CTAs to be resident.
-void launch_small_wave(const WaveArgs &A, int iters, int resident, cudaStream_t st) {
-  int64_t const per_cta = (A.npaths + resident - 1) / resident;
-  k_small_wave<<<static_cast<int>((A.npaths + per_cta - 1) / per_cta), kThreads, 0, st>>>(A, iters,
-                                                                                         static_cast<int>(per_cta));
-}
-
 Grids wave_grids(int device) {
   static std::mutex mu;
   static Grids table[64];
@@ -420,8 +413,10 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
         // Shadow rays go with the next bounce's extension rays (k_trace_both);
         // profiled renders keep the two classes apart.
         bool const both = prof == XYZGPU_PROFILE_OFF;
-        if (both && !adj && !guide && !imp && !spectral && A.npaths <= kSmallWave) {
-          launch_small_wave(A, iters, G.small_wave, st);
+        bool const plain = both && !adj && !guide && !imp && !spectral;
+        int const small_grid = static_cast<int>(std::min<int64_t>(G.small_wave, A.npaths));
+        if (plain && A.npaths <= kSmallWave) {
+          k_small_wave<<<small_grid, kThreads, 0, st>>>(A, iters, 0);
           ++launches;
           return XYZGPU_OK;
         }
@@ -461,6 +456,10 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
             ++launches;
           }
           XYZ_MARK(2, true);
+          if (plain && small_wave_at(b)) {
+            k_small_wave<<<small_grid, kThreads, 0, st>>>(A, iters, b);
+            ++launches;
+          }
           if (spectral)
             k_shade_spectral<<<G.shade_sp, kThreads, 0, st>>>(A, b);
           else if (imp)
@@ -774,9 +773,11 @@ int render_noalloc_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_r
       int const gr = static_cast<int>(std::min<int64_t>(dev.raygen, (A.npaths + kThreads - 1) / kThreads));
       k_raygen<false><<<gr, kThreads, 0, st>>>(A);
       bool const small = A.npaths <= kSmallWave;
-      if (small) launch_small_wave(A, iters, dev.small_wave, st);
+      int const small_grid = static_cast<int>(std::min<int64_t>(dev.small_wave, A.npaths));
+      if (small) k_small_wave<<<small_grid, kThreads, 0, st>>>(A, iters, 0);
       for (int b = 0; b < iters && !small; ++b) {
         if (b == 0) k_trace_queue<false, false><<<dev.trace_e, kThreads, 0, st>>>(A, b, tally + 8);
+        if (small_wave_at(b)) k_small_wave<<<small_grid, kThreads, 0, st>>>(A, iters, b);
         k_shade<kModePlain><<<dev.shade, kThreads, 0, st>>>(A, b);
         if (b + 1 < iters && A.npaths <= kMixedPaths)
           k_trace_both<true, kModePlain><<<dev.both[1], kThreads, 0, st>>>(A, b);
