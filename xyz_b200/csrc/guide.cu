@@ -766,7 +766,7 @@ __global__ void __launch_bounds__(kGuideThreads, 1)
 // Guide inference for a render's extension queue: the hit point and shading
 // normal of every queue entry (computed as the shading kernel does) through
 // the network; per entry the mixture (weights, concentrations, means) as 40
-// fp16 values.  Persistent CTAs of three groups; the queue length is read on
+// fp16 values.  Persistent CTAs of kGroups groups; the queue length is read on
 // the device.
 struct InferArgs {
   const float4 *qo, *qd, *hits;

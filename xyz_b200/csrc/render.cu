@@ -643,10 +643,10 @@ constexpr size_t seg(size_t bytes) { return (bytes + kSeg - 1) / kSeg * kSeg; }
 constexpr size_t kNoAllocF4 = seg(kNoAllocPaths * sizeof(float4));
 constexpr size_t kNoAllocI4 = seg(kNoAllocPaths * sizeof(int32_t));
 constexpr size_t kNoAllocCounts = seg((kNoAllocDepth + 2) * kCountStride * sizeof(int32_t));
-constexpr size_t kNoAllocTally = seg(16 * sizeof(unsigned long long));
+constexpr size_t kNoAllocSpare = 256;
 // beta, radiance, q_o[2], q_d[2], hits, s_o, s_d, s_pb: 10 float4 arrays;
-// misc, q_slot[2], s_target: 4 int arrays.
-constexpr size_t kNoAllocBytes = 10 * kNoAllocF4 + 4 * kNoAllocI4 + kNoAllocCounts + kNoAllocTally;
+// misc, q_slot[2], s_target: 4 int arrays.  (The size is part of the interface.)
+constexpr size_t kNoAllocBytes = 10 * kNoAllocF4 + 4 * kNoAllocI4 + kNoAllocCounts + kNoAllocSpare;
 static_assert(kNoAllocBytes == XYZGPU_NOALLOC_SCRATCH_BYTES,
               "XYZGPU_NOALLOC_SCRATCH_BYTES must match the scratch layout");
 
@@ -663,7 +663,7 @@ std::mutex g_noalloc_mu;
 // g_noalloc_mu, only once all of its fields are set.
 struct NoAllocDevice {
   unsigned char *base;
-  int raygen, trace_e, trace_s, both[2], shade, film, small_wave;
+  int raygen, film, small_wave;
 };
 NoAllocDevice g_noalloc_dev[64] = {};
 
@@ -681,11 +681,6 @@ int noalloc_device(int device, NoAllocDevice *out) {
                        cudaGetErrorString(e));
     NoAllocDevice d;
     d.raygen = occupancy_grid(k_raygen<false>, device);
-    d.trace_e = occupancy_grid(k_trace_queue<false, false>, device);
-    d.trace_s = occupancy_grid(k_trace_queue<true, false>, device);
-    d.both[0] = occupancy_grid(k_trace_both<false, kModePlain>, device);
-    d.both[1] = occupancy_grid(k_trace_both<true, kModePlain>, device);
-    d.shade = occupancy_grid(k_shade<kModePlain>, device);
     d.small_wave = occupancy_grid(k_small_wave, device);
     d.film = occupancy_grid(k_film, device);
     d.base = static_cast<unsigned char *>(p);
@@ -741,7 +736,6 @@ int render_noalloc_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_r
   for (int q = 0; q < 2; ++q) A.q_slot[q] = reinterpret_cast<int32_t *>(take(kNoAllocI4));
   A.s_target = reinterpret_cast<int32_t *>(take(kNoAllocI4));
   A.counts = reinterpret_cast<int32_t *>(take(kNoAllocCounts));
-  unsigned long long *tally = reinterpret_cast<unsigned long long *>(take(kNoAllocTally));
 
   A.S = s.dev;
   A.cam = camera_setup(cam, rp.width, rp.height);
@@ -756,7 +750,6 @@ int render_noalloc_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_r
   int64_t const cap = rp.wave_paths > 0 ? rp.wave_paths : kNoAllocPaths;
   int const iters = rp.max_depth;
   if (!rp.accumulate) XYZ_CUDA_TRY(cudaMemsetAsync(film, 0, 3 * npix_total * sizeof(float), st));
-  XYZ_CUDA_TRY(cudaMemsetAsync(tally, 0, kNoAllocTally, st));
   int64_t const spp_per_wave =
       std::max<int64_t>(1, std::min<int64_t>(rp.spp, cap / std::max<int64_t>(1, npix_total)));
   int64_t const pix_per_wave = std::min<int64_t>(npix_total, cap);
@@ -772,20 +765,8 @@ int render_noalloc_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_r
       XYZ_CUDA_TRY(cudaMemsetAsync(A.counts, 0, kNoAllocCounts, st));
       int const gr = static_cast<int>(std::min<int64_t>(dev.raygen, (A.npaths + kThreads - 1) / kThreads));
       k_raygen<false><<<gr, kThreads, 0, st>>>(A);
-      bool const small = A.npaths <= kSmallWave;
-      int const small_grid = static_cast<int>(std::min<int64_t>(dev.small_wave, A.npaths));
-      if (small) k_small_wave<<<small_grid, kThreads, 0, st>>>(A, iters, 0);
-      for (int b = 0; b < iters && !small; ++b) {
-        if (b == 0) k_trace_queue<false, false><<<dev.trace_e, kThreads, 0, st>>>(A, b, tally + 8);
-        if (small_wave_at(b)) k_small_wave<<<small_grid, kThreads, 0, st>>>(A, iters, b);
-        k_shade<kModePlain><<<dev.shade, kThreads, 0, st>>>(A, b);
-        if (b + 1 < iters && A.npaths <= kMixedPaths)
-          k_trace_both<true, kModePlain><<<dev.both[1], kThreads, 0, st>>>(A, b);
-        else if (b + 1 < iters)
-          k_trace_both<false, kModePlain><<<dev.both[0], kThreads, 0, st>>>(A, b);
-        else
-          k_trace_queue<true, false><<<dev.trace_s, kThreads, 0, st>>>(A, b, tally + 8);
-      }
+      static_assert(kNoAllocPaths <= kSmallWave, "all bounces of these waves run in one launch");
+      k_small_wave<<<static_cast<int>(std::min<int64_t>(dev.small_wave, A.npaths)), kThreads, 0, st>>>(A, iters, 0);
       int const gf = static_cast<int>(std::min<int64_t>(dev.film, (A.npix + kThreads - 1) / kThreads));
       k_film<<<gf, kThreads, 0, st>>>(A, film);
       XYZ_CUDA_TRY(cudaGetLastError());

@@ -19,6 +19,10 @@
 //                               triangle (xyz/bsdf/lambert.cpp:151-172)
 //   film                        film[p] += path radiance, samples in order
 //
+// The shadow trace of a bounce shares its launch with the next bounce's
+// extension trace (k_trace_both; apart in profiled renders), and in waves of few
+// paths, or once few are left, all bounces run in one launch (k_small_wave).
+//
 // Queue lengths live in device memory, so the host issues the whole sequence
 // without synchronising; kernels whose queue is empty return at once.
 // Queue appends are compacted per warp: a ballot over the lanes that append,
@@ -574,9 +578,9 @@ struct ShadowSink {
   }
 };
 
-// CTAs per SM: extension rays run at 9 (56 registers, no spills: 5 % faster
-// than 10 CTAs at 48 registers with ~50 bytes of spills), shadow rays at 10
-// (measured on B200, 1M-triangle scene).
+// CTAs per SM: 8 (64 registers) for the wide tree, which spills at 10 (+45 % on
+// the 1M-triangle scene); counted renders, on the kd-tree, run at 9 (extension
+// rays, 56 registers) and 10 (shadow rays, 48).
 template <bool kShadow, bool kCount, int kMode = kModePlain>
 __global__ void __launch_bounds__(kThreads, kCount ? (kShadow ? 10 : 9) : 8) k_trace_queue(WaveArgs A, int b,
                                                           unsigned long long *prof) {
