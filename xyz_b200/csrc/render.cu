@@ -21,7 +21,8 @@ constexpr int64_t kMaxGuidedWave = int64_t{1} << 23;
 struct Grids {
   int raygen, trace_e, trace_s, trace_s_adj, trace_s_guide, trace_s_imp;
   int both[2], both_sp[2], both_adj[2], both_guide[2], both_imp[2];  // [1]: k_trace_both<true>
-  int shade, shade_adj, shade_guide, shade_sp, shade_imp, film, small_wave;
+  int shade, shade_adj, shade_guide, shade_sp, shade_imp, film;
+  int small_wave[2];  // [1]: spectral
   // No larger than waves of `paths` paths can use: a queue is never longer, and
   // CTAs without work still cost their launch (a trace of one ray: 5.0 us with
   // the full grid, 3.8 with one CTA).  Traces get a CTA per 32 rays (8 a warp,
@@ -70,7 +71,8 @@ Grids wave_grids(int device) {
     g.trace_s_imp = occupancy_grid(k_trace_queue<true, false, kModeImporton>, device);
     g.shade_imp = occupancy_grid(k_shade<kModeImporton>, device);
     g.film = occupancy_grid(k_film, device);
-    g.small_wave = occupancy_grid(k_small_wave, device);
+    g.small_wave[0] = occupancy_grid(k_small_wave<false>, device);
+    g.small_wave[1] = occupancy_grid(k_small_wave<true>, device);
     table[d] = g;
     ready[d] = true;
   }
@@ -413,10 +415,11 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
         // Shadow rays go with the next bounce's extension rays (k_trace_both);
         // profiled renders keep the two classes apart.
         bool const both = prof == XYZGPU_PROFILE_OFF;
-        bool const plain = both && !adj && !guide && !imp && !spectral;
-        int const small_grid = static_cast<int>(std::min<int64_t>(G.small_wave, A.npaths));
+        bool const plain = both && !adj && !guide && !imp;
+        auto const small_wave = spectral ? k_small_wave<true> : k_small_wave<false>;
+        int const small_grid = static_cast<int>(std::min<int64_t>(G.small_wave[spectral], A.npaths));
         if (plain && A.npaths <= kSmallWave) {
-          k_small_wave<<<small_grid, kThreads, 0, st>>>(A, iters, 0);
+          small_wave<<<small_grid, kThreads, 0, st>>>(A, iters, 0);
           ++launches;
           return XYZGPU_OK;
         }
@@ -457,7 +460,7 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
           }
           XYZ_MARK(2, true);
           if (plain && small_wave_at(b)) {
-            k_small_wave<<<small_grid, kThreads, 0, st>>>(A, iters, b);
+            small_wave<<<small_grid, kThreads, 0, st>>>(A, iters, b);
             ++launches;
           }
           if (spectral)
@@ -681,7 +684,7 @@ int noalloc_device(int device, NoAllocDevice *out) {
                        cudaGetErrorString(e));
     NoAllocDevice d;
     d.raygen = occupancy_grid(k_raygen<false>, device);
-    d.small_wave = occupancy_grid(k_small_wave, device);
+    d.small_wave = occupancy_grid(k_small_wave<false>, device);
     d.film = occupancy_grid(k_film, device);
     d.base = static_cast<unsigned char *>(p);
     g_noalloc_dev[device] = d;
@@ -766,7 +769,7 @@ int render_noalloc_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_r
       int const gr = static_cast<int>(std::min<int64_t>(dev.raygen, (A.npaths + kThreads - 1) / kThreads));
       k_raygen<false><<<gr, kThreads, 0, st>>>(A);
       static_assert(kNoAllocPaths <= kSmallWave, "all bounces of these waves run in one launch");
-      k_small_wave<<<static_cast<int>(std::min<int64_t>(dev.small_wave, A.npaths)), kThreads, 0, st>>>(A, iters, 0);
+      k_small_wave<false><<<static_cast<int>(std::min<int64_t>(dev.small_wave, A.npaths)), kThreads, 0, st>>>(A, iters, 0);
       int const gf = static_cast<int>(std::min<int64_t>(dev.film, (A.npix + kThreads - 1) / kThreads));
       k_film<<<gf, kThreads, 0, st>>>(A, film);
       XYZ_CUDA_TRY(cudaGetLastError());

@@ -578,6 +578,11 @@ struct ShadowSink {
   }
 };
 
+// Set by k_small_wave when it takes over the rest of a wave (1 + the bounce): the
+// kernels of the bounces have nothing to do then.  In the last row of the
+// counters, which no bounce uses.
+XYZ_DEV int32_t *wave_taken(const WaveArgs &A) { return A.counts + A.kmax * kCountStride; }
+
 // CTAs per SM: 8 (64 registers) for the wide tree, which spills at 10 (+45 % on
 // the 1M-triangle scene); counted renders, on the kd-tree, run at 9 (extension
 // rays, 56 registers) and 10 (shadow rays, 48).
@@ -590,6 +595,8 @@ __global__ void __launch_bounds__(kThreads, kCount ? (kShadow ? 10 : 9) : 8) k_t
     if (b < 0) return;
   }
   int32_t *const cnt = A.counts + b * kCountStride;
+  // (the last bounce's shadow rays of a spectral wave, if it was taken over)
+  if (kShadow && !kCount && kMode == kModePlain && *wave_taken(A)) return;
   int const n = kShadow ? cnt[kCShadow] : cnt[kCExt];
   int const lane = threadIdx.x & 31;
   int const qi = b & 1;
@@ -647,11 +654,6 @@ __global__ void __launch_bounds__(kThreads, kCount ? (kShadow ? 10 : 9) : 8) k_t
 // / 5.66 / 5.78, 67 M paths of the 1M-triangle mesh 44.3 / 44.4 / 42.6.
 constexpr int64_t kMixedPaths = int64_t{1} << 18;
 
-// Set by k_small_wave when it takes over the rest of a wave (1 + the bounce): the
-// kernels of the bounces have nothing to do then.  In the last row of the
-// counters, which no bounce uses.
-XYZ_DEV int32_t *wave_taken(const WaveArgs &A) { return A.counts + A.kmax * kCountStride; }
-
 template <bool kSpec, int kMode>
 struct BothSink {
   static constexpr bool kTarget = true, kMixed = true;
@@ -682,7 +684,7 @@ __global__ void __launch_bounds__(kThreads, kMixed ? 7 : 8) k_trace_both(WaveArg
   constexpr bool kBatch = kMode == kModeBatch;
   static_assert(!(kMixed && kBatch), "a mixed queue holds rays of one scene");
   if constexpr (kBatch) b = A.cursor->bounce - 1;
-  if (kMode == kModePlain && !kSpec && *wave_taken(A)) return;
+  if (kMode == kModePlain && *wave_taken(A)) return;
   int32_t *const next = A.counts + (b + 1) * kCountStride, *const cnt = b >= 0 ? next - kCountStride : next;
   int const qi = (b + 1) & 1, n_ext = next[kCExt], n_shadow = b >= 0 ? cnt[kCShadow] : 0;
   __shared__ WideList s_list;
@@ -1316,103 +1318,6 @@ __global__ void __launch_bounds__(kThreads, kMode == kModeGuided ? 5 : 6) k_shad
   shade_queue<kMode>(A, b, hits, cnt, cnt + kCountStride, 0);
 }
 
-// ------------------------------------------------------------ small waves
-// BothSink over the queues of one CTA, whose entries lie from q0 on and were
-// written in this launch (no read-only loads).
-struct LocalSink {
-  static constexpr bool kTarget = true, kMixed = true;
-  ExtSink<false> ext;
-  ShadowSink<false> shadow;
-  int n_ext, q0;
-  XYZ_DEV int at(int i) const { return q0 + (i < n_ext ? i : i - n_ext); }
-  XYZ_DEV bool targeted(int i) const { return i >= n_ext; }
-  XYZ_DEV int32_t target(int i) const { return shadow.A->s_target[at(i)]; }
-  XYZ_DEV void load(int i, f3 &o, f3 &d, float &tmin, float &tmax) const {
-    if (i < n_ext)
-      ext.load(at(i), o, d, tmin, tmax);
-    else
-      shadow.load(at(i), o, d, tmin, tmax);
-  }
-  XYZ_DEV const DevScene *scene(int) const { return nullptr; }
-  XYZ_DEV void store(int i, const RayHit &h) {
-    if (i < n_ext)
-      ext.store(at(i), h);
-    else
-      shadow.store(at(i), h);
-  }
-};
-
-// The rest of a wave from bounce b0 on in one launch: CTA c takes the c-th
-// share of the extension queue through bounce after bounce with queues and
-// counters of its own, in the same stretch of the wave's buffers.  A launch per bounce ends when the
-// slowest of all rays does, 15 + 8 us a bounce however few paths are left; here
-// a CTA waits for its own rays only, and what a path gets does not depend on who
-// shares its queue.  A 64 x 64 preview of 15 bounces 362 -> 169 us.
-// Four CTAs per SM (128 registers: the shading and the traversal in one kernel),
-// half the warps of the kernels apart, which long queues need: renders of depth 10
-// (us), kernels apart / in one: 4,096 paths 301 / 159 (Cornell box), 534 / 184
-// (247,042-triangle mesh), 568 / 264 (room); 65,536 paths 392 / 218, 802 / 422,
-// 816 / 622; 131,072 paths 456 / 282, 970 / 543, 1042 / 1012; 262,144 paths
-// 549 / 414, 1312 / 804, 1430 / 1750.
-// Larger waves: launched before the shading of every second bounce from the
-// fifth on (small_wave_at), it takes over once that few rays are left (traced
-// already: a path's shadow ray of the bounce before is in another CTA's share) and
-// is empty until then.  Depth 10, without / with it: 204,800 paths 476 / 447 us
-// (box), 1097 / 1017 (mesh), 1622 / 1463 (1M-triangle mesh), 1275 / 1275 (room);
-// 4.2 M paths 3303 / 3316, 3856 / 3671, 4816 / 4435, 13369 / 13396.  Before every
-// bounce the empty launches cost a closed room up to 4 % and a box of depth 4
-// 13 %; taking over at 2^15 or 2^16 rays gains the meshes a third to two
-// thirds as much.
-constexpr int64_t kSmallWave = int64_t{1} << 17;
-constexpr bool small_wave_at(int b) { return b >= 4 && (b & 1) == 0; }
-
-__global__ void __launch_bounds__(kThreads, 4) k_small_wave(WaveArgs A, int iters, int b0) {
-  __shared__ WideList s_list;
-  __shared__ int32_t s_ring[kThreads / 32][64];
-  __shared__ int32_t s_cnt[2][kCountStride];
-  int const tid = static_cast<int>(threadIdx.x);
-  int const n = A.counts[b0 * kCountStride + kCExt];
-  if (b0 > 0) {
-    // (every CTA finds the same: no kernel of this launch changes n, and the
-    // mark only to this bounce's)
-    int32_t const mark = *static_cast<volatile int32_t *>(wave_taken(A));
-    if ((mark != 0 && mark != b0 + 1) || n > kSmallWave) return;
-    if (tid == 0) *static_cast<volatile int32_t *>(wave_taken(A)) = b0 + 1;
-  }
-  int const per_cta = (n + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
-  int const q0 = static_cast<int>(blockIdx.x) * per_cta;
-  if (q0 >= n) return;
-  if (tid < 2 * kCountStride) s_cnt[tid / kCountStride][tid % kCountStride] = 0;
-  __syncthreads();
-  if (tid == 0) s_cnt[b0 & 1][kCExt] = min(per_cta, n - q0);
-  __syncthreads();
-  for (int b = b0; b <= iters; ++b) {
-    int32_t *const cnt = s_cnt[b & 1], *const other = s_cnt[(b & 1) ^ 1];  // other: bounce b - 1, then b + 1
-    int const n_ext = cnt[kCExt], n_shadow = other[kCShadow];
-    int const qi = b & 1;
-    if ((b == 0 || b > b0) && n_ext + n_shadow > 0) {
-      LocalSink sink{{A.q_o[qi], A.q_d[qi], A.hits, &A}, {&A, 0u, b - 1}, n_ext, q0};
-      trace_closest_hits(A.S, n_ext + n_shadow, &cnt[kCFetchExt], sink, s_list, kThreads / 32);
-      uint32_t const visible = __reduce_add_sync(0xffffffffu, sink.shadow.visible);
-      if ((tid & 31) == 0 && visible) atomicAdd(&other[kCVisible], static_cast<int32_t>(visible));
-    }
-    __syncthreads();
-    if (tid < kCountStride) {
-      // the wave's totals (the rays of bounce b0 are counted)
-      int32_t *const total = A.counts + b * kCountStride;
-      if (b > b0 && (tid == kCShadow || tid == kCVisible) && other[tid])
-        atomicAdd(&total[tid - kCountStride], other[tid]);
-      if (b > b0 && tid == kCExt && n_ext) atomicAdd(&total[tid], n_ext);
-      other[tid] = 0;
-    }
-    __syncthreads();
-    if (n_ext == 0) break;
-    HitRing hits(s_ring[tid >> 5], q0, q0 + n_ext);
-    shade_queue<kModePlain>(A, b, hits, cnt, other, q0);
-    __syncthreads();
-  }
-}
-
 // ------------------------------------------------------------ spectral shade
 // One vertex of the reference's spectral estimator, tgir::Scene::
 // EvaluteRussianRoulette (renderer/core/SceneStrategy.cpp:60-145), for H hero
@@ -1455,16 +1360,12 @@ XYZ_DEV float4 spd_values(const WaveArgs &A, const float *spd, const HeroSet &hs
 
 XYZ_DEV float4 mul4(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
 
-__global__ void __launch_bounds__(kThreads, 6) k_shade_spectral(WaveArgs A, int b) {
-  int32_t *const cnt = A.counts + b * kCountStride;
-  int32_t *const cnt_next = A.counts + (b + 1) * kCountStride;
+// shade_queue of a spectral wave; s_light: the light's spectrum in shared memory
+// (the lanes read different bins).
+XYZ_DEV void shade_spectral_queue(const WaveArgs &A, int b, HitRing &hits, int32_t *cnt, int32_t *cnt_next, int q0,
+                                  const float *s_light) {
   int const qi = b & 1, qo = qi ^ 1;
   DevScene const &S = A.S;
-  __shared__ float s_light[kSpecBins];  // the lanes read different bins
-  if (threadIdx.x < kSpecBins) s_light[threadIdx.x] = S.spd_light[threadIdx.x];
-  __syncthreads();
-  __shared__ int32_t s_ring[kThreads / 32][64];
-  HitRing hits(s_ring[threadIdx.x >> 5], cnt[kCExt]);
   for (;;) {
     bool any;
     int const i = hits.next([&](int j) { return __float_as_int(A.hits[j].w); }, &any);
@@ -1605,7 +1506,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_shade_spectral(WaveArgs A, int 
         }
       }
     }
-    int32_t const js = warp_append(&cnt[kCShadow], push_sh);
+    int32_t const js = q0 + warp_append(&cnt[kCShadow], push_sh);
     if (push_sh) {
       A.s_o[js] = make_float4(lpos.x, lpos.y, lpos.z, __int_as_float(0x7f800000));
       A.s_d[js] = make_float4(vin.x, vin.y, vin.z, nk2nk3);
@@ -1613,7 +1514,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_shade_spectral(WaveArgs A, int 
       A.s_slot[js] = slot;
       A.s_target[js] = tri;
     }
-    int32_t const je = warp_append(&cnt_next[kCExt], push_ext);
+    int32_t const je = q0 + warp_append(&cnt_next[kCExt], push_ext);
     if (push_ext) {
       A.q_o[qo][je] = make_float4(pos.x, pos.y, pos.z, kRayTMin);
       A.q_d[qo][je] = make_float4(dir.x, dir.y, dir.z, __int_as_float(0x7f800000));
@@ -1622,6 +1523,123 @@ __global__ void __launch_bounds__(kThreads, 6) k_shade_spectral(WaveArgs A, int 
       A.fsn[slot] = fsn_out;
       A.misc[slot] = misc;
     }
+  }
+}
+
+__global__ void __launch_bounds__(kThreads, 6) k_shade_spectral(WaveArgs A, int b) {
+  int32_t *const cnt = A.counts + b * kCountStride;
+  __shared__ float s_light[kSpecBins];
+  if (threadIdx.x < kSpecBins) s_light[threadIdx.x] = A.S.spd_light[threadIdx.x];
+  __syncthreads();
+  __shared__ int32_t s_ring[kThreads / 32][64];
+  HitRing hits(s_ring[threadIdx.x >> 5], *wave_taken(A) ? 0 : cnt[kCExt]);
+  shade_spectral_queue(A, b, hits, cnt, cnt + kCountStride, 0, s_light);
+}
+
+// ------------------------------------------------------------ small waves
+// BothSink over the queues of one CTA, whose entries lie from q0 on and were
+// written in this launch (no read-only loads).
+template <bool kSpec>
+struct LocalSink {
+  static constexpr bool kTarget = true, kMixed = true;
+  ExtSink<false> ext;
+  ShadowSink<kSpec> shadow;
+  int n_ext, q0;
+  XYZ_DEV int at(int i) const { return q0 + (i < n_ext ? i : i - n_ext); }
+  XYZ_DEV bool targeted(int i) const { return i >= n_ext; }
+  XYZ_DEV int32_t target(int i) const { return shadow.A->s_target[at(i)]; }
+  XYZ_DEV void load(int i, f3 &o, f3 &d, float &tmin, float &tmax) const {
+    if (i < n_ext)
+      ext.load(at(i), o, d, tmin, tmax);
+    else
+      shadow.load(at(i), o, d, tmin, tmax);
+  }
+  XYZ_DEV const DevScene *scene(int) const { return nullptr; }
+  XYZ_DEV void store(int i, const RayHit &h) {
+    if (i < n_ext)
+      ext.store(at(i), h);
+    else
+      shadow.store(at(i), h);
+  }
+};
+
+// The rest of a wave from bounce b0 on in one launch: CTA c takes the c-th
+// share of the extension queue through bounce after bounce with queues and
+// counters of its own, in the same stretch of the wave's buffers.  A launch per bounce ends when the
+// slowest of all rays does, 15 + 8 us a bounce however few paths are left; here
+// a CTA waits for its own rays only, and what a path gets does not depend on who
+// shares its queue.  A 64 x 64 preview of 15 bounces 362 -> 169 us.
+// Four CTAs per SM (128 registers: the shading and the traversal in one kernel),
+// half the warps of the kernels apart, which long queues need: renders of depth 10
+// (us), kernels apart / in one: 4,096 paths 301 / 159 (Cornell box), 534 / 184
+// (247,042-triangle mesh), 568 / 264 (room); 65,536 paths 392 / 218, 802 / 422,
+// 816 / 622; 131,072 paths 456 / 282, 970 / 543, 1042 / 1012; 262,144 paths
+// 549 / 414, 1312 / 804, 1430 / 1750.
+// Larger waves: launched before the shading of every second bounce from the
+// fifth on (small_wave_at), it takes over once that few rays are left (traced
+// already: a path's shadow ray of the bounce before is in another CTA's share) and
+// is empty until then.  Depth 10, without / with it: 204,800 paths 476 / 447 us
+// (box), 1097 / 1017 (mesh), 1622 / 1463 (1M-triangle mesh), 1275 / 1275 (room);
+// 4.2 M paths 3303 / 3316, 3856 / 3671, 4816 / 4435, 13369 / 13396.  Before every
+// Spectral waves (kSpec) alike: continuous, depth 10, 2,304 paths 325 / 179 us (box),
+// 486 / 199 (mesh); 131,072 paths 454 / 305, 966 / 542; 524,288 paths 790 / 729,
+// 1673 / 1490.
+// Before every bounce the empty launches cost a closed room up to 4 % and a box of depth 4
+// 13 %; taking over at 2^15 or 2^16 rays gains the meshes a third to two
+// thirds as much.
+constexpr int64_t kSmallWave = int64_t{1} << 17;
+constexpr bool small_wave_at(int b) { return b >= 4 && (b & 1) == 0; }
+
+template <bool kSpec>
+__global__ void __launch_bounds__(kThreads, 4) k_small_wave(WaveArgs A, int iters, int b0) {
+  __shared__ WideList s_list;
+  __shared__ int32_t s_ring[kThreads / 32][64];
+  __shared__ int32_t s_cnt[2][kCountStride];
+  int const tid = static_cast<int>(threadIdx.x);
+  int const n = A.counts[b0 * kCountStride + kCExt];
+  if (b0 > 0) {
+    // (every CTA finds the same: no kernel of this launch changes n, and the
+    // mark only to this bounce's)
+    int32_t const mark = *static_cast<volatile int32_t *>(wave_taken(A));
+    if ((mark != 0 && mark != b0 + 1) || n > kSmallWave) return;
+    if (tid == 0) *static_cast<volatile int32_t *>(wave_taken(A)) = b0 + 1;
+  }
+  int const per_cta = (n + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+  int const q0 = static_cast<int>(blockIdx.x) * per_cta;
+  if (q0 >= n) return;
+  __shared__ float s_light[kSpecBins];
+  if (kSpec && tid < kSpecBins) s_light[tid] = A.S.spd_light[tid];
+  if (tid < 2 * kCountStride) s_cnt[tid / kCountStride][tid % kCountStride] = 0;
+  __syncthreads();
+  if (tid == 0) s_cnt[b0 & 1][kCExt] = min(per_cta, n - q0);
+  __syncthreads();
+  for (int b = b0; b <= iters; ++b) {
+    int32_t *const cnt = s_cnt[b & 1], *const other = s_cnt[(b & 1) ^ 1];  // other: bounce b - 1, then b + 1
+    int const n_ext = b < iters ? cnt[kCExt] : 0, n_shadow = other[kCShadow];
+    int const qi = b & 1;
+    if ((b == 0 || b > b0) && n_ext + n_shadow > 0) {
+      LocalSink<kSpec> sink{{A.q_o[qi], A.q_d[qi], A.hits, &A}, {&A, 0u, b - 1}, n_ext, q0};
+      trace_closest_hits(A.S, n_ext + n_shadow, &cnt[kCFetchExt], sink, s_list, kThreads / 32);
+      uint32_t const visible = __reduce_add_sync(0xffffffffu, sink.shadow.visible);
+      if ((tid & 31) == 0 && visible) atomicAdd(&other[kCVisible], static_cast<int32_t>(visible));
+    }
+    __syncthreads();
+    if (tid < kCountStride) {
+      // the wave's totals (the rays of bounce b0 are counted)
+      int32_t *const total = A.counts + b * kCountStride;
+      if (b > b0 && (tid == kCShadow || tid == kCVisible) && other[tid])
+        atomicAdd(&total[tid - kCountStride], other[tid]);
+      if (b > b0 && tid == kCExt && n_ext) atomicAdd(&total[tid], n_ext);
+      other[tid] = 0;
+    }
+    __syncthreads();
+    if (n_ext == 0) break;
+    HitRing hits(s_ring[tid >> 5], q0, q0 + n_ext);
+    if constexpr (kSpec)
+      shade_spectral_queue(A, b, hits, cnt, other, q0, s_light);
+    else
+      shade_queue<kModePlain>(A, b, hits, cnt, other, q0);
+    __syncthreads();
   }
 }
 
