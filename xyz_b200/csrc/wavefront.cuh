@@ -1580,13 +1580,13 @@ struct LocalSink {
 // already: a path's shadow ray of the bounce before is in another CTA's share) and
 // is empty until then.  Depth 10, without / with it: 204,800 paths 476 / 447 us
 // (box), 1097 / 1017 (mesh), 1622 / 1463 (1M-triangle mesh), 1275 / 1275 (room);
-// 4.2 M paths 3303 / 3316, 3856 / 3671, 4816 / 4435, 13369 / 13396.  Before every
+// 4.2 M paths 3303 / 3316, 3856 / 3671, 4816 / 4435, 13369 / 13396.
 // Spectral waves (kSpec) alike: continuous, depth 10, 2,304 paths 325 / 179 us (box),
 // 486 / 199 (mesh); 131,072 paths 454 / 305, 966 / 542; 524,288 paths 790 / 729,
 // 1673 / 1490.
-// Before every bounce the empty launches cost a closed room up to 4 % and a box of depth 4
-// 13 %; taking over at 2^15 or 2^16 rays gains the meshes a third to two
-// thirds as much.
+// Launched before every bounce, the empty launches cost a closed room up to 4 %
+// and an early take-over a box of depth 4 13 %; taking over at 2^15 or 2^16 rays
+// gains the meshes a third to two thirds as much.
 constexpr int64_t kSmallWave = int64_t{1} << 17;
 constexpr bool small_wave_at(int b) { return b >= 4 && (b & 1) == 0; }
 
