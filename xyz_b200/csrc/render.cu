@@ -415,7 +415,7 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
         // Shadow rays go with the next bounce's extension rays (k_trace_both);
         // profiled renders keep the two classes apart.
         bool const both = prof == XYZGPU_PROFILE_OFF;
-        bool const plain = both && !adj && !guide && !imp;
+        bool const plain = both && !replay && !guide && !imp;  // (an adjoint's primal pass is one)
         auto const small_wave = spectral ? k_small_wave<true> : k_small_wave<false>;
         int const small_grid = static_cast<int>(std::min<int64_t>(G.small_wave[spectral], A.npaths));
         if (plain && A.npaths <= kSmallWave) {
@@ -459,7 +459,7 @@ int render_launch(SceneImpl &s, const xyzgpu_camera &cam, const xyzgpu_render_pa
             ++launches;
           }
           XYZ_MARK(2, true);
-          if (plain && small_wave_at(b)) {
+          if (plain && small_wave_at(b, iters)) {
             small_wave<<<small_grid, kThreads, 0, st>>>(A, iters, b);
             ++launches;
           }

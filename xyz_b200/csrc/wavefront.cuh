@@ -1576,7 +1576,8 @@ struct LocalSink {
 // 816 / 622; 131,072 paths 456 / 282, 970 / 543, 1042 / 1012; 262,144 paths
 // 549 / 414, 1312 / 804, 1430 / 1750.
 // Larger waves: launched before the shading of every second bounce from the
-// fifth on (small_wave_at), it takes over once that few rays are left (traced
+// fifth on while four are left (small_wave_at; with two left the adjoint below of
+// 262,144 paths loses 2 %), it takes over once that few rays are left (traced
 // already: a path's shadow ray of the bounce before is in another CTA's share) and
 // is empty until then.  Depth 10, without / with it: 204,800 paths 476 / 447 us
 // (box), 1097 / 1017 (mesh), 1622 / 1463 (1M-triangle mesh), 1275 / 1275 (room);
@@ -1584,11 +1585,14 @@ struct LocalSink {
 // Spectral waves (kSpec) alike: continuous, depth 10, 2,304 paths 325 / 179 us (box),
 // 486 / 199 (mesh); 131,072 paths 454 / 305, 966 / 542; 524,288 paths 790 / 729,
 // 1673 / 1490.
+// An adjoint's primal pass takes it too: forward and backward of 4,096 / 32,768 /
+// 131,072 / 262,144 paths of a room 572 / 758 / 1574 / 2406 -> 506 / 669 / 1504 /
+// 2392 us.
 // Launched before every bounce, the empty launches cost a closed room up to 4 %
 // and an early take-over a box of depth 4 13 %; taking over at 2^15 or 2^16 rays
 // gains the meshes a third to two thirds as much.
 constexpr int64_t kSmallWave = int64_t{1} << 17;
-constexpr bool small_wave_at(int b) { return b >= 4 && (b & 1) == 0; }
+constexpr bool small_wave_at(int b, int iters) { return b >= 4 && (b & 1) == 0 && b + 4 <= iters; }
 
 template <bool kSpec>
 __global__ void __launch_bounds__(kThreads, 4) k_small_wave(WaveArgs A, int iters, int b0) {
