@@ -1,0 +1,93 @@
+"""The wide tree's answers where rounding decides: rays aimed at and beside the
+edges of slivers, on the CPU against a host kd loop (tests/cpp/wide_kd_check.cpp)
+and on the GPU against counting calls, which walk the kd-tree.  Equal in every bit."""
+
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def check(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("wide") / "wide_kd_check")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-I/usr/local/cuda/include",
+                    os.path.join(ROOT, "tests", "cpp", "wide_kd_check.cpp"),
+                    os.path.join(ROOT, "xyz_b200", "csrc", "kdbuild_host.cpp"), "-o", exe], check=True)
+
+    def run(scene, rays, kind):
+        r = subprocess.run([exe, scene, str(rays), kind], capture_output=True, text=True, check=True)
+        return [float(x) for x in r.stdout.split()]
+    return run
+
+
+@pytest.mark.parametrize("scene", ["sliver:1e-2", "sliver:1e-3", "sliver:1e-4", "sliver:1e-5", "soup:0.1", "boxes"])
+def test_answers_beside_edges(check, scene):
+    rays, hits, unsettled, differ = check(scene, 200000, "edge")[:4]
+    assert hits > rays / 10 and unsettled < rays / 1000
+    assert differ == 0
+
+
+def scene_of(pos):
+    """A scene of loose triangles, the last of them a light."""
+    from xyz_b200 import scenes
+    n = pos.shape[0]
+    mat = np.zeros(n, np.int32)
+    mat[-1] = 1
+    return scenes.SceneData(pos.reshape(-1, 3).astype(np.float32), np.arange(3 * n, dtype=np.int32).reshape(-1, 3), mat,
+                            np.full((2, 3), 0.5, np.float32), np.array([0, 1], np.int32), np.ones(3, np.float32))
+
+
+def slivers(width, seed=1, n=200):
+    rng = np.random.default_rng(seed)
+    c, a = rng.uniform(-1, 1, (n, 3)), rng.normal(size=(n, 3))
+    a /= np.linalg.norm(a, axis=1, keepdims=True)
+    b = np.cross(a, rng.normal(size=(n, 3)))
+    b /= np.linalg.norm(b, axis=1, keepdims=True)
+    l, s = rng.uniform(0.3, 1.0, (2, n, 1))
+    return np.stack([c, c + l * a, c + l * s * a + width * l * b], 1)
+
+
+def edge_rays(pos, n, seed):
+    """Rays at points 1e-7 to 1e-1 of a triangle inside or beyond one of its edges."""
+    rng = np.random.default_rng(seed)
+    t = pos[rng.integers(0, pos.shape[0], n)].astype(np.float64)
+    k = rng.integers(0, 3, n)
+    i = np.arange(n)
+    a, b, c = t[i, k], t[i, (k + 1) % 3], t[i, (k + 2) % 3]
+    e = a + rng.uniform(0, 1, (n, 1)) * (b - a)
+    p = e + 10.0 ** rng.uniform(-7, -1, (n, 1)) * np.where(rng.random((n, 1)) < 0.75, 1, -1) * (e - c)
+    d = rng.normal(size=(n, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    size = 0.5 * np.ptp(pos.reshape(-1, 3), axis=0).max()
+    r = np.empty((n, 8), np.float32)
+    r[:, 0:3] = p - d * size * 10.0 ** rng.uniform(-1.5, 0.5, (n, 1))
+    r[:, 3] = 1e-5
+    r[:, 4:7] = d
+    r[:, 7] = np.inf
+    return r
+
+
+def compare(sd, rays, **build):
+    """Hits of the rays by the wide tree and by the kd-tree; returns the number of hits."""
+    import torch
+    from xyz_b200 import api
+    rays = torch.from_numpy(rays).cuda()
+    with api.Scene(sd, **build) as s:
+        a, b = (torch.empty((rays.shape[0], 4), dtype=torch.float32, device="cuda") for _ in range(2))
+        s.trace_device(rays, a)
+        c = s.trace_device(rays, b, counted=True)
+    same = (a.view(torch.int32) == b.view(torch.int32)).all(1)
+    assert bool(same.all()), int((~same).sum())
+    return c["hits"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width", [1e-2, 1e-3, 1e-4, 1e-5])
+@pytest.mark.parametrize("builder", ["device", "host"])
+def test_sliver_hits_equal_the_kd_tree(width, builder):
+    pos = slivers(width).astype(np.float32)
+    assert compare(scene_of(pos), edge_rays(pos, 1 << 20, 3), builder=builder) > 1 << 17

@@ -995,16 +995,16 @@ __global__ void k_wide_assign(const float4 *__restrict__ tri, int n, const uint2
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     float4 const a = tri[3 * i], b = tri[3 * i + 1], c = tri[3 * i + 2];
     // vertices as the intersection test sees them: v0, v0 + e1, v0 + e2
-    f3 const v0 = xyz3(a), v1 = add3(v0, xyz3(b)), v2 = add3(v0, xyz3(c));
-    int32_t const leaf = wide_leaf_of(nodes, scl3(add3(add3(v0, v1), v2), 1.0f / 3.0f));
+    f3 const v0 = xyz3(a), e1 = xyz3(b), e2 = xyz3(c);
+    int32_t const leaf = wide_leaf_of(nodes, scl3(add3(add3(v0, add3(v0, e1)), add3(v0, e2)), 1.0f / 3.0f));
+    WideTri const w = wide_triangle(v0, e1, e2, mk3(a.w, b.w, c.w));
     owner[i] = leaf;
     uint32_t *const lo = reinterpret_cast<uint32_t *>(T.lo + leaf);
     uint32_t *const hi = reinterpret_cast<uint32_t *>(T.hi + leaf);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      float const x = comp3(v0, k), y = comp3(v1, k), z = comp3(v2, k);
-      atomicMin(lo + k, float_key(fminf(fminf(x, y), z)));
-      atomicMax(hi + k, float_key(fmaxf(fmaxf(x, y), z)));
+      atomicMin(lo + k, float_key(w.lo[k]));
+      atomicMax(hi + k, float_key(w.hi[k]));
     }
     atomicAdd(hi + 3, 1u);
   }
@@ -1058,7 +1058,8 @@ __global__ void k_wide_tris(const float4 *__restrict__ tri, int n, WideSets T, c
     out[rec] = a;
     out[rec + 1] = b;
     out[rec + 2] = c;
-    out[rec + 3] = make_float4(__int_as_float(i), norm1(xyz3(b)) + norm1(xyz3(c)), norm1(mk3(a.w, b.w, c.w)), 0.0f);
+    WideTri const w = wide_triangle(xyz3(a), xyz3(b), xyz3(c), mk3(a.w, b.w, c.w));
+    out[rec + 3] = make_float4(__int_as_float(i), w.e, w.n, 0.0f);
   }
 }
 

@@ -30,52 +30,6 @@ struct TraceCount {
   uint32_t nodes, leaves, tris;
 };
 
-struct RayHit {
-  float t, f, g;
-  int32_t id;    // triangle id, -1 = miss
-  int32_t back;  // 1 = hit from the back side (det > 0)
-};
-
-// FindIntersectionDF (xyz/geom/triangle.cpp:127-165) on a packed triangle
-// (a, b, c): the hit within [tmin, tmax], its side and 1 / det.
-XYZ_DEV bool test_triangle(float4 a, float4 b, float4 c, f3 o, f3 d, float tmin, float tmax, float *t_out,
-                           float *f_out, float *g_out, int32_t *back_out, float *inv_out) {
-  f3 const e2xe1 = mk3(a.w, b.w, c.w);
-  float const det = dot3(d, e2xe1);
-  if (fabsf(det) < kEpsilon) return false;
-  float const inv_det = __frcp_rn(det);
-  f3 const vmo = sub3(xyz3(a), o);
-  float const t = inv_det * dot3(vmo, e2xe1);
-  if ((t < tmin) || (tmax < t)) return false;
-  f3 const dxvmo = cross3(d, vmo);
-  float const f = inv_det * dot3(xyz3(c), dxvmo);
-  if ((f < 0.0f) || (f > 1.0f)) return false;
-  float const g = inv_det * -dot3(xyz3(b), dxvmo);
-  if ((g < 0.0f) || ((f + g) > 1.0f)) return false;
-  *t_out = t;
-  *f_out = f;
-  *g_out = g;
-  *back_out = det > 0.0f;
-  *inv_out = inv_det;
-  return true;
-}
-
-// The test on triangle i of the scene; updates best_t on acceptance.
-XYZ_DEV bool hit_triangle(const float4 *__restrict__ tri, int32_t i, f3 o, f3 d, float tmin,
-                          RayHit &h) {
-  float t, f, g, inv_det;
-  int32_t back;
-  if (!test_triangle(__ldg(&tri[3 * i + 0]), __ldg(&tri[3 * i + 1]), __ldg(&tri[3 * i + 2]), o, d, tmin, h.t, &t, &f,
-                     &g, &back, &inv_det))
-    return false;
-  h.t = t;
-  h.f = f;
-  h.g = g;
-  h.id = i;
-  h.back = back;
-  return true;
-}
-
 // A deferred far child: its node and exit distance.  Its entry distance is
 // not stored: in front-to-back order the far child pushed last is popped
 // right after the subtree that ends at its split plane, so the entry equals
@@ -293,17 +247,21 @@ XYZ_DEV void trace_persistent(const DevScene &S, int n, int *fetch, Sink &sink, 
 // order of the tests or the choice of the cells decides: a hit so close to an
 // edge of its triangle that rounding decides whether the ray's kd cells hold
 // it, or two hits whose distances differ by less than their rounding.  Such
-// rays are recognised while they are traced (wide_margin: the hit is closer
-// to an edge, or a second accepted hit closer in distance, than the error
-// bound of the test).  About 0.1 to 1 % of the rays are (edges of a 1M-triangle
-// mesh).  Where no split plane of the kd-tree passes within the error of the hit
-// point (wide_settled), all these hits lie in the one leaf that holds it, whose
-// triangles the kd loop tests in ascending order: it keeps the nearest, and of
-// equal distances the highest id, which is what this loop keeps.  The rest
-// (1 % of the 1 %), and rays the wide tree cannot serve (wide_usable), go into
-// a list of the warp in shared memory and are traced through the kd-tree once
-// the list is full or the queue is empty.  Everywhere else a correct traversal
-// of either tree finds the same triangle.
+// rays are recognised while they are traced (wide_take: 0.1 to 1 % of them on a
+// 1M-triangle mesh), and the leaf of the kd-tree in which the kd loop would stop says
+// what it would answer (wide_leaf_answer).  Where that leaf does not decide (one
+// of 10,000 of them), and for rays the wide tree cannot serve (wide_usable),
+// the ray goes into a list of the warp in shared memory and is
+// traced through the kd-tree once the list is full or the queue is empty.
+//
+// The claim rests on every triangle being tested that the kd loop could accept
+// (wide_triangle, kWidePad) and leaves out one kind of ray: one
+// within about 1e-4 of the plane of a triangle, where the determinant is of the
+// size of its own rounding, that passes the triangle beside an edge.  The test may
+// then report a hit far beyond the edge; the kd loop takes it where the ray's
+// cells hold the triangle, this loop where the ray meets its box.  Of rays made
+// to be so (grazing to 1e-6, within a tenth of an edge) one in a million differs
+// among loose triangles, none in 16 million in the closed scenes.
 //
 // Why: the kd loop runs at 8 of 32 lanes per instruction and 351 warp
 // instructions per ray, 43 dependent node loads and 16 triangle tests a ray;
@@ -311,33 +269,6 @@ XYZ_DEV void trace_persistent(const DevScene &S, int n, int *fetch, Sink &sink, 
 // 32-byte loads, and a ray needs about ten of them.
 constexpr int kWideRetry = 128;  // list entries per warp; 64 + one refill + the lanes under way fit
 constexpr int kWideRetryFull = 64;
-
-// Error bounds of an accepted hit: `dt` in its distance, `m` in its
-// barycentric coordinates.  The test rounds differences of the ray's and the
-// triangle's coordinates, at most t + |e| long (for |d| <= 2), and 1 / det
-// scales what is left: 16 roundings of that length over the triangle's
-// height (e / det) and the angle between the ray and its plane (n / det).
-XYZ_DEV void wide_margin(float t, float e, float n, float inv_det, float *m, float *dt) {
-  float const r = (fabsf(t) + e) * fabsf(inv_det) * (1.0f / 1048576.0f);
-  *m = r * e;
-  *dt = r * n;
-}
-
-// Whether the point at distance t lies in one kd leaf together with every hit
-// within `slack` of it: the descent to its leaf meets no split plane closer
-// than twice the error of the hits (along the ray and across it, for |d| <= 2)
-// plus the rounding of the point itself.
-XYZ_DEV bool wide_settled(const uint2 *__restrict__ nodes, f3 o, f3 d, float t, float slack) {
-  f3 const p = add3(o, scl3(d, t));
-  float const eps = 4.0f * slack + (norm1(o) + norm1(p)) * (1.0f / 2097152.0f);
-  uint2 nd = __ldg(&nodes[0]);
-  while ((nd.y & 3u) != kKdLeafTag) {
-    float const off = comp3(p, static_cast<int>(nd.y & 3u)) - __uint_as_float(nd.x);
-    if (!(fabsf(off) > eps)) return false;
-    nd = __ldg(&nodes[(nd.y >> 2) + (off > 0.0f ? 1u : 0u)]);
-  }
-  return true;
-}
 
 template <class Sink>
 struct RetrySink {
@@ -382,7 +313,8 @@ constexpr int kRaysPerCta = 32;
 // taken together, once enough lanes are not under way, so that neither runs
 // for a lane or two at a time.
 template <bool kBatch = false, class Sink>
-XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_t *list, int *list_fetch, int warps) {
+XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_t *list, float *list_t, int *list_fetch,
+                        int warps) {
   constexpr bool kTarget = SinkHasTarget<Sink>::value;
   int const lane = threadIdx.x & 31;
   unsigned const lanes_below = (1u << lane) - 1u;
@@ -401,7 +333,7 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
     WideRay R{};
     float tmin = 0.0f, tlim = 0.0f;
     RayHit h{};
-    float slack = 0.0f;  // > 0: rounding could decide the answer (wide_settled)
+    float slack = 0.0f;  // > 0: rounding could decide the answer (wide_take)
     uint32_t base = 0, group = 0;             // node group: first child, hits (visiting order) << 8 | inner slots
     uint32_t tri_base = 0, tri_valid = 0, tri_hits = 0;
     int sp = 0;
@@ -410,12 +342,14 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
       unsigned under_way = __ballot_sync(0xffffffffu, live);
       if (__popc(under_way) <= refill_at) {
         int retry = -1;
+        float retry_t = __int_as_float(0x7fffffff);  // a hit's distance, or no number
         if (ray >= 0 && !live) {
-          const uint2 *const kd = kBatch ? lane_scene->nodes : S.nodes;
-          if (h.id >= 0 && slack > 0.0f && !wide_settled(kd, R.o, d, h.t, slack))
+          if (h.id >= 0 && slack > 0.0f) {
             retry = ray;
-          else
+            retry_t = h.t;
+          } else {
             sink.store(ray, h);
+          }
           ray = -1;
         }
         // a full list is traced before more rays are taken
@@ -465,7 +399,8 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
                     live = test_triangle(a, b, c, o, d, tmin, tmax, &t, &f, &g, &back, &inv_det);
                     if (live) {
                       float m, dt;
-                      wide_margin(t, norm1(xyz3(b)) + norm1(xyz3(c)), norm1(mk3(a.w, b.w, c.w)), inv_det, &m, &dt);
+                      float const l1 = norm1(xyz3(b)), l2 = norm1(xyz3(c));
+                      wide_margin(t, norm1(d), l1 + l2, norm1(mk3(a.w, b.w, c.w)) + l1 * l2, inv_det, &m, &dt);
                       if (f < m || g < m || 1.0f - (f + g) < m || t < tmin + dt || tmax < t + dt) slack = dt;
                       h.t = t;
                       h.f = f;
@@ -481,11 +416,15 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
           }
         }
         unsigned const again = __ballot_sync(0xffffffffu, retry >= 0);
-        if (retry >= 0) list[n_list + __popc(again & lanes_below)] = retry;
+        if (retry >= 0) {
+          int const at = n_list + __popc(again & lanes_below);
+          list[at] = retry;
+          list_t[at] = retry_t;
+        }
         n_list += __popc(again);
         // a whole warp of rays that the tree cannot serve: the rest of the queue
         // is taken to be like them
-        if (again == 0xffffffffu) {
+        if (__all_sync(0xffffffffu, retry >= 0 && !(retry_t == retry_t))) {
           kd_only = true;
           break;
         }
@@ -543,26 +482,14 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
           if (test_triangle(vec(0), vec(1), vec(2), R.o, d, tmin, tlim, &t, &f, &g, &back, &inv_det)) {
             int32_t const id = static_cast<int32_t>(w[12]);
             float m, dt;
-            wide_margin(t, __uint_as_float(w[13]), __uint_as_float(w[14]), inv_det, &m, &dt);
-            bool const edge = f < m || g < m || 1.0f - (f + g) < m || t < tmin + dt;
-            if (kTarget && id != h.id && !edge && t + dt < h.t && sink_targeted(sink, ray)) {
+            wide_margin(t, norm1(d), __uint_as_float(w[13]), __uint_as_float(w[14]), inv_det, &m, &dt);
+            if (kTarget && id != h.id && t + dt < h.t && f >= m && g >= m && 1.0f - (f + g) >= m && t >= tmin + dt &&
+                sink_targeted(sink, ray)) {
               // certainly before the target: the ray is answered
               h.id = -1;
               live = false;
             } else if (id != h.id) {
-              // the largest error among the hits that are too close to tell apart
-              float const both = fmaxf(fmaxf(slack, tlim - h.t), dt);
-              if (t < h.t || (t == h.t && id > h.id)) {
-                slack = h.t <= t + dt ? both : (edge ? dt : 0.0f);
-                h.t = t;
-                h.f = f;
-                h.g = g;
-                h.id = id;
-                h.back = back;
-                tlim = t + dt;
-              } else {
-                slack = both;
-              }
+              wide_take(t, f, g, id, back, m, dt, tmin, h, tlim, slack);
             }
           }
         }
@@ -578,12 +505,34 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
         }
       }
     }
-    if (n_list > 0) {
+    __syncwarp();
+    int n_kd = 0;
+    for (int j0 = 0; j0 < n_list; j0 += 32) {
+      int i = j0 + lane < n_list ? list[j0 + lane] : -1;
+      if (i >= 0) {
+        RayHit a{list_t[j0 + lane], 0.0f, 0.0f, -1, 0};
+        if (a.t == a.t) {
+          f3 o, dir;
+          float t0, t1;
+          sink.load(i, o, dir, t0, t1);
+          const DevScene *SL = &S;
+          if constexpr (kBatch) SL = sink.scene(i);
+          if (wide_leaf_answer(*SL, o, dir, t0, a)) {
+            sink.store(i, a);
+            i = -1;
+          }
+        }
+      }
+      unsigned const kept = __ballot_sync(0xffffffffu, i >= 0);
+      if (i >= 0) list[n_kd + __popc(kept & lanes_below)] = i;
+      n_kd += __popc(kept);
+    }
+    if (n_kd > 0) {
       if (lane == 0) *list_fetch = 0;
       __syncwarp();
       RetrySink<Sink> again{&sink, list};
       TraceCount tc{};
-      trace_persistent<false, kBatch>(S, n_list, list_fetch, again, tc);
+      trace_persistent<false, kBatch>(S, n_kd, list_fetch, again, tc);
       __syncwarp();
     }
     if (kd_only) {
@@ -599,6 +548,7 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
 constexpr int kTraceWarps = 4;
 struct WideList {
   int32_t entry[kTraceWarps][kWideRetry];
+  float t[kTraceWarps][kWideRetry];
   int fetch[kTraceWarps];
 };
 
@@ -612,7 +562,7 @@ XYZ_DEV void trace_closest_hits(const DevScene &S, int n, int *fetch, Sink &sink
                                 int warps = grid_warps()) {
   if (kBatch || S.wide) {
     int const w = threadIdx.x >> 5;
-    trace_wide<kBatch>(S, n, fetch, sink, L.entry[w], &L.fetch[w], warps);
+    trace_wide<kBatch>(S, n, fetch, sink, L.entry[w], L.t[w], &L.fetch[w], warps);
   } else {
     TraceCount tc{};
     trace_persistent<false, kBatch>(S, n, fetch, sink, tc);

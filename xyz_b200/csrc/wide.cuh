@@ -17,7 +17,7 @@
 //   12..17 box minima, 8 bytes per axis (byte s = slot s); 18..23 box maxima
 // Inner children lie consecutively in slot order, triangle records in bit order.
 // Triangle record: 64 bytes, (v0, n.x) (e1, n.y) (e2, n.z) as in DevScene::tri,
-// then the triangle id, |e1| + |e2| and |n| (1-norms, for the error margins).
+// then the triangle id and two lengths for the error margins (WideTri).
 //
 // A 1M-triangle mesh: 11 MB of nodes and 63 MB of records, where the kd-tree
 // keeps 38 MB of nodes, 35 MB of references and 47 MB of triangles.
@@ -137,6 +137,48 @@ struct WideBox {
 XYZ_HD WideBox wide_box(const WideSets &T, int32_t node) {
   uint4 const l = T.lo[node], h = T.hi[node];
   return WideBox{{key_float(l.x), key_float(l.y), key_float(l.z)}, {key_float(h.x), key_float(h.y), key_float(h.z)}};
+}
+
+// A triangle's box and the lengths its error margins need (wide_margin).
+//
+// The box holds every point that the triangle test may report, so that the walk
+// tests each triangle the kd loop could accept.  The test divides by
+// det = d.n, and n carries the rounding of its products (2.8 u |e1||e2|, u =
+// 2^-24) as do the sums (3 u each): an accepted ray passes the triangle in its
+// plane within 12 u e |e1||e2| |d| / |det| (e the longer edge), the part that
+// grows with the ray's length left to kWidePad.  For a well-shaped triangle
+// that is a millionth of its size, for a sliver of width q e it is 12 u e / q:
+// beyond its far edge rays are accepted that miss it by many times its width.
+// |det| is at least kEpsilon (of a ray of |d| <= 2 here), and slopes below 1/16
+// are left out: a box grown for every slope would have no bound.
+// 200 slivers 1e-4 / 1e-5 as wide as long, 2 M rays aimed beside their edges: the
+// box of the corners alone misses 1 / 47 hits that the kd loop reports, this one
+// none of 16 M; triangle tests a ray 9.7 -> 12.6 / 10.2 -> 46.3.
+struct WideTri {
+  float lo[3], hi[3];
+  float e, n;  // |e1| + |e2| and |n| + |e1||e2| (1-norms)
+};
+
+constexpr float kWideGrow = 12.0f / 16777216.0f;
+
+XYZ_HD WideTri wide_triangle(f3 v0, f3 e1, f3 e2, f3 n) {
+  WideTri w;
+  float const a = norm1(e1), b = norm1(e2), l1 = sqrtf(dot3(e1, e1)), l2 = sqrtf(dot3(e2, e2));
+  float const top = fmaxf(fmaxf(fabsf(n.x), fabsf(n.y)), fabsf(n.z));
+  f3 const u = top > 0.0f ? scl3(n, 1.0f / top) : n;
+  float const uu = dot3(u, u), ln = top * sqrtf(uu);
+  w.e = a + b;
+  w.n = norm1(n) + a * b;
+  float const grow = kWideGrow * fmaxf(l1, l2) * (l1 * l2) / fmaxf(0.5f * kEpsilon, 0.0625f * ln);
+  for (int k = 0; k < 3; ++k) {
+    float const x = comp3(v0, k), p = comp3(e1, k), q = comp3(e2, k), c = comp3(u, k);
+    // in the triangle's plane: an axis along the normal needs none
+    float const along = sqrtf(fmaxf(0.0f, 1.0f - c * c / uu)) + 4.0f / 16777216.0f * (l1 * l2) / ln;
+    float const g = top > 0.0f ? grow * fminf(1.0f, along) : 0.0f;
+    w.lo[k] = fminf(x, fminf(x + p, x + q)) - g;
+    w.hi[k] = fmaxf(x, fmaxf(x + p, x + q)) + g;
+  }
+  return w;
 }
 
 // The smallest power of two s >= 2^-100 with 252 s >= extent (the grid starts
@@ -420,6 +462,134 @@ XYZ_HD uint32_t wide_spread(uint32_t h) {
   h = (h | (h << 4)) & 0x0c30c3u;
   h = (h | (h << 2)) & 0x249249u;
   return h * 7u;
+}
+
+// ---------------------------------------------------------------- hits
+struct RayHit {
+  float t, f, g;
+  int32_t id;    // -1 = miss
+  int32_t back;  // 1 = hit from the back side (det > 0)
+};
+
+#ifdef __CUDA_ARCH__
+#define XYZ_LDG(x) __ldg(&(x))
+#else
+#define XYZ_LDG(x) (x)
+#endif
+
+XYZ_HD float reciprocal(float x) {
+#ifdef __CUDA_ARCH__
+  return __frcp_rn(x);
+#else
+  return 1.0f / x;
+#endif
+}
+
+// FindIntersectionDF (xyz/geom/triangle.cpp:127-165) on a packed triangle
+// (a, b, c): the hit within [tmin, tmax], its side and 1 / det.
+XYZ_HD bool test_triangle(float4 a, float4 b, float4 c, f3 o, f3 d, float tmin, float tmax, float *t_out,
+                          float *f_out, float *g_out, int32_t *back_out, float *inv_out) {
+  f3 const e2xe1 = mk3(a.w, b.w, c.w);
+  float const det = dot3(d, e2xe1);
+  if (fabsf(det) < kEpsilon) return false;
+  float const inv_det = reciprocal(det);
+  f3 const vmo = sub3(xyz3(a), o);
+  float const t = inv_det * dot3(vmo, e2xe1);
+  if ((t < tmin) || (tmax < t)) return false;
+  f3 const dxvmo = cross3(d, vmo);
+  float const f = inv_det * dot3(xyz3(c), dxvmo);
+  if ((f < 0.0f) || (f > 1.0f)) return false;
+  float const g = inv_det * -dot3(xyz3(b), dxvmo);
+  if ((g < 0.0f) || ((f + g) > 1.0f)) return false;
+  *t_out = t;
+  *f_out = f;
+  *g_out = g;
+  *back_out = det > 0.0f;
+  *inv_out = inv_det;
+  return true;
+}
+
+// The test on triangle i of the scene; updates best_t on acceptance.
+XYZ_HD bool hit_triangle(const float4 *__restrict__ tri, int32_t i, f3 o, f3 d, float tmin, RayHit &h) {
+  float t, f, g, inv_det;
+  int32_t back;
+  if (!test_triangle(XYZ_LDG(tri[3 * i + 0]), XYZ_LDG(tri[3 * i + 1]), XYZ_LDG(tri[3 * i + 2]), o, d, tmin, h.t, &t,
+                     &f, &g, &back, &inv_det))
+    return false;
+  h = RayHit{t, f, g, i, back};
+  return true;
+}
+
+// Error bounds of an accepted hit of a ray with |d| = s (1-norm): `dt` in its
+// distance, `m` in its barycentric coordinates.  The sums over the differences of
+// the ray's and the triangle's coordinates, at most t s + |e| long, round by 3 u
+// of their terms (u = 2^-24), the normal by 2.8 u |e1||e2|: 7 u |n| + 5.7 u |e1||e2|
+// and 5.7 u t s |e| + 18 u |e1||e2| over det, both below the 8 u of w.n and w.e.
+XYZ_HD void wide_margin(float t, float s, float e, float n, float inv_det, float *m, float *dt) {
+  float const r = (fabsf(t) * s + e) * fabsf(inv_det) * (1.0f / 2097152.0f);
+  *m = r * e * s;
+  *dt = r * n;
+}
+
+// Takes a hit of triangle id into the ray's answer h: the nearest, and of equal
+// distances the highest id.  The walk goes on to tlim, the answer's distance and
+// its error; slack is positive where rounding could decide the kd loop's answer:
+// the hit closer to an edge (or to tmin), or a second hit closer in distance,
+// than its error.
+XYZ_HD void wide_take(float t, float f, float g, int32_t id, int32_t back, float m, float dt, float tmin, RayHit &h,
+                      float &tlim, float &slack) {
+  bool const edge = f < m || g < m || 1.0f - (f + g) < m || t < tmin + dt;
+  float const both = fmaxf(fmaxf(slack, tlim - h.t), dt);
+  if (t < h.t || (t == h.t && id > h.id)) {
+    slack = h.t <= t + dt ? both : (edge ? dt : 0.0f);
+    h = RayHit{t, f, g, id, back};
+    tlim = t + dt;
+  } else {
+    slack = both;
+  }
+}
+
+// The kd loop's answer where h is the nearest hit of all triangles, if one leaf
+// decides it.  The loop stops at the latest in the leaf whose interval of
+// distances, as it computes them, holds h.t: if that leaf refers to h's
+// triangle, or to others hit at the same distance, the last of them is the
+// answer (a leaf's triangles are tested in order, and equal distances replace).
+// False where it refers to none: the answer then depends on the leaves before.
+XYZ_HD bool wide_leaf_answer(const DevScene &S, f3 o, f3 d, float tmin, RayHit &h) {
+  f3 const inv = mk3(reciprocal(d.x), reciprocal(d.y), reciprocal(d.z));
+  float tn = tmin, tf = INFINITY;
+  for (int k = 0; k < 3; ++k) {
+    float const ta = (comp3(S.bmin, k) - comp3(o, k)) * comp3(inv, k);
+    float const tb = (comp3(S.bmax, k) - comp3(o, k)) * comp3(inv, k);
+    tn = fmaxf(tn, fminf(ta, tb));
+    tf = fminf(tf, fmaxf(ta, tb));
+  }
+  if (!(tn <= tf && tn <= h.t)) return false;
+  uint2 nd = XYZ_LDG(S.nodes[0]);
+  while ((nd.y & 3u) != kKdLeafTag) {
+    int const ax = static_cast<int>(nd.y & 3u);
+    float const split = wide_float(nd.x), oa = comp3(o, ax);
+    float const tp = (split - oa) * comp3(inv, ax);
+    uint32_t const first = (oa < split || (oa == split && comp3(d, ax) <= 0.0f)) ? 0u : 1u;
+    bool in_first = true;
+    if (!(tp > tf || tp <= 0.0f)) {
+      if (tp < tn) {
+        in_first = false;
+      } else if (h.t <= tp) {
+        tf = tp;
+      } else {
+        in_first = false;
+        tn = tp;
+      }
+    }
+    nd = XYZ_LDG(S.nodes[(nd.y >> 2) + (in_first ? first : first ^ 1u)]);
+  }
+  RayHit a = h;
+  a.id = -1;
+  for (uint32_t j = 0; j < (nd.y >> 2); ++j) hit_triangle(S.tri, XYZ_LDG(S.refs[nd.x + j]), o, d, tmin, a);
+  if (a.id < 0 || a.t < h.t) return false;
+  h = a;
+  return true;
 }
 
 }  // namespace xyzgpu
