@@ -91,7 +91,7 @@ bool build(const std::vector<f3> &V, Trees &B) {
   for (uint32_t b = 0; b < made; ++b) {
     if (made > max_nodes) return false;
     wide_make_node(
-        nd.data(), W, task[b], reach * kWidePad, &B.wide[static_cast<size_t>(b) * kWideWords],
+        nd.data(), W, task[b], 0.0f, &B.wide[static_cast<size_t>(b) * kWideWords],
         [&](int k) { return (made += k) - k; }, [&](int k) { return (recs += k) - k; },
         [&](uint32_t at, WideTask t) { task[at] = t; }, [&](int32_t at, uint32_t r) { dst[at] = static_cast<int>(r); });
   }

@@ -91,3 +91,48 @@ def compare(sd, rays, **build):
 def test_sliver_hits_equal_the_kd_tree(width, builder):
     pos = slivers(width).astype(np.float32)
     assert compare(scene_of(pos), edge_rays(pos, 1 << 20, 3), builder=builder) > 1 << 17
+
+
+# ---- coordinates that are large beside the triangles
+@pytest.mark.parametrize("scene", ["terrain:0", "terrain:1000", "terrain:10000", "ground:10", "ground:1000", "ground:3000"])
+def test_work_does_not_depend_on_the_coordinates(check, scene):
+    """Wherever the triangles lie a ray meets fewer than half the nodes that it
+    meets in the kd-tree, and not many more triangles (at 10,000 the corners are
+    rounded to a tenth of a triangle, which the kd-tree's splits suffer from too)."""
+    differ, nodes, tests, kd_nodes, kd_tests = check(scene, 30000, "local")[3:]
+    assert differ == 0
+    assert nodes < 0.5 * kd_nodes
+    assert tests < 1.5 * kd_tests
+
+
+@pytest.mark.parametrize("scene", ["terrain:0", "terrain:10000", "ground:300", "ground:3000"])
+def test_answers_at_large_coordinates(check, scene):
+    rays, hits, unsettled, differ = check(scene, 100000, "edge")[:4]
+    assert hits > rays / 2 and unsettled < rays / 100
+    assert differ == 0
+
+
+def terrain(n, at):
+    x = np.linspace(-1, 1, n + 1)
+    X, Z = np.meshgrid(x, x, indexing="ij")
+    Y = 0.1 * np.sin(7 * X) * np.cos(5 * Z) + 0.004 * np.random.default_rng(5).normal(size=X.shape)
+    P = np.stack([X + at, Y, Z + at], -1)
+    a, b, c, d = P[:-1, :-1], P[1:, :-1], P[1:, 1:], P[:-1, 1:]
+    return np.concatenate([np.stack(t, 2).reshape(-1, 3, 3) for t in ((a, b, c), (a, c, d))])
+
+
+def ground(h):
+    q = [(-h, -1, -h), (h, -1, -h), (h, -1, h), (-h, -1, h)]
+    return np.concatenate([terrain(100, 0.0), np.array([[q[0], q[1], q[2]], [q[0], q[2], q[3]]], np.float64)])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("pos", [terrain(100, 1000.0), terrain(100, 10000.0), ground(300.0), ground(3000.0)],
+                         ids=["terrain1000", "terrain10000", "ground300", "ground3000"])
+def test_hits_equal_the_kd_tree_at_large_coordinates(pos):
+    pos = pos.astype(np.float32)
+    rays = edge_rays(pos, 1 << 19, 4)
+    m = rays.shape[0] // 2  # the other half from nearby
+    near = rays[m:, 0:3] + rays[m:, 4:7] * (0.9 * np.linalg.norm(rays[m:, 0:3] - pos.reshape(-1, 3).mean(0), axis=1))[:, None]
+    rays[m:, 0:3] = near
+    assert compare(scene_of(pos), rays) > 1 << 16

@@ -1022,13 +1022,13 @@ struct WideCounters {
 constexpr int kWideThreads = 64;
 
 __global__ void __launch_bounds__(kWideThreads)
-    k_wide_nodes(const uint2 *__restrict__ kd, WideSets T, float pad, int l, WideCounters *C, WideTask *task,
+    k_wide_nodes(const uint2 *__restrict__ kd, WideSets T, int l, WideCounters *C, WideTask *task,
                  uint32_t max_nodes, uint32_t *__restrict__ out, int32_t *__restrict__ dst) {
   uint32_t const b = C->level[l], e = C->level[l + 1];
   for (uint32_t i = b + blockIdx.x * blockDim.x + threadIdx.x; i < e; i += gridDim.x * blockDim.x) {
     uint32_t w[kWideWords];
     wide_make_node(
-        kd, T, task[i], pad, w, [&](int k) { return atomicAdd(&C->nodes, static_cast<uint32_t>(k)); },
+        kd, T, task[i], 0.0f, w, [&](int k) { return atomicAdd(&C->nodes, static_cast<uint32_t>(k)); },
         [&](int k) { return atomicAdd(&C->tris, static_cast<uint32_t>(k)); },
         [&](uint32_t at, WideTask t) {
           if (at < max_nodes) task[at] = t;
@@ -1246,7 +1246,7 @@ struct WideBufs {
 
 // Fills the wide tree from the sets of the breadth-first kd nodes.  A tree
 // deeper than the traversal's stack is dropped (the kd-tree serves alone).
-int wide_build(SceneImpl &s, WideBufs &B, const WideSets &T, float pad, cudaStream_t st) {
+int wide_build(SceneImpl &s, WideBufs &B, const WideSets &T, cudaStream_t st) {
   int const dev = s.device, n = s.n_tris;
   uint32_t const max_nodes = static_cast<uint32_t>(wide_max_nodes(n));
   WideCounters h{};
@@ -1263,7 +1263,7 @@ int wide_build(SceneImpl &s, WideBufs &B, const WideSets &T, float pad, cudaStre
   for (int group = n > 4096 ? 10 : 4; more && done < kWideStack; group = 4) {
     int const upto = std::min(kWideStack, done + group);
     for (; done < upto; ++done)
-      k_wide_nodes<<<grid, kWideThreads, 0, st>>>(s.d_nodes, T, pad, done, B.counters.p, B.task.p, max_nodes,
+      k_wide_nodes<<<grid, kWideThreads, 0, st>>>(s.d_nodes, T, done, B.counters.p, B.task.p, max_nodes,
                                                   B.nodes.p, B.dst.p);
     XYZ_BUILD_TRY(cudaGetLastError());
     XYZ_BUILD_TRY(cudaMemcpyAsync(&h, B.counters.p, sizeof(h), cudaMemcpyDeviceToHost, st));
@@ -1338,7 +1338,7 @@ int kd_layout_depth_first(SceneImpl &s, const std::vector<int64_t> &level_start,
   k_layout_scatter<<<grid_for(n, 256, dev), 256, 0, st>>>(s.d_nodes, n, pos.p, base.p, out.p);
   XYZ_BUILD_TRY(cudaGetLastError());
   if (wide) {
-    int const rc = wide_build(s, B, T, reach * kWidePad, st);
+    int const rc = wide_build(s, B, T, st);
     if (rc) return rc;
     s.dev.wide_reach = reach * kWideReach;
   }

@@ -248,14 +248,15 @@ XYZ_DEV void trace_persistent(const DevScene &S, int n, int *fetch, Sink &sink, 
 // edge of its triangle that rounding decides whether the ray's kd cells hold
 // it, or two hits whose distances differ by less than their rounding.  Such
 // rays are recognised while they are traced (wide_take: 0.1 to 1 % of them on a
-// 1M-triangle mesh), and the leaf of the kd-tree in which the kd loop would stop says
+// 1M-triangle mesh, nearly all where rays are 10,000 times as long as the
+// triangles), and the leaf of the kd-tree in which the kd loop would stop says
 // what it would answer (wide_leaf_answer).  Where that leaf does not decide (one
 // of 10,000 of them), and for rays the wide tree cannot serve (wide_usable),
 // the ray goes into a list of the warp in shared memory and is
 // traced through the kd-tree once the list is full or the queue is empty.
 //
 // The claim rests on every triangle being tested that the kd loop could accept
-// (wide_triangle, kWidePad) and leaves out one kind of ray: one
+// (wide_triangle and the slack of wide_test) and leaves out one kind of ray: one
 // within about 1e-4 of the plane of a triangle, where the determinant is of the
 // size of its own rounding, that passes the triangle beside an edge.  The test may
 // then report a hit far beyond the edge; the kd loop takes it where the ray's

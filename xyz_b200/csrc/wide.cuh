@@ -37,12 +37,22 @@ constexpr int kWideWords = 24;       // 32-bit words of a node
 constexpr int kWideLeafTris = 3;     // triangles of a leaf child
 constexpr int kWideStack = 64;       // node groups a ray may hold: the tree is no deeper
 constexpr int kWideTriVec = 4;       // float4 per triangle record
-// Boxes grow by this share of the largest scene coordinate S on every side,
-// and rays whose origin has a coordinate beyond kWideReach * S do not use the
-// tree: the grid arithmetic errs by at most 2^-22 of the largest |box - origin|
-// (9 S * 2^-22 = 2.1e-6 S), the padding is 3.8e-6 S.
-constexpr float kWidePad = 1.0f / 262144.0f;
-constexpr float kWideReach = 8.0f;
+// While a ray is tested the boxes grow by kWideSlack of their distance from its
+// origin (wide_test), which is small beside the triangles wherever the scene lies
+// and however far it reaches.  An allowance for the longest possible ray, as a
+// share of the largest coordinate S, is not (boxes grown by 2^-18 S / this, us for
+// 2^21 rays between two points):
+// an 80,000-triangle terrain 2 wide at coordinates of 0 / 1,000 / 10,000
+// 1,203 / 1,938 / 17,649 and 1,215 / 1,238 / 1,368; a 1M-triangle object 6 wide in a
+// ground of half width 300 / 1,000 / 3,000 2,390 / 3,516 / 8,022 and 1,391 / 1,445 /
+// 1,454 (the kd loop 2,550 to 2,490).  Where it buys nothing it costs 2 %.  Rays
+// from all over such a ground at the object's triangles, 10^4 to 10^5 times as long
+// as these, are close calls to the last one: 5,455 / 7,388 / 13,718 and 2,101 /
+// 2,965 / 5,588 (the kd loop 2,470 to 2,540, which is faster from 1,000 on).
+// Rays whose origin has a coordinate beyond kWideReach * S do not use the tree.
+constexpr float kWideSlack = 1.0f / 524288.0f;
+constexpr float kWidePad = 1.0f / 8388608.0f;  // of S: for boxes whose corners are rounded to nearest
+constexpr float kWideReach = 65536.0f;
 
 // Triangle sets of the kd-tree's (breadth-first) nodes while the tree is built.
 struct WideSets {
@@ -76,6 +86,16 @@ XYZ_HD float key_float(uint32_t k) {
   return f;
 #endif
 }
+// The sum, rounded down and up.
+XYZ_HD float add_down(float a, float b) {
+#ifdef __CUDA_ARCH__
+  return __fadd_rd(a, b);
+#else
+  float const r = a + b;
+  return static_cast<long double>(r) > static_cast<long double>(a) + b ? std::nextafter(r, -INFINITY) : r;
+#endif
+}
+XYZ_HD float add_up(float a, float b) { return -add_down(-a, -b); }
 XYZ_HD uint32_t wide_bits(float f) {
 #ifdef __CUDA_ARCH__
   return __float_as_uint(f);
@@ -146,7 +166,7 @@ XYZ_HD WideBox wide_box(const WideSets &T, int32_t node) {
 // det = d.n, and n carries the rounding of its products (2.8 u |e1||e2|, u =
 // 2^-24) as do the sums (3 u each): an accepted ray passes the triangle in its
 // plane within 12 u e |e1||e2| |d| / |det| (e the longer edge), the part that
-// grows with the ray's length left to kWidePad.  For a well-shaped triangle
+// grows with the ray's length left to wide_test.  For a well-shaped triangle
 // that is a millionth of its size, for a sliver of width q e it is 12 u e / q:
 // beyond its far edge rays are accepted that miss it by many times its width.
 // |det| is at least kEpsilon (of a ray of |d| <= 2 here), and slopes below 1/16
@@ -175,14 +195,14 @@ XYZ_HD WideTri wide_triangle(f3 v0, f3 e1, f3 e2, f3 n) {
     // in the triangle's plane: an axis along the normal needs none
     float const along = sqrtf(fmaxf(0.0f, 1.0f - c * c / uu)) + 4.0f / 16777216.0f * (l1 * l2) / ln;
     float const g = top > 0.0f ? grow * fminf(1.0f, along) : 0.0f;
-    w.lo[k] = fminf(x, fminf(x + p, x + q)) - g;
-    w.hi[k] = fmaxf(x, fmaxf(x + p, x + q)) + g;
+    w.lo[k] = add_down(fminf(x, fminf(add_down(x, p), add_down(x, q))), -g);
+    w.hi[k] = add_up(fmaxf(x, fmaxf(add_up(x, p), add_up(x, q))), g);
   }
   return w;
 }
 
 // The smallest power of two s >= 2^-100 with 252 s >= extent (the grid starts
-// 1/64 step before the boxes and each bound may round one step outwards).
+// 1/32 step before the boxes and each bound may round one step outwards).
 XYZ_HD float wide_step(float extent) {
   float const r = extent * (1.0f / 252.0f);
   uint32_t e = (wide_bits(r) >> 23) & 0xffu;
@@ -191,10 +211,10 @@ XYZ_HD float wide_step(float extent) {
   return wide_float(e << 23);
 }
 
-// Builds one node of the tree.  alloc_nodes(k) / alloc_tris(k) reserve k
-// consecutive node / record indices; put_task(i, t) names the task of inner
-// node i, put_tri(pos, rec) the record of the triangle at depth-first
-// position pos.
+// Builds one node of the tree from the boxes of T, grown by `pad`.
+// alloc_nodes(k) / alloc_tris(k) reserve k consecutive node / record indices;
+// put_task(i, t) names the task of inner node i, put_tri(pos, rec) the record of
+// the triangle at depth-first position pos.
 template <class AllocNodes, class AllocTris, class PutTask, class PutTri>
 XYZ_HD void wide_make_node(const uint2 *nodes, const WideSets &T, WideTask root, float pad, uint32_t *w,
                            AllocNodes alloc_nodes, AllocTris alloc_tris, PutTask put_task, PutTri put_tri) {
@@ -265,8 +285,9 @@ XYZ_HD void wide_make_node(const uint2 *nodes, const WideSets &T, WideTask root,
   for (int k = 0; k < kWideWords; ++k) w[k] = 0u;
   float step[3], org[3];
   for (int k = 0; k < 3; ++k) {
-    step[k] = wide_step(all.hi[k] - all.lo[k]);
-    org[k] = all.lo[k] - step[k] * (1.0f / 64.0f);
+    // (2^-22 of the coordinate: the rounding of the origin)
+    step[k] = wide_step(all.hi[k] - all.lo[k] + fmaxf(fabsf(all.lo[k]), fabsf(all.hi[k])) * (1.0f / 4194304.0f));
+    org[k] = add_down(all.lo[k], step[k] * (-1.0f / 32.0f));
     w[k] = wide_bits(org[k]);
     w[4 + k] = wide_bits(step[k]);
   }
@@ -300,10 +321,10 @@ XYZ_HD void wide_make_node(const uint2 *nodes, const WideSets &T, WideTask root,
       }
     }
     for (int k = 0; k < 3; ++k) {
-      // wide_test places a plane to 1/256 step (its bytes are read as 65536 +
-      // byte): a bound rounds outwards from 1/128 step beyond the box
-      float const ql = floorf((box[i].lo[k] - org[k]) / step[k] - (1.0f / 128.0f));
-      float const qh = ceilf((box[i].hi[k] - org[k]) / step[k] + (1.0f / 128.0f));
+      // wide_test places a plane to 1/128 step (its bytes are read as 65536 +
+      // byte): a bound rounds outwards from 1/64 step beyond the box
+      float const ql = floorf((box[i].lo[k] - org[k]) / step[k] - (1.0f / 64.0f));
+      float const qh = ceilf((box[i].hi[k] - org[k]) / step[k] + (1.0f / 64.0f));
       uint32_t const bl = static_cast<uint32_t>(fminf(fmaxf(ql, 0.0f), 255.0f));
       uint32_t const bh = static_cast<uint32_t>(fminf(fmaxf(qh, 0.0f), 255.0f));
       w[12 + 2 * k + (s >> 2)] |= bl << (8 * (s & 3));
@@ -381,6 +402,14 @@ XYZ_HD float wide_min3(float a, float b, float c) {
 #endif
 }
 
+XYZ_HD float wide_fma(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
+  return __fmaf_rn(a, b, c);
+#else
+  return std::fma(a, b, c);
+#endif
+}
+
 // Two fused multiply-adds q * a + c of one axis (packed FP32 on the device).
 XYZ_HD void wide_fma2(float q0, float q1, float a, float c, float *t0, float *t1) {
 #ifdef __CUDA_ARCH__
@@ -399,13 +428,13 @@ XYZ_HD void wide_fma2(float q0, float q1, float a, float c, float *t0, float *t1
 // Slots kSlot + J and kSlot + J + 1 of a node (bytes J, J + 1 of the words n, f):
 // 2^slot added to m where the ray's box interval meets [tmin, tlim].
 template <int kSlot, int J>
-XYZ_HD float wide_pair(const uint32_t n[3], const uint32_t f[3], const float a[3], const float c[3], float tmin,
-                       float tlim, float m) {
+XYZ_HD float wide_pair(const uint32_t n[3], const uint32_t f[3], const float a[3], const float cn[3], const float cf[3],
+                       float tmin, float tlim, float m) {
   float tn[3][2], tf[3][2];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    wide_fma2(wide_byte<J>(n[k]), wide_byte<J + 1>(n[k]), a[k], c[k], &tn[k][0], &tn[k][1]);
-    wide_fma2(wide_byte<J>(f[k]), wide_byte<J + 1>(f[k]), a[k], c[k], &tf[k][0], &tf[k][1]);
+    wide_fma2(wide_byte<J>(n[k]), wide_byte<J + 1>(n[k]), a[k], cn[k], &tn[k][0], &tn[k][1]);
+    wide_fma2(wide_byte<J>(f[k]), wide_byte<J + 1>(f[k]), a[k], cf[k], &tf[k][0], &tf[k][1]);
   }
 #pragma unroll
   for (int s = 0; s < 2; ++s) {
@@ -420,19 +449,23 @@ XYZ_HD float wide_pair(const uint32_t n[3], const uint32_t f[3], const float a[3
 // may report a hit (their box is the grid's first cell): neither an inner bit
 // nor a triangle bit of the node belongs to them.
 XYZ_HD uint32_t wide_test(const uint32_t *w, const WideRay &r, float tmin, float tlim) {
-  float a[3], c[3];
+  float a[3], cn[3], cf[3];
   float const inv[3] = {r.inv.x, r.inv.y, r.inv.z}, o[3] = {r.o.x, r.o.y, r.o.z};
   uint32_t near0[3], near1[3], far0[3], far1[3];
+  // The boxes are widened by kWideSlack of their distance (32 u, u = 2^-24): the
+  // plane distances err by 3 u of it, and the triangle test, whose differences and
+  // products are as long as the ray, reports hits up to 4.9 u of it beside an edge,
+  // over the slope of the ray to the triangle (above 0.17 here).
+  float const slack =
+      kWideSlack * fmaxf(fmaxf(fabsf(wide_float(w[0]) - o[0]), fabsf(wide_float(w[1]) - o[1])), fabsf(wide_float(w[2]) - o[2]));
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     a[k] = wide_float(w[4 + k]) * inv[k];
     // (origin - o) * inv - 65536 * a: the bytes are read as 65536 + byte
     float const po = wide_float(w[k]) - o[k];
-#ifdef __CUDA_ARCH__
-    c[k] = __fmaf_rn(-65536.0f, a[k], po * inv[k]);
-#else
-    c[k] = std::fma(-65536.0f, a[k], po * inv[k]);
-#endif
+    float const c = wide_fma(-65536.0f, a[k], po * inv[k]);
+    cn[k] = wide_fma(-slack, fabsf(inv[k]), c);
+    cf[k] = wide_fma(slack, fabsf(inv[k]), c);
     bool const pos = (r.octinv >> k) & 1u;
     near0[k] = pos ? w[12 + 2 * k] : w[18 + 2 * k];
     near1[k] = pos ? w[13 + 2 * k] : w[19 + 2 * k];
@@ -440,10 +473,10 @@ XYZ_HD uint32_t wide_test(const uint32_t *w, const WideRay &r, float tmin, float
     far1[k] = pos ? w[19 + 2 * k] : w[13 + 2 * k];
   }
   float m = 8388608.0f;  // 2^23: the sum's low mantissa bits are the slots
-  m = wide_pair<0, 0>(near0, far0, a, c, tmin, tlim, m);
-  m = wide_pair<0, 2>(near0, far0, a, c, tmin, tlim, m);
-  m = wide_pair<4, 0>(near1, far1, a, c, tmin, tlim, m);
-  m = wide_pair<4, 2>(near1, far1, a, c, tmin, tlim, m);
+  m = wide_pair<0, 0>(near0, far0, a, cn, cf, tmin, tlim, m);
+  m = wide_pair<0, 2>(near0, far0, a, cn, cf, tmin, tlim, m);
+  m = wide_pair<4, 0>(near1, far1, a, cn, cf, tmin, tlim, m);
+  m = wide_pair<4, 2>(near1, far1, a, cn, cf, tmin, tlim, m);
   return wide_bits(m) & 0xffu;
 }
 
