@@ -171,14 +171,12 @@ bool wide_loop(const Trees &B, f3 o, f3 d, float tmin, float tmax, RayHit &h, do
     group = (wide_order(hit & w[8] & 0xffu, R.octinv) << 8) | (w[8] & 0xffu);
     for (uint32_t th = wide_spread(hit) & valid; th; th &= th - 1) {
       int const id = B.record[w[7] + __builtin_popcount(valid & ((1u << __builtin_ctz(th)) - 1u))];
-      float t, f, g, inv_det, m, dt;
-      int32_t back;
+      float t, f, g, det, m, dt;
       *tests += 1;
-      if (!test_triangle(B.tri[3 * id], B.tri[3 * id + 1], B.tri[3 * id + 2], o, d, tmin, tlim, &t, &f, &g, &back,
-                         &inv_det))
+      if (!test_triangle(B.tri[3 * id], B.tri[3 * id + 1], B.tri[3 * id + 2], o, d, tmin, tlim, &t, &f, &g, &det))
         continue;
-      wide_margin(t, norm1(d), B.lengths[id].e, B.lengths[id].n, inv_det, &m, &dt);
-      wide_take(t, f, g, id, back, m, dt, tmin, h, tlim, slack);
+      wide_margin(t, norm1(d), B.lengths[id].e, B.lengths[id].n, reciprocal(det), &m, &dt);
+      wide_take(t, f, g, id, det > 0.0f, m, dt, tmin, h, tlim, slack);
     }
     if (group >> 8) continue;
     if (stack.empty()) break;

@@ -136,3 +136,35 @@ def test_hits_equal_the_kd_tree_at_large_coordinates(pos):
     near = rays[m:, 0:3] + rays[m:, 4:7] * (0.9 * np.linalg.norm(rays[m:, 0:3] - pos.reshape(-1, 3).mean(0), axis=1))[:, None]
     rays[m:, 0:3] = near
     assert compare(scene_of(pos), rays) > 1 << 16
+
+
+# ---- rays whose direction is not of unit length, or has no extent along an axis
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale", [1e-3, 0.03, 3.0, 1e4, None])
+def test_directions_of_any_length(scale):
+    pos = np.concatenate([slivers(1e-2), terrain(40, 0.0)]).astype(np.float32)
+    rays = edge_rays(pos, 1 << 18, 5)
+    s = scale if scale else 10.0 ** np.random.default_rng(1).uniform(-8, 8, (rays.shape[0], 1))
+    rays[:, 4:7] *= s
+    # (the triangle test bounds d . n from below, so short directions hit little)
+    assert compare(scene_of(pos), rays) > (0 if not scale or scale < 0.1 else 1 << 15)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("extra", [-1, 0, 33])
+@pytest.mark.parametrize("share", [1.0, 0.9])
+def test_queues_of_axis_parallel_rays(extra, share):
+    """Queues around the size from which the kd-tree's own kernel follows, all
+    or most of whose rays have no extent along two axes."""
+    import torch
+    n = 2 * 8 * 128 * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    pos = terrain(60, 0.0).astype(np.float32)
+    rng = np.random.default_rng(6)
+    rays = edge_rays(pos, n, 7)
+    flat = rng.random(n) < share
+    d = np.zeros((n, 3), np.float32)
+    d[np.arange(n), rng.integers(0, 3, n)] = rng.choice([-1.0, 1.0], n)
+    p = rays[:, 0:3] + rays[:, 4:7] * np.linalg.norm(rays[:, 0:3], axis=1, keepdims=True)
+    rays[flat, 4:7] = d[flat]
+    rays[flat, 0:3] = (p - d)[flat]
+    assert compare(scene_of(pos), rays) > 1 << 14

@@ -1,10 +1,11 @@
 // Closest-hit entry point (xyzgpu_trace_closest): the batch form of
 // Scene::FindIntersection (xyz/core/scene.hpp:277-295).
 //
-// Persistent warps with per-lane refill (trace_wide in traverse.cuh, counting
-// calls walk the kd-tree with trace_persistent): rays are taken from a global
-// counter as lanes free up, so long and short rays balance across lanes and SMs.  Rays are read as two 16-byte vectors and
-// hits written as one.
+// Persistent warps with per-lane refill (trace_wide in traverse.cuh; counting
+// calls and queues of axis-parallel rays walk the kd-tree with trace_persistent):
+// rays are taken from a global counter as lanes free up, so long and short rays
+// balance across lanes and SMs.  Rays are read as two 16-byte vectors and hits
+// written as one.
 #include <algorithm>
 
 #include "scene.h"
@@ -36,16 +37,38 @@ struct ApiSink {
   }
 };
 
+// Whether 32 rays spread over the queue are all rays that the wide tree cannot
+// serve (a grid of axis-parallel rays): every warp of the grid finds the same.
+XYZ_DEV bool kd_queue(const DevScene &S, const ApiSink &sink, int n) {
+  f3 o, d;
+  float tmin, tmax;
+  sink.load(static_cast<int>(threadIdx.x & 31) * (n / 32), o, d, tmin, tmax);
+  return __all_sync(0xffffffffu, !S.wide || !wide_usable(o, d, S.wide_reach));
+}
+
+// The kd-tree's kernel for such queues: the loop takes 9 CTAs per SM where the
+// wide loop takes 8, in which it is 11 to 15 % slower (2^21 axis-parallel rays of
+// a 1M-triangle mesh / a room / box stacks: 1,708 / 1,281 / 1,110 us in 9,
+// 1,926 / 1,502 / 1,247 in 8).  Launched after the wide kernel where the
+// queue fills the grid twice; it finds the queue empty in 2 us otherwise.
+__global__ void __launch_bounds__(kTraceThreads, 9)
+    k_trace_kd(DevScene S, const float4 *__restrict__ rays, int n, float4 *__restrict__ hits, int *__restrict__ fetch) {
+  TraceCount c{0u, 0u, 0u};
+  ApiSink sink{rays, hits, 0u, 0u};
+  trace_persistent<false>(S, n, fetch, sink, c);
+}
+
 template <bool kCount>
 __global__ void __launch_bounds__(kTraceThreads, kCount ? 9 : 8)
     k_trace_api(DevScene S, const float4 *__restrict__ rays, int n, float4 *__restrict__ hits,
-                int *__restrict__ fetch, unsigned long long *__restrict__ counts) {
+                int *__restrict__ fetch, unsigned long long *__restrict__ counts, int kd_follows) {
   int const lane = threadIdx.x & 31;
   TraceCount c{0u, 0u, 0u};
   ApiSink sink{rays, hits, 0u, 0u};
   if constexpr (kCount) {
     trace_persistent<true>(S, n, fetch, sink, c);
   } else {
+    if (kd_follows && kd_queue(S, sink, n)) return;
     __shared__ WideList s_list;
     trace_closest_hits(S, n, fetch, sink, s_list);
   }
@@ -62,13 +85,11 @@ __global__ void __launch_bounds__(kTraceThreads, kCount ? 9 : 8)
   }
 }
 
-template <bool kCount>
-int grid_for(int device) {
-  static int blocks = 0;
+template <class Kernel>
+int grid_for(Kernel k, int &blocks, int device) {
   if (blocks == 0) {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace_api<kCount>, kTraceThreads,
-                                                      0) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kTraceThreads, 0) != cudaSuccess ||
         per_sm <= 0)
       per_sm = 4;
     blocks = per_sm * sm_count(device);
@@ -88,8 +109,9 @@ int trace_api_launch(SceneImpl &s, const float *rays, int n, float *hits, cudaSt
   float4 *h4 = reinterpret_cast<float4 *>(hits);
   if (counters) {
     XYZ_CUDA_TRY(cudaMemsetAsync(s.d_trace_counts, 0, 8 * sizeof(unsigned long long), st));
-    k_trace_api<true><<<grid_for<true>(s.device), kTraceThreads, 0, st>>>(s.dev, r4, n, h4, s.d_fetch,
-                                                                        s.d_trace_counts);
+    static int counted_grid = 0;
+    k_trace_api<true><<<grid_for(k_trace_api<true>, counted_grid, s.device), kTraceThreads, 0, st>>>(
+        s.dev, r4, n, h4, s.d_fetch, s.d_trace_counts, 0);
     XYZ_CUDA_TRY(cudaGetLastError());
     unsigned long long c[8];
     XYZ_CUDA_TRY(cudaMemcpyAsync(c, s.d_trace_counts, sizeof(c), cudaMemcpyDeviceToHost, st));
@@ -100,9 +122,16 @@ int trace_api_launch(SceneImpl &s, const float *rays, int n, float *hits, cudaSt
     counters->tri_tests = c[3];
     counters->hits = c[4];
   } else {
-    int const grid = std::min(grid_for<false>(s.device), (n + kRaysPerCta - 1) / kRaysPerCta);
-    k_trace_api<false><<<grid, kTraceThreads, 0, st>>>(s.dev, r4, n, h4, s.d_fetch, nullptr);
+    static int wide_grid = 0, kd_grid = 0;
+    int const full = grid_for(k_trace_api<false>, wide_grid, s.device);
+    int const grid = std::min(full, (n + kRaysPerCta - 1) / kRaysPerCta);
+    bool const kd_follows = n / (2 * kTraceThreads) >= full;
+    k_trace_api<false><<<grid, kTraceThreads, 0, st>>>(s.dev, r4, n, h4, s.d_fetch, nullptr, kd_follows);
     XYZ_CUDA_TRY(cudaGetLastError());
+    if (kd_follows) {
+      k_trace_kd<<<grid_for(k_trace_kd, kd_grid, s.device), kTraceThreads, 0, st>>>(s.dev, r4, n, h4, s.d_fetch);
+      XYZ_CUDA_TRY(cudaGetLastError());
+    }
   }
   return XYZGPU_OK;
 }

@@ -395,19 +395,18 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
                     int32_t const own = sink.target(i);
                     float4 const a = __ldg(&SL.tri[3 * own]), b = __ldg(&SL.tri[3 * own + 1]),
                                  c = __ldg(&SL.tri[3 * own + 2]);
-                    float t, f, g, inv_det;
-                    int32_t back;
-                    live = test_triangle(a, b, c, o, d, tmin, tmax, &t, &f, &g, &back, &inv_det);
+                    float t, f, g, det;
+                    live = test_triangle(a, b, c, o, d, tmin, tmax, &t, &f, &g, &det);
                     if (live) {
                       float m, dt;
                       float const l1 = norm1(xyz3(b)), l2 = norm1(xyz3(c));
-                      wide_margin(t, norm1(d), l1 + l2, norm1(mk3(a.w, b.w, c.w)) + l1 * l2, inv_det, &m, &dt);
+                      wide_margin(t, norm1(d), l1 + l2, norm1(mk3(a.w, b.w, c.w)) + l1 * l2, reciprocal(det), &m, &dt);
                       if (f < m || g < m || 1.0f - (f + g) < m || t < tmin + dt || tmax < t + dt) slack = dt;
                       h.t = t;
                       h.f = f;
                       h.g = g;
                       h.id = own;
-                      h.back = back;
+                      h.back = det > 0.0f;
                       tlim = t + dt;
                     }
                   }
@@ -478,19 +477,18 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
             return make_float4(__uint_as_float(w[4 * q]), __uint_as_float(w[4 * q + 1]), __uint_as_float(w[4 * q + 2]),
                                __uint_as_float(w[4 * q + 3]));
           };
-          float t, f, g, inv_det;
-          int32_t back;
-          if (test_triangle(vec(0), vec(1), vec(2), R.o, d, tmin, tlim, &t, &f, &g, &back, &inv_det)) {
+          float t, f, g, det;
+          if (test_triangle(vec(0), vec(1), vec(2), R.o, d, tmin, tlim, &t, &f, &g, &det)) {
             int32_t const id = static_cast<int32_t>(w[12]);
             float m, dt;
-            wide_margin(t, norm1(d), __uint_as_float(w[13]), __uint_as_float(w[14]), inv_det, &m, &dt);
+            wide_margin(t, norm1(d), __uint_as_float(w[13]), __uint_as_float(w[14]), reciprocal(det), &m, &dt);
             if (kTarget && id != h.id && t + dt < h.t && f >= m && g >= m && 1.0f - (f + g) >= m && t >= tmin + dt &&
                 sink_targeted(sink, ray)) {
               // certainly before the target: the ray is answered
               h.id = -1;
               live = false;
             } else if (id != h.id) {
-              wide_take(t, f, g, id, back, m, dt, tmin, h, tlim, slack);
+              wide_take(t, f, g, id, det > 0.0f, m, dt, tmin, h, tlim, slack);
             }
           }
         }

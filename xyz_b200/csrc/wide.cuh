@@ -360,14 +360,13 @@ XYZ_HD WideRay wide_ray(f3 o, f3 d) {
   return r;
 }
 
-// Rays the tree answers: origin within reach of the scene, direction of
-// about unit length (the margins of wide_margin assume |d| <= 2), no component
-// so small that its reciprocal is infinite: such a ray can lie in a split plane
-// of the kd-tree, whose distance is then not a number, and the kd loop's choice
-// of cells is its own.
+// Rays the tree answers: within the range of the box arithmetic, no component so
+// small that its reciprocal is infinite: such a ray can lie in a split plane of
+// the kd-tree, whose distance is then not a number, and the kd loop's choice of
+// cells is its own.
 XYZ_HD bool wide_usable(f3 o, f3 d, float reach) {
   float const dd = dot3(d, d);
-  return fabsf(o.x) <= reach && fabsf(o.y) <= reach && fabsf(o.z) <= reach && dd <= 4.0f && dd >= 1e-4f &&
+  return fabsf(o.x) <= reach && fabsf(o.y) <= reach && fabsf(o.z) <= reach && dd <= 1e12f && dd >= 1e-12f &&
          fminf(fminf(fabsf(d.x), fabsf(d.y)), fabsf(d.z)) >= 1e-37f;
 }
 
@@ -519,9 +518,9 @@ XYZ_HD float reciprocal(float x) {
 }
 
 // FindIntersectionDF (xyz/geom/triangle.cpp:127-165) on a packed triangle
-// (a, b, c): the hit within [tmin, tmax], its side and 1 / det.
+// (a, b, c): the hit within [tmin, tmax] and det (positive: from the back side).
 XYZ_HD bool test_triangle(float4 a, float4 b, float4 c, f3 o, f3 d, float tmin, float tmax, float *t_out,
-                          float *f_out, float *g_out, int32_t *back_out, float *inv_out) {
+                          float *f_out, float *g_out, float *det_out) {
   f3 const e2xe1 = mk3(a.w, b.w, c.w);
   float const det = dot3(d, e2xe1);
   if (fabsf(det) < kEpsilon) return false;
@@ -537,19 +536,17 @@ XYZ_HD bool test_triangle(float4 a, float4 b, float4 c, f3 o, f3 d, float tmin, 
   *t_out = t;
   *f_out = f;
   *g_out = g;
-  *back_out = det > 0.0f;
-  *inv_out = inv_det;
+  *det_out = det;
   return true;
 }
 
 // The test on triangle i of the scene; updates best_t on acceptance.
 XYZ_HD bool hit_triangle(const float4 *__restrict__ tri, int32_t i, f3 o, f3 d, float tmin, RayHit &h) {
-  float t, f, g, inv_det;
-  int32_t back;
+  float t, f, g, det;
   if (!test_triangle(XYZ_LDG(tri[3 * i + 0]), XYZ_LDG(tri[3 * i + 1]), XYZ_LDG(tri[3 * i + 2]), o, d, tmin, h.t, &t,
-                     &f, &g, &back, &inv_det))
+                     &f, &g, &det))
     return false;
-  h = RayHit{t, f, g, i, back};
+  h = RayHit{t, f, g, i, det > 0.0f};
   return true;
 }
 
