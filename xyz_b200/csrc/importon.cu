@@ -299,8 +299,8 @@ XYZ_DEV void imp_cells(const ImpGrid &M, ImpQuery &Q) {
 
 XYZ_DEV float importon_histogram_warp(const ImpGrid &M, const ImpQuery &Q, int lane, ImpScratch &W) {
   f3 const pos = Q.pos, sn = Q.sn, tan = Q.tan, bin = Q.bin;
-  // rows: at most four cells per axis (three, and one more by rounding), so
-  // that lane 4 z + y takes one each
+  // rows: at most four cells per axis (build_grid), so that lane 4 z + y takes
+  // one each
   int b = 0, cnt = 0;
   if ((lane & 3) < Q.ny && (lane >> 2) < Q.nz) {
     int const row = Q.row0 + ((lane >> 2) * M.g1 + (lane & 3)) * M.g0;
@@ -477,11 +477,17 @@ struct DevArray {
 
 // Sorts importons (unsorted device arrays of n) into the map's grid.
 int build_grid(ImportonImpl &m, const float4 *pos, const float4 *dir, int64_t n, cudaStream_t st) {
-  // grid over the scene box, cells of at least the radius, at most 2^24 cells
+  // grid over the scene box, cells of at least the radius, at most 2^24 cells, and
+  // none smaller than eight times the rounding of the largest coordinate: a point's
+  // neighbourhood then spans 2.5 cells of an axis at most (two, a sixteenth for the
+  // rounding of each end and of its distance from the box, an eighth for its
+  // division), so four rows hold it (importon_histogram_warp)
   DevScene const &S = m.scene->dev;
   float const r = m.cfg.radius;
   float const ext[3] = {S.bmax.x - S.bmin.x, S.bmax.y - S.bmin.y, S.bmax.z - S.bmin.z};
-  float cs = r;
+  float const far = std::max({std::fabs(S.bmin.x), std::fabs(S.bmin.y), std::fabs(S.bmin.z), std::fabs(S.bmax.x),
+                              std::fabs(S.bmax.y), std::fabs(S.bmax.z)});
+  float cs = std::max(r, far / 1048576.0f);
   for (;;) {
     int64_t cells = 1;
     for (int k = 0; k < 3; ++k) cells *= static_cast<int64_t>(ext[k] / cs) + 1;
