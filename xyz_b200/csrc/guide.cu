@@ -36,6 +36,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "error_word.h"
 #include "scene.h"
 #include "tc.cuh"
 
@@ -1090,13 +1091,17 @@ double rand_sym(uint64_t &s) {
   return static_cast<double>(z >> 11) * (2.0 / 9007199254740992.0) - 1.0;
 }
 
-int check_err(GuideImpl &g, cudaStream_t st, const char *who) {
-  XYZ_CUDA_TRY(cudaStreamSynchronize(st));
-  volatile int *const e = g.h_err;
-  if (*e) {
-    *e = 0;
-    return set_error(XYZGPU_E_CUDA, "%s: a tensor-core wait timed out", who);
-  }
+// Every call that launches the network's kernels holds one of these from before
+// its first launch.
+auto error_word(GuideImpl &g, cudaStream_t st) {
+  return ErrorWordUse(g.h_err, [st] { return cudaStreamSynchronize(st); });
+}
+
+template <class Word>
+int check_err(Word &word, const char *who) {
+  bool const gave_up = word.take();
+  XYZ_CUDA_TRY(static_cast<cudaError_t>(word.status()));
+  if (gave_up) return set_error(XYZGPU_E_CUDA, "%s: a tensor-core wait timed out", who);
   return XYZGPU_OK;
 }
 
@@ -1385,9 +1390,10 @@ int xyzgpu_guide_forward(xyzgpu_guide h, const float *features, int n, float *ou
   GuideImpl &g = h->g;
   cudaStream_t const st = static_cast<cudaStream_t>(stream);
   XYZ_CUDA_TRY(cudaSetDevice(g.device));
+  auto word = error_word(g, st);
   int const rc = guide_forward_launch(g, features, n, out, st);
   if (rc) return rc;
-  return check_err(g, st, "guide_forward");
+  return check_err(word, "guide_forward");
 }
 
 int xyzgpu_guide_gradient(xyzgpu_guide h, const float *records, int n, float scale, float *grad, void *stream) {
@@ -1397,9 +1403,10 @@ int xyzgpu_guide_gradient(xyzgpu_guide h, const float *records, int n, float sca
   GuideImpl &g = h->g;
   cudaStream_t const st = static_cast<cudaStream_t>(stream);
   XYZ_CUDA_TRY(cudaSetDevice(g.device));
+  auto word = error_word(g, st);
   int const rc = guide_gradient_launch(g, records, n, scale, grad, st);
   if (rc) return rc;
-  return check_err(g, st, "guide_gradient");
+  return check_err(word, "guide_gradient");
 }
 
 int xyzgpu_render_guided(xyzgpu_guide h, const xyzgpu_camera *cam, const xyzgpu_render_params *rp, int train,
@@ -1428,10 +1435,11 @@ int xyzgpu_render_guided(xyzgpu_guide h, const xyzgpu_camera *cam, const xyzgpu_
     return set_error(XYZGPU_E_INVALID, "render_guided: scenes with mirror or metal materials are not guided");
   cudaStream_t const st = static_cast<cudaStream_t>(stream);
   XYZ_CUDA_TRY(cudaSetDevice(g.device));
+  auto word = error_word(g, st);
   GuideHooks hooks{&g, train != 0};
   int const rc = render_launch(*g.scene, *cam, *rp, film, st, nullptr, &hooks);
   if (rc) return rc;
-  return check_err(g, st, "render_guided");
+  return check_err(word, "render_guided");
 }
 
 int xyzgpu_guide_stats_get(xyzgpu_guide h, xyzgpu_guide_stats *out) {
@@ -1452,13 +1460,14 @@ int xyzgpu_guide_train_step(xyzgpu_guide h, const float *records, int n, void *s
   GuideImpl &g = h->g;
   cudaStream_t const st = static_cast<cudaStream_t>(stream);
   XYZ_CUDA_TRY(cudaSetDevice(g.device));
+  auto word = error_word(g, st);
   int rc = guide_gradient_launch(g, records, n, 1.0f / static_cast<float>(n), g.d_grad, st);
   if (rc) return rc;
   rc = adam_pack_launch(g, guide_dev(g), 0, 0, 0, st);
   if (rc) return rc;
   k_guide_advance<<<1, 32, 0, st>>>(g.d_ts, 1, 0, 0, 0);
   XYZ_CUDA_TRY(cudaGetLastError());
-  return check_err(g, st, "guide_train_step");
+  return check_err(word, "guide_train_step");
 }
 
 int xyzgpu_guide_reserve(xyzgpu_guide h, int64_t wave_paths, int train, void *stream) {
