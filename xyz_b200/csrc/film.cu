@@ -266,7 +266,9 @@ __global__ void __launch_bounds__(kFilmThreads)
     k_film_tonemap(const float *__restrict__ film, int W, int H, ToneArgs T, int vec, int words,
                    uint8_t *__restrict__ out) {
   float const white = T.white_bits ? __uint_as_float(*T.white_bits) : T.white;
-  float const inv_white2 = __fdividef(1.0f, white * white);
+  // (a white point whose square is far out of range: tone_fast has no answer)
+  float const white2 = white * white;
+  float const inv_white2 = white2 > 1e-30f && white2 < 1e30f ? 1.0f / white2 : __int_as_float(0x7fffffff);
   int64_t const stride_b = (3 * static_cast<int64_t>(W) + 3) & ~int64_t{3};
   int const quads = (W + 3) >> 2;
   int64_t const n = static_cast<int64_t>(quads) * H;
