@@ -213,34 +213,49 @@ __device__ __forceinline__ float rcp_fast(float x) {
   return r;
 }
 
+__device__ __forceinline__ float clamp_nan(float x, float lo, float hi) {
+  float r;
+  asm("{ .reg .f32 t; max.NaN.f32 t, %1, %2; min.NaN.f32 %0, t, %3; }" : "=f"(r) : "f"(x), "f"(lo), "f"(hi));
+  return r;
+}
+
 // The same byte by the fast reciprocal, exponential and logarithm where their
-// result p (in 256ths) lies clear of an integer, or -1 where tone_exact has to
-// be asked.  With L = log2 v and g <= 1, p errs by p (1.7e-7 (1 + |L|) g + 2.4e-7)
-// from the logarithm (2^-22, relative below 1/2) and the power, and by p 1e-6 g
-// from the operator (6 roundings and a reciprocal of 1 ulp): at most 4.5e-4, so
-// 5e-4 is clear.  The film operator 1 - e^-x, used from x = 0.05 on, errs by
-// 256 * 3.6e-6 = 9e-4 (the cancellation, on either side): 2e-3.  Zeros,
-// infinities and NaN (which end at 0 or 1e6 exactly) and other exponents are
-// not clear.
+// result p (in 256ths) lies clear of an integer, or -1 where tone_exact has to be
+// asked.  p = 256 v^g up to 257 errs, with L = log2 v, by p (1.7e-7 (1 + |L|) g +
+// 2.4e-7) from the logarithm (2^-22, relative below 1/2) and the power, by 1e-6 p g
+// from the operator (6 roundings and a reciprocal of 1 ulp) and tone_exact by 2.4e-7 p
+// from its power: 1.5e-4 + 3e-4 g, so 2e-4 + 3.5e-4 g is clear.  Of the film
+// operator's v = 1 - e^-x either side may be off by 2.1e-7 (the cancellation; below
+// 1/4 the series x - x^2/2 + ... is used here, tone_exact stays off): p by
+// 5e-7 g p / v.  Below half and above 255.5 no integer can matter (bytes 0 and 255),
+// except that a v too small for the fast logarithm may still be seen by exponents
+// below 0.1.  Where a rounding could take the Reinhard operators out of range (light
+// of 1e37 on, a white point whose square is not within 1e-30 .. 1e30; inv_white2 is
+// NaN then), for exponents above 16 and for NaN, tone_exact is asked.
+template <int kOp>
 __device__ __forceinline__ int tone_fast(float light, const ToneArgs &T, float inv_white2) {
   float v = T.exposure * light;
-  bool fast = T.gamma <= 1.0f;
-  float clear = 5e-4f;
-  if (T.op == XYZGPU_TONEMAP_REINHARD) {
+  float clear = T.gamma <= 16.0f ? 2e-4f + 3.5e-4f * T.gamma : 1.0f;
+  if (kOp == XYZGPU_TONEMAP_REINHARD) {
     v = v * rcp_fast(1.0f + light);
-  } else if (T.op == XYZGPU_TONEMAP_REINHARD_WHITE) {
+  } else if (kOp == XYZGPU_TONEMAP_REINHARD_WHITE) {
     v = v * (1.0f + light * inv_white2) * rcp_fast(1.0f + light);
-  } else if (T.op == XYZGPU_TONEMAP_FILM) {
-    fast = fast && v >= 0.05f;
-    clear = 2e-3f;
-    v = 1.0f - exp2_fast(-1.44269504f * v);
+  } else if (kOp == XYZGPU_TONEMAP_FILM) {
+    float s = __fmaf_rn(v, -1.0f / 720.0f, 1.0f / 120.0f);
+    s = __fmaf_rn(v, s, -1.0f / 24.0f);
+    s = __fmaf_rn(v, s, 1.0f / 6.0f);
+    s = __fmaf_rn(v, s, -0.5f);
+    s = __fmaf_rn(v, s, 1.0f);
+    v = fabsf(v) < 0.25f ? v * s : 1.0f - exp2_fast(-1.44269504f * v);
   }
-  float const p = fminf(exp2_fast(T.gamma * log2_fast(v)) * 256.0f, 1e6f);
+  // (a NaN stays one)
+  float const p = clamp_nan(exp2_fast(T.gamma * log2_fast(v)) * 256.0f, T.gamma >= 0.1f ? 0.5f : 0.0f, 255.5f);
+  if (kOp == XYZGPU_TONEMAP_FILM) clear += 5e-7f * T.gamma * p * rcp_fast(fabsf(v));
   // nearest integer in the low bits of p + 2^23
   float const q = p + 8388608.0f, r = q - 8388608.0f;
-  int const byte = min((__float_as_int(q) & 0x7fffff) - (p < r ? 1 : 0), 255);
-  fast = fast && fabsf(p - r) > clear;
-  return light <= 0.0f ? 0 : (fast ? byte : -1);
+  int const byte = (__float_as_int(q) & 0x7fffff) - (p < r ? 1 : 0);
+  bool const sure = fabsf(p - r) > clear && (kOp == XYZGPU_TONEMAP_LINEAR || kOp == XYZGPU_TONEMAP_FILM || light < 1e37f);
+  return light <= 0.0f ? 0 : (sure ? byte : -1);
 }
 
 __device__ __forceinline__ void tone_channels(const ToneArgs &T, float X, float Y, float Z, float c[3]) {
@@ -260,13 +275,15 @@ __device__ __forceinline__ void tone_channels(const ToneArgs &T, float X, float 
 // the film) and byte order (blue, green, red = channel 2, 1, 0); the row's
 // padding bytes are zero (the caller's buffer may hold anything).
 // Measured at 1920 x 1080 (Reinhard with the image's white): a pixel per
-// thread with powf and byte stores 37.0 us, this form 16.3 (issue-bound: 76 % of
-// cycles); the maximum before it 9.5 -> 5.1.
+// thread with powf and byte stores 37.0 us, this form 16.4 (issue-bound: 76 % of
+// cycles); the maximum before it 9.5 -> 5.1.  The film operator 18.8, on a film a
+// hundredth as bright too: whole calls 68 us with powf, 77 (89 if dark) with the
+// fast form for exposures from 0.05 and exponents up to 1 only, 52 now.
+template <int kOp>
 __global__ void __launch_bounds__(kFilmThreads)
     k_film_tonemap(const float *__restrict__ film, int W, int H, ToneArgs T, int vec, int words,
                    uint8_t *__restrict__ out) {
   float const white = T.white_bits ? __uint_as_float(*T.white_bits) : T.white;
-  // (a white point whose square is far out of range: tone_fast has no answer)
   float const white2 = white * white;
   float const inv_white2 = white2 > 1e-30f && white2 < 1e30f ? 1.0f / white2 : __int_as_float(0x7fffffff);
   int64_t const stride_b = (3 * static_cast<int64_t>(W) + 3) & ~int64_t{3};
@@ -285,7 +302,7 @@ __global__ void __launch_bounds__(kFilmThreads)
       tone_channels(T, v[3 * k], v[3 * k + 1], v[3 * k + 2], c);
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
-        int const at = 3 * k + j, byte = tone_fast(c[2 - j], T, inv_white2);
+        int const at = 3 * k + j, byte = tone_fast<kOp>(c[2 - j], T, inv_white2);
         w[at >> 2] |= static_cast<uint32_t>(byte & 0xff) << (8 * (at & 3));
         if (byte < 0 && k < m) ask |= 1u << at;
         if (k >= m) w[at >> 2] &= ~(0xffu << (8 * (at & 3)));
@@ -442,7 +459,11 @@ int xyzgpu_film_tonemap(const float *film, int width, int height, const xyzgpu_t
                                                                           aligned(film, 16), scratch_white);
     T.white_bits = scratch_white;
   }
-  k_film_tonemap<<<film_grid((static_cast<int64_t>(width) + 3) / 4 * height), kFilmThreads, 0, st>>>(
+  auto const kernel = tp->op == XYZGPU_TONEMAP_LINEAR           ? k_film_tonemap<XYZGPU_TONEMAP_LINEAR>
+                      : tp->op == XYZGPU_TONEMAP_REINHARD       ? k_film_tonemap<XYZGPU_TONEMAP_REINHARD>
+                      : tp->op == XYZGPU_TONEMAP_REINHARD_WHITE ? k_film_tonemap<XYZGPU_TONEMAP_REINHARD_WHITE>
+                                                                : k_film_tonemap<XYZGPU_TONEMAP_FILM>;
+  kernel<<<film_grid((static_cast<int64_t>(width) + 3) / 4 * height), kFilmThreads, 0, st>>>(
       film, width, height, T, aligned(film, 16) && width % 4 == 0, aligned(out, 4), out);
   XYZ_CUDA_TRY(cudaGetLastError());
   return XYZGPU_OK;
