@@ -152,7 +152,7 @@ RayHit kd_loop(const DevScene &S, f3 o, f3 d, float tmin, float tmax, double *no
 
 // The wide loop for one ray; false: it leaves the ray to the kd loop.
 bool wide_loop(const Trees &B, f3 o, f3 d, float tmin, float tmax, RayHit &h, double *nodes, double *tests) {
-  if (!wide_usable(o, d, B.S.wide_reach)) return false;
+  if (!wide_usable(o, d, B.S.wide_reach) || !(0.0f <= tmin && tmin <= tmax)) return false;
   h = RayHit{tmax, 0.0f, 0.0f, -1, 0};
   float tlim = tmax, slack = 0.0f;
   WideRay const R = wide_ray(o, d);

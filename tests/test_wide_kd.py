@@ -168,3 +168,20 @@ def test_queues_of_axis_parallel_rays(extra, share):
     rays[flat, 4:7] = d[flat]
     rays[flat, 0:3] = (p - d)[flat]
     assert compare(scene_of(pos), rays) > 1 << 14
+
+
+@pytest.mark.gpu
+def test_intervals_that_are_no_interval():
+    """tmin or tmax not a number (which the triangle test lets pass), negative tmin,
+    empty intervals, an infinite tmin."""
+    pos = np.concatenate([slivers(1e-2), terrain(40, 0.0)]).astype(np.float32)
+    rays = edge_rays(pos, 1 << 17, 8)
+    k = np.arange(rays.shape[0]) % 8
+    rays[k == 0, 7] = np.nan
+    rays[k == 1, 3] = np.nan
+    rays[k == 2, 3] = -np.inf
+    rays[k == 3, 3] = -3.0
+    rays[k == 4, 7] = 0.0
+    rays[k == 5, 3] = np.inf
+    rays[k == 6, 3:8:4] = np.nan
+    assert compare(scene_of(pos), rays) > 1 << 14
