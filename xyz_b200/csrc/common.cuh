@@ -58,6 +58,12 @@ XYZ_HD int octant_of(float y, float x) {
   return 2 * quad + (((quad & 1) != 0) != steep ? 1 : 0);
 }
 
+// Queue arithmetic up to the largest int: CTAs or lanes for n items, `per` each
+// (n >= 0), and whether item i, taken from a counter that runs past n by as much
+// as there are lanes, lies beyond the queue.
+XYZ_HD int ceil_div(int n, int per) { return n > 0 ? (n - 1) / per + 1 : 0; }
+XYZ_HD bool beyond_queue(int i, int n) { return static_cast<uint32_t>(i) >= static_cast<uint32_t>(n); }
+
 // ---------------------------------------------------------------- random
 // Philox4x32-10 (Salmon et al., SC'11).  Stream layout in include/xyzgpu.h.
 XYZ_HD void philox4x32_10(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, uint32_t k0,

@@ -124,7 +124,7 @@ int trace_api_launch(SceneImpl &s, const float *rays, int n, float *hits, cudaSt
   } else {
     static int wide_grid = 0, kd_grid = 0;
     int const full = grid_for(k_trace_api<false>, wide_grid, s.device);
-    int const grid = std::min(full, (n + kRaysPerCta - 1) / kRaysPerCta);
+    int const grid = std::min(full, ceil_div(n, kRaysPerCta));
     bool const kd_follows = n / (2 * kTraceThreads) >= full;
     k_trace_api<false><<<grid, kTraceThreads, 0, st>>>(s.dev, r4, n, h4, s.d_fetch, nullptr, kd_follows);
     XYZ_CUDA_TRY(cudaGetLastError());

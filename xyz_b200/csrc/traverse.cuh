@@ -125,7 +125,7 @@ XYZ_DEV void trace_persistent(const DevScene &S, int n, int *fetch, Sink &sink, 
       base = __shfl_sync(0xffffffffu, base, leader);
       if (need) {
         int const i = base + __popc(want & lanes_below);
-        if (i >= n) {
+        if (beyond_queue(i, n)) {
           exhausted = true;
         } else {
           float tmax;
@@ -321,7 +321,7 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
   unsigned const lanes_below = (1u << lane) - 1u;
   // short queues: fewer lanes per warp, so that all warps have a share and a
   // warp's rays wait for fewer others
-  int const width = min(32, max(1, (n + warps - 1) / warps));
+  int const width = min(32, max(1, ceil_div(n, warps)));
   int const refill_at = width < 32 ? 0 : 32 - ((kBatch || S.n_wide > kWideTinyNodes) ? kWideRefill : kWideRefillTiny);
   bool exhausted = lane >= width;
   bool kd_only = false;  // the same on every lane
@@ -363,7 +363,7 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
           first = __shfl_sync(0xffffffffu, first, leader);
           if (want & (1u << lane)) {
             int const i = first + __popc(want & lanes_below);
-            if (i >= n) {
+            if (beyond_queue(i, n)) {
               exhausted = true;
             } else {
               float tmax;
