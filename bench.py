@@ -41,9 +41,8 @@ W_PIX, H_PIX, SPP, MAX_DEPTH, SEED = 1024, 1024, 64, 10, 0
 METRIC = "Msamples/s on 1 B200 (path samples per second, 1M-triangle scene)"
 UNIT = "Msamples/s"
 L2_FLUSH_BYTES = 256 << 20
-TRI_BYTES_ALGO = 36   # v0, e1, e2 as the reference stores a triangle
-NODE_BYTES = 8
-REF_BYTES = 4
+NODE_BYTES = 96       # wide-tree node
+TRI_BYTES = 64        # its triangle record
 RAY_IO_BYTES = 32 + 16
 
 
@@ -710,16 +709,18 @@ def trace_micro_bench(scene, sd, n=1 << 24, seed=0, reps=5):
         ms = timed(r, hts)
         c = scene.trace_device(r, hts, counted=True)
         nr = max(1, c["rays"])
-        algo = (RAY_IO_BYTES * c["rays"] + NODE_BYTES * c["nodes_visited"] +
-                (REF_BYTES + TRI_BYTES_ALGO) * c["tri_tests"]) / nr
-        gbs = algo * (hi - lo) / (ms * 1e-3) / 1e9
+        per_kind = [wide_bytes_per_ray(k) for k in {"all": ("camera", "bounce"), "primary": ("camera",),
+                                                    "bounce": ("bounce",)}[name]]
+        algo = None if None in per_kind else sum(per_kind) / len(per_kind)
+        gbs = None if algo is None else algo * (hi - lo) / (ms * 1e-3) / 1e9
         res[name] = {"rays": hi - lo, "ms": round(ms, 3), "mrays_per_s": round((hi - lo) / ms / 1e3, 1),
                      "hit_rate": round(c["hits"] / nr, 4),
-                     "per_ray": {"nodes": round(c["nodes_visited"] / nr, 2),
-                                 "leaves": round(c["leaves_visited"] / nr, 2),
-                                 "tri_tests": round(c["tri_tests"] / nr, 2)},
-                     "algorithmic_bytes_per_ray": round(algo, 1),
-                     "achieved_gbs": round(gbs, 1), "frac_of_hbm": round(gbs / peak, 4)}
+                     "kd_tree_per_ray": {"nodes": round(c["nodes_visited"] / nr, 2),
+                                         "leaves": round(c["leaves_visited"] / nr, 2),
+                                         "tri_tests": round(c["tri_tests"] / nr, 2)},
+                     "algorithmic_bytes_per_ray": None if algo is None else round(algo, 1),
+                     "achieved_gbs": None if gbs is None else round(gbs, 1),
+                     "frac_of_hbm": None if gbs is None else round(gbs / peak, 4)}
     res["peak_gbs"] = peak
     res["peak_source"] = peak_kind
     res["config"] = ("2^24 rays of the workload's scene and kd-tree: 2^23 pinhole camera rays through "
@@ -784,9 +785,9 @@ def gpu_lead(ms: float = 100.0):
     torch.cuda._sleep(int(ms * 1e-3 * 1.9e9))
 
 
-def profiled_traffic(key: str = "dram_bytes_per_ray"):
-    """Bytes per traced ray of the trace kernel (`key`: dram_bytes_per_ray or
-    l2_bytes_per_ray) from the committed ncu summary
+def profiled(key: str):
+    """A per-ray figure of the trace kernels (dram_bytes_per_ray, l2_bytes_per_ray,
+    wide_nodes_per_..., wide_tests_per_...) from the committed profile
     (profiles/trace_queue_spheres1m.txt), if present."""
     p = os.path.join(ROOT, "profiles", "trace_queue_spheres1m.txt")
     if not os.path.exists(p):
@@ -798,6 +799,14 @@ def profiled_traffic(key: str = "dram_bytes_per_ray"):
             except ValueError:
                 return None
     return None
+
+
+def wide_bytes_per_ray(kind: str):
+    """Bytes of a `kind` (extension, shadow, camera, bounce) ray of the workload's
+    scene: the ray and its hit, and the nodes and triangle records that the
+    eight-wide tree's walk reads for it."""
+    nodes, tests = profiled(f"wide_nodes_per_{kind}_ray"), profiled(f"wide_tests_per_{kind}_ray")
+    return None if nodes is None or tests is None else RAY_IO_BYTES + nodes * NODE_BYTES + tests * TRI_BYTES
 
 
 def measure_l2_copy_gbs(mib: int = 32, reps: int = 100):
@@ -897,21 +906,20 @@ def run_gpu_arm(args, rank, world):
     ms_cls = {c: prof["ms"][c] * args.steps for c in api.KERNEL_CLASSES}
     n_cls = {c: prof["launches"][c] * args.steps for c in api.KERNEL_CLASSES}
     launches = scene.render_counters()["kernel_launches"] * args.steps
-    # work per ray from one counted render (outside the timed region): of the
-    # kd-tree walk, so that the figure compares between traversals
+    # rays of a step, and the kd-tree's work per ray (a counted render walks it),
+    # outside the timed region; the timed kernels walk the wide tree, whose work
+    # per ray the committed profile gives
     step(offset, profile=2)
     cp = scene.render_profile()
     counters = scene.render_counters()
-    ext_bytes = (cp["ext_rays"] * RAY_IO_BYTES + cp["ext_nodes"] * NODE_BYTES +
-                 cp["ext_tri_tests"] * (REF_BYTES + TRI_BYTES_ALGO))
-    sh_bytes = (cp["shadow_rays"] * RAY_IO_BYTES + cp["shadow_nodes"] * NODE_BYTES +
-                cp["shadow_tri_tests"] * (REF_BYTES + TRI_BYTES_ALGO))
+    ext_ray, sh_ray = wide_bytes_per_ray("extension"), wide_bytes_per_ray("shadow")
+    algo_bytes = None if ext_ray is None or sh_ray is None else cp["ext_rays"] * ext_ray + cp["shadow_rays"] * sh_ray
     trace_ms = (ms_cls["trace_extension"] + ms_cls["trace_shadow"]) / max(1, args.steps)
     trace_launches = (n_cls["trace_extension"] + n_cls["trace_shadow"]) / max(1, args.steps)
     peak, peak_kind = measured_peaks()
-    achieved = (ext_bytes + sh_bytes) / (trace_ms / 1000.0) / 1e9 if trace_ms > 0 else 0.0
+    achieved = algo_bytes / (trace_ms / 1000.0) / 1e9 if algo_bytes is not None and trace_ms > 0 else 0.0
     rays = cp["ext_rays"] + cp["shadow_rays"]
-    per_ray_traffic = profiled_traffic()
+    per_ray_traffic = profiled("dram_bytes_per_ray")
     traffic = None
     if per_ray_traffic is not None and trace_launches:
         traffic = per_ray_traffic * rays / trace_launches
@@ -920,10 +928,10 @@ def run_gpu_arm(args, rank, world):
         "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
         "frac": round(achieved / peak, 4), "peak_source": peak_kind,
         "traffic": traffic,
-        "algorithmic_bytes_per_ray": round((ext_bytes + sh_bytes) / max(1, rays), 1),
-        "bytes_source": "per-ray counts of a counted render, which walks the kd-tree; the timed kernels walk "
-                        "the eight-wide tree derived from it, so a fraction above what they move is possible",
-        "per_ray": {"nodes": round((cp["ext_nodes"] + cp["shadow_nodes"]) / max(1, rays), 2),
+        "algorithmic_bytes_per_ray": None if algo_bytes is None else round(algo_bytes / max(1, rays), 1),
+        "bytes_source": "48 bytes a ray, 96 a node and 64 a triangle record of the wide tree's walk "
+                        "(per-ray counts of profiles/trace_queue_spheres1m.txt)",
+        "kd_tree_per_ray": {"nodes": round((cp["ext_nodes"] + cp["shadow_nodes"]) / max(1, rays), 2),
                     "tri_tests": round((cp["ext_tri_tests"] + cp["shadow_tri_tests"]) / max(1, rays), 2),
                     "extension": {"rays": cp["ext_rays"],
                                   "nodes": round(cp["ext_nodes"] / max(1, cp["ext_rays"]), 2),
@@ -942,7 +950,7 @@ def run_gpu_arm(args, rank, world):
     }
     # the traversal's working set (tree and triangles, about 100 MB) lives in
     # L2, so its roof is also stated against a copy that stays in L2
-    l2_per_ray = profiled_traffic("l2_bytes_per_ray")
+    l2_per_ray = profiled("l2_bytes_per_ray")
     if l2_per_ray is not None and trace_ms > 0:
         l2_peak = measure_l2_copy_gbs()
         l2_ach = l2_per_ray * rays / (trace_ms * 1e-3) / 1e9

@@ -39,3 +39,16 @@ def test_relmse_of_the_reference_itself_is_zero_on_average():
     relmse, ref_noise, _ = bench.relmse_estimator(a, b)
     # an image as noisy as one half has twice the reference's own noise
     assert abs(relmse(c) - 2 * ref_noise) < 0.05 * ref_noise
+
+
+def test_trace_roofline_counts_the_wide_walk():
+    """The roofline's bytes per ray are those of the walk that is timed: the ray
+    and its hit, 96 bytes a wide node and 64 a triangle record, for every kind of
+    ray the bench times."""
+    import bench
+    for kind in ("extension", "shadow", "camera", "bounce"):
+        nodes = bench.profiled(f"wide_nodes_per_{kind}_ray")
+        tests = bench.profiled(f"wide_tests_per_{kind}_ray")
+        assert nodes >= 1.0 and tests > 0.0
+        assert bench.wide_bytes_per_ray(kind) == 48 + 96 * nodes + 64 * tests
+    assert bench.wide_bytes_per_ray("no such") is None
