@@ -264,10 +264,11 @@ XYZ_DEV void trace_persistent(const DevScene &S, int n, int *fetch, Sink &sink, 
 // to be so (grazing to 1e-6, within a tenth of an edge) one in a million differs
 // among loose triangles, none in 16 million in the closed scenes.
 //
-// Why: the kd loop runs at 8 of 32 lanes per instruction and 351 warp
-// instructions per ray, 43 dependent node loads and 16 triangle tests a ray;
-// a wide node costs one round of uniform arithmetic on eight boxes for three
-// 32-byte loads, and a ray needs about ten of them.
+// Why: a cosine bounce on a 1M-triangle mesh takes the kd loop 44 dependent node
+// loads and 15 triangle tests, at 8 of 32 lanes and 351 warp instructions a ray (the
+// second bounce of a render); a wide node costs one round of uniform arithmetic on
+// eight boxes for three 32-byte loads, and the ray needs eight of them and five
+// tests, at 17 lanes and 174 instructions.
 constexpr int kWideRetry = 128;  // list entries per warp; 64 + one refill + the lanes under way fit
 constexpr int kWideRetryFull = 64;
 

@@ -583,9 +583,11 @@ struct ShadowSink {
 // counters, which no bounce uses.
 XYZ_DEV int32_t *wave_taken(const WaveArgs &A) { return A.counts + A.kmax * kCountStride; }
 
-// CTAs per SM: 8 (64 registers) for the wide tree, which spills at 10 (+45 % on
-// the 1M-triangle scene); counted renders, on the kd-tree, run at 9 (extension
-// rays, 56 registers) and 10 (shadow rays, 48).
+// CTAs per SM: 8 (64 registers) for the wide tree, whose kernels spill up to 80
+// bytes a thread there (batched k_trace_both 112) and far more at 10 (+45 % on the
+// 1M-triangle scene); counted renders, on the kd-tree, run at 9 (extension rays, 56
+// registers) and 10 (shadow rays, 48 and 124 bytes).  The kernels hold the stacks
+// of both walks, 512 and 480 bytes.
 template <bool kShadow, bool kCount, int kMode = kModePlain>
 __global__ void __launch_bounds__(kThreads, kCount ? (kShadow ? 10 : 9) : 8) k_trace_queue(WaveArgs A, int b,
                                                           unsigned long long *prof) {
@@ -648,10 +650,17 @@ __global__ void __launch_bounds__(kThreads, kCount ? (kShadow ? 10 : 9) : 8) k_t
 // not depend on one another, in one launch: one tail instead of two per bounce.
 // Long queues are traced one after the other by every warp (shadow rays first);
 // short ones, which are all tail, as one queue whose rays share their warps
-// (BothSink, extension rays first).  Device time of a render (ms), two launches /
-// one queue / one after the other: 4,096-path preview 0.55 / 0.36 / 0.40, 1 M
-// spectral paths 1.17 / 1.05 / 1.01, 1.6 M paths of a 247,042-triangle frame 6.54
-// / 5.66 / 5.78, 67 M paths of the 1M-triangle mesh 44.3 / 44.4 / 42.6.
+// (BothSink, extension rays first).  Renders of depth 10 (us), one after the
+// other / one queue: XYZ (smaller waves run in one launch, k_small_wave) 134,400
+// paths 445 / 406 (Cornell box), 646 / 597 (62,722-triangle mesh), 1,012 / 941
+// (984,322); 262,144 paths 534 / 515, 783 / 729, 1,206 / 1,123; spectral (box,
+// depth 8) 420 / 376 and 512 / 480; guided 4,096 / 65,536 / 262,144 paths 738 / 689,
+// 1,060 / 902, 1,593 / 1,374; importance-driven 967 / 866, 1,770 / 1,512, 3,486 /
+// 3,245; adjoint iterations whose replay traces, depth 6, 65,536 / 524,288 paths
+// 1,488 / 1,330 and 4,517 / 4,193.  Above the line it depends on the scene: 2^19,
+// 2^20, 2^22 paths 754 / 727, 1,146 / 1,153, 3,465 / 3,604 (box), 1,416 / 1,343,
+// 1,799 / 1,667, 3,756 / 3,634 (984,322 triangles; 67 M paths, with an earlier walk,
+// 42.6 / 44.4 ms).
 constexpr int64_t kMixedPaths = int64_t{1} << 18;
 
 template <bool kSpec, int kMode>
@@ -1576,8 +1585,8 @@ struct LocalSink {
 // 816 / 622; 131,072 paths 456 / 282, 970 / 543, 1042 / 1012; 262,144 paths
 // 549 / 414, 1312 / 804, 1430 / 1750.
 // Larger waves: launched before the shading of every second bounce from the
-// fifth on while four are left (small_wave_at; with two left the adjoint below of
-// 262,144 paths loses 2 %), it takes over once that few rays are left (traced
+// fifth on while four are left (small_wave_at; with two left an adjoint of 262,144
+// paths and depth 6 loses 2 %), it takes over once that few rays are left (traced
 // already: a path's shadow ray of the bounce before is in another CTA's share) and
 // is empty until then.  Depth 10, without / with it: 204,800 paths 476 / 447 us
 // (box), 1097 / 1017 (mesh), 1622 / 1463 (1M-triangle mesh), 1275 / 1275 (room);
@@ -1586,8 +1595,9 @@ struct LocalSink {
 // 486 / 199 (mesh); 131,072 paths 454 / 305, 966 / 542; 524,288 paths 790 / 729,
 // 1673 / 1490.
 // An adjoint's primal pass takes it too: forward and backward of 4,096 / 32,768 /
-// 131,072 / 262,144 paths of a room 572 / 758 / 1574 / 2406 -> 506 / 669 / 1504 /
-// 2392 us.
+// 131,072 / 262,144 paths of a room of depth 6 658 / 886 / 1410 / 2017 -> 486 / 742 /
+// 1368 / 2018 us (the last is not taken over), of depth 10 990 / 1366 / 2075 / 2933 ->
+// 690 / 1102 / 1959 / 2929.
 // Launched before every bounce, the empty launches cost a closed room up to 4 %
 // and an early take-over a box of depth 4 13 %; taking over at 2^15 or 2^16 rays
 // gains the meshes a third to two thirds as much.
