@@ -50,11 +50,13 @@ bool build(const std::vector<f3> &V, Trees &B) {
   const std::vector<uint2> &nd = B.nodes;
   std::vector<uint4> lo(nn, make_uint4(~0u, ~0u, ~0u, ~0u)), hi(nn, make_uint4(0, 0, 0, 0));
   std::vector<int32_t> first(nn, 0), owner(n);
+  std::vector<uint32_t> extents(kWideExtents, 0u);
   for (int i = 0; i < n; ++i) {
     f3 const v0 = V[3 * i], e1 = xyz3(B.tri[3 * i + 1]), e2 = xyz3(B.tri[3 * i + 2]);
     WideTri const w =
         wide_triangle(v0, e1, e2, mk3(B.tri[3 * i].w, B.tri[3 * i + 1].w, B.tri[3 * i + 2].w));
     B.lengths.push_back(w);
+    ++extents[wide_extent_bucket(w.e)];
     f3 const sum = add3(add3(v0, add3(v0, e1)), add3(v0, e2));
     int const l = owner[i] = wide_leaf_of(nd.data(), scl3(sum, 1.0f / 3.0f));
     uint32_t *const L = &lo[l].x, *const H = &hi[l].x;
@@ -101,9 +103,11 @@ bool build(const std::vector<f3> &V, Trees &B) {
   B.S.tri = B.tri.data();
   B.S.nodes = B.nodes.data();
   B.S.refs = B.kd.refs.data();
-  B.S.wide_reach = reach * kWideReach;
   B.S.bmin = mk3(B.kd.bmin[0], B.kd.bmin[1], B.kd.bmin[2]);
   B.S.bmax = mk3(B.kd.bmax[0], B.kd.bmax[1], B.kd.bmax[2]);
+  f3 const half = scl3(sub3(B.S.bmax, B.S.bmin), 0.5f);
+  B.S.wide_mid = add3(B.S.bmin, half);
+  B.S.wide_reach = wide_reach_of(std::max({half.x, half.y, half.z}), reach, extents.data(), static_cast<uint32_t>(n));
   return true;
 }
 
@@ -150,9 +154,8 @@ RayHit kd_loop(const DevScene &S, f3 o, f3 d, float tmin, float tmax, double *no
   }
 }
 
-// The wide loop for one ray; false: it leaves the ray to the kd loop.
+// The wide loop for one ray that the tree takes; false: it leaves the ray to the kd loop.
 bool wide_loop(const Trees &B, f3 o, f3 d, float tmin, float tmax, RayHit &h, double *nodes, double *tests) {
-  if (!wide_usable(o, d, B.S.wide_reach) || !(0.0f <= tmin && tmin <= tmax)) return false;
   h = RayHit{tmax, 0.0f, 0.0f, -1, 0};
   float tlim = tmax, slack = 0.0f;
   WideRay const R = wide_ray(o, d);
@@ -203,10 +206,10 @@ void terrain(std::vector<f3> &v, int m, float at) {
 
 }  // namespace
 
-// scenes: sliver:WIDTH (200 long thin triangles), soup:SIZE, terrain:OFFSET, ground:HALF (a terrain patch above a
-// ground that wide), boxes
+// scenes: sliver:WIDTH (200 long thin triangles), soup:SIZE, terrain:OFFSET, grid:SIDE (a terrain of so many squares
+// a side), ground:HALF (a terrain patch above a ground that wide), boxes
 // kinds: edge (rays at a point 1e-7 to 1e-1 of a triangle inside or beyond one of its edges, from near and far),
-// local (rays between two points of the scene's finely divided part)
+// far (the same from 10 to 30,000 scene sizes), local (rays between two points of the scene's finely divided part)
 int main(int argc, char **argv) {
   if (argc != 4) return 1;
   std::string const scene = argv[1], kind = argv[3];
@@ -229,6 +232,8 @@ int main(int argc, char **argv) {
     }
   } else if (scene.rfind("terrain", 0) == 0) {
     terrain(v, 120, arg);
+  } else if (scene.rfind("grid", 0) == 0) {
+    terrain(v, static_cast<int>(arg), 0.0f);
   } else if (scene.rfind("ground", 0) == 0) {
     terrain(v, 120, 0.0f);
     quad(v, mk3(-arg, -1, -arg), mk3(arg, -1, -arg), mk3(arg, -1, arg), mk3(-arg, -1, arg));
@@ -254,13 +259,13 @@ int main(int argc, char **argv) {
   for (long r = std::atol(argv[2]); r > 0; --r) {
     int const i = static_cast<int>(g() % fine);
     f3 o, d;
-    if (kind == "edge") {
+    if (kind == "edge" || kind == "far") {
       int const k = static_cast<int>(g() % 3);
       f3 const a = v[3 * i + k], b = v[3 * i + (k + 1) % 3], c = v[3 * i + (k + 2) % 3];
       float const past = std::pow(10.0f, -4 + 3 * U(g)) * (g() % 4 ? 1.0f : -1.0f);
       f3 const e = add3(a, scl3(sub3(b, a), 0.5f + 0.5f * U(g)));
       d = unit(mk3(N(g), N(g), N(g)));
-      o = sub3(add3(e, scl3(sub3(e, c), past)), scl3(d, size * std::pow(10.0f, -0.5f + U(g))));
+      o = sub3(add3(e, scl3(sub3(e, c), past)), scl3(d, size * std::pow(10.0f, kind == "far" ? 2.75f + 1.75f * U(g) : -0.5f + U(g))));
     } else {
       float const a = 0.5f + 0.5f * U(g), b = (0.5f + 0.5f * U(g)) * (1 - a);
       o = add3(point(static_cast<int>(g() % fine), 0.3f, 0.3f), mk3(0, 0.3f + 0.2f * U(g), 0));
@@ -269,6 +274,7 @@ int main(int argc, char **argv) {
     RayHit w, k = kd_loop(B.S, o, d, kRayTMin, INFINITY, &n[2], &n[3]);
     ++rays;
     hits += k.id >= 0;
+    if (!wide_usable(sub3(o, B.S.wide_mid), d, B.S.wide_reach)) continue;
     if (!wide_loop(B, o, d, kRayTMin, INFINITY, w, &n[0], &n[1]))
       ++unsettled;
     else

@@ -112,6 +112,14 @@ def test_answers_at_large_coordinates(check, scene):
     assert differ == 0
 
 
+def test_rays_from_far_beyond_the_scene(check):
+    """Rays up to 30,000 scene sizes away keep the kd-tree's work: the tree's boxes,
+    widened by the distance, would no longer separate the triangles."""
+    rays, hits, _, differ, _, tests, _, kd_tests = check("terrain:0", 100000, "far")
+    assert hits > rays / 2 and differ == 0
+    assert tests < 1.5 * kd_tests
+
+
 def terrain(n, at):
     x = np.linspace(-1, 1, n + 1)
     X, Z = np.meshgrid(x, x, indexing="ij")
@@ -185,3 +193,20 @@ def test_intervals_that_are_no_interval():
     rays[k == 5, 3] = np.inf
     rays[k == 6, 3:8:4] = np.nan
     assert compare(scene_of(pos), rays) > 1 << 14
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("side", [7, 60])
+def test_far_rays_hit_as_in_the_kd_tree(side):
+    """Rays from 10 to 10,000 scene sizes at a terrain they meet at all slopes, some
+    so small that the triangle test's error exceeds the triangles."""
+    pos = terrain(side, 0.0).astype(np.float32)
+    rng = np.random.default_rng(9)
+    n = 1 << 21
+    t = pos[rng.integers(0, pos.shape[0], n)].astype(np.float64)
+    d = rng.normal(size=(n, 3)) * [1.0, 0.05, 1.0]
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    rays = np.empty((n, 8), np.float32)
+    rays[:, 0:3] = (rng.dirichlet([1, 1, 1], n)[..., None] * t).sum(1) - d * 2.0 * 10.0 ** rng.uniform(1, 4, (n, 1))
+    rays[:, 3], rays[:, 4:7], rays[:, 7] = 1e-5, d, np.inf
+    assert compare(scene_of(pos), rays) > 1 << 19

@@ -139,7 +139,8 @@ struct DevScene {
   const int32_t *refs;
   const uint32_t *wide;     // wide tree (wide.cuh) and its triangle records, or null
   const float4 *wide_tri;
-  float wide_reach;         // largest origin coordinate of the rays it serves
+  f3 wide_mid;              // the scene's middle, and how far from it (along an
+  float wide_reach;         // axis) the rays that it serves may start
   int n_wide;               // its nodes
   int n_lights;
   float light_area;

@@ -35,6 +35,7 @@
 // positions in depth-first order from the root down; k_wide_nodes then builds
 // the wide nodes level by level and k_wide_tris writes the triangle records.
 #include <algorithm>
+#include <cstddef>
 #include <vector>
 
 #include "scene.h"
@@ -990,8 +991,12 @@ __global__ void k_layout_scatter(const uint2 *__restrict__ nodes, int64_t n, con
 // ---- wide tree
 // Each triangle joins the kd leaf that holds its centroid: the leaf's box and
 // count take it in.
-__global__ void k_wide_assign(const float4 *__restrict__ tri, int n, const uint2 *__restrict__ nodes, WideSets T,
-                              int32_t *__restrict__ owner) {
+__global__ void __launch_bounds__(256)
+    k_wide_assign(const float4 *__restrict__ tri, int n, const uint2 *__restrict__ nodes, WideSets T,
+                  int32_t *__restrict__ owner, uint32_t *extents) {
+  __shared__ uint32_t s_extents[kWideExtents];
+  for (int i = threadIdx.x; i < kWideExtents; i += blockDim.x) s_extents[i] = 0u;
+  __syncthreads();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     float4 const a = tri[3 * i], b = tri[3 * i + 1], c = tri[3 * i + 2];
     // vertices as the intersection test sees them: v0, v0 + e1, v0 + e2
@@ -999,6 +1004,7 @@ __global__ void k_wide_assign(const float4 *__restrict__ tri, int n, const uint2
     int32_t const leaf = wide_leaf_of(nodes, scl3(add3(add3(v0, add3(v0, e1)), add3(v0, e2)), 1.0f / 3.0f));
     WideTri const w = wide_triangle(v0, e1, e2, mk3(a.w, b.w, c.w));
     owner[i] = leaf;
+    atomicAdd(&s_extents[wide_extent_bucket(w.e)], 1u);
     uint32_t *const lo = reinterpret_cast<uint32_t *>(T.lo + leaf);
     uint32_t *const hi = reinterpret_cast<uint32_t *>(T.hi + leaf);
 #pragma unroll
@@ -1008,6 +1014,9 @@ __global__ void k_wide_assign(const float4 *__restrict__ tri, int n, const uint2
     }
     atomicAdd(hi + 3, 1u);
   }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kWideExtents; i += blockDim.x)
+    if (s_extents[i]) atomicAdd(&extents[i], s_extents[i]);
 }
 
 // State of the level-by-level construction: nodes and records handed out, the
@@ -1017,6 +1026,7 @@ struct WideCounters {
   uint32_t nodes, tris;
   uint32_t level[kWideStack + 3];
   uint32_t done[kWideStack + 1];
+  uint32_t extents[kWideExtents];  // triangles by extent (k_wide_assign)
 };
 
 constexpr int kWideThreads = 64;
@@ -1246,14 +1256,14 @@ struct WideBufs {
 
 // Fills the wide tree from the sets of the breadth-first kd nodes.  A tree
 // deeper than the traversal's stack is dropped (the kd-tree serves alone).
-int wide_build(SceneImpl &s, WideBufs &B, const WideSets &T, cudaStream_t st) {
+int wide_build(SceneImpl &s, WideBufs &B, const WideSets &T, float largest, cudaStream_t st) {
   int const dev = s.device, n = s.n_tris;
   uint32_t const max_nodes = static_cast<uint32_t>(wide_max_nodes(n));
   WideCounters h{};
   h.nodes = 1;
   h.level[1] = 1;
   WideTask const root{0, 0, n};
-  XYZ_BUILD_TRY(cudaMemcpyAsync(B.counters.p, &h, sizeof(h), cudaMemcpyHostToDevice, st));
+  XYZ_BUILD_TRY(cudaMemcpyAsync(B.counters.p, &h, offsetof(WideCounters, extents), cudaMemcpyHostToDevice, st));
   XYZ_BUILD_TRY(cudaMemcpyAsync(B.task.p, &root, sizeof(root), cudaMemcpyHostToDevice, st));
   int const grid = grid_for(n / 8 + 1, kWideThreads, dev);
   int done = 0;
@@ -1284,6 +1294,9 @@ int wide_build(SceneImpl &s, WideBufs &B, const WideSets &T, cudaStream_t st) {
   s.n_wide = h.nodes;
   s.d_wide = out.release();
   s.d_wide_tri = B.tris.release();
+  f3 const half = scl3(sub3(s.dev.bmax, s.dev.bmin), 0.5f);
+  s.dev.wide_mid = add3(s.dev.bmin, half);
+  s.dev.wide_reach = wide_reach_of(std::max({half.x, half.y, half.z}), largest, h.extents, static_cast<uint32_t>(n));
   return XYZGPU_OK;
 }
 
@@ -1320,7 +1333,8 @@ int kd_layout_depth_first(SceneImpl &s, const std::vector<int64_t> &level_start,
     T = WideSets{B.lo.p, B.hi.p, B.first.p};
     XYZ_BUILD_TRY(cudaMemsetAsync(B.lo.p, 0xff, n * sizeof(uint4), st));
     XYZ_BUILD_TRY(cudaMemsetAsync(B.hi.p, 0, n * sizeof(uint4), st));
-    k_wide_assign<<<grid_for(nt, 256, dev), 256, 0, st>>>(s.d_tri, nt, s.d_nodes, T, B.owner.p);
+    XYZ_BUILD_TRY(cudaMemsetAsync(B.counters.p, 0, sizeof(WideCounters), st));
+    k_wide_assign<<<grid_for(nt, 256, dev), 256, 0, st>>>(s.d_tri, nt, s.d_nodes, T, B.owner.p, B.counters.p->extents);
   }
   int const levels = static_cast<int>(level_start.size()) - 1;
   TopLevels V{};
@@ -1338,9 +1352,8 @@ int kd_layout_depth_first(SceneImpl &s, const std::vector<int64_t> &level_start,
   k_layout_scatter<<<grid_for(n, 256, dev), 256, 0, st>>>(s.d_nodes, n, pos.p, base.p, out.p);
   XYZ_BUILD_TRY(cudaGetLastError());
   if (wide) {
-    int const rc = wide_build(s, B, T, st);
+    int const rc = wide_build(s, B, T, reach, st);
     if (rc) return rc;
-    s.dev.wide_reach = reach * kWideReach;
   }
   XYZ_BUILD_TRY(cudaFreeAsync(s.d_nodes, st));
   s.d_nodes = out.release();

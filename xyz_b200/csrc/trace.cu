@@ -43,7 +43,7 @@ XYZ_DEV bool kd_queue(const DevScene &S, const ApiSink &sink, int n) {
   f3 o, d;
   float tmin, tmax;
   sink.load(static_cast<int>(threadIdx.x & 31) * (n / 32), o, d, tmin, tmax);
-  return __all_sync(0xffffffffu, !S.wide || !wide_usable(o, d, S.wide_reach) || !(0.0f <= tmin && tmin <= tmax));
+  return __all_sync(0xffffffffu, !S.wide || !wide_usable(sub3(o, S.wide_mid), d, S.wide_reach) || !(0.0f <= tmin && tmin <= tmax));
 }
 
 // The kd-tree's kernel for such queues: the loop takes 9 CTAs per SM where the

@@ -378,7 +378,7 @@ XYZ_DEV void trace_wide(const DevScene &S, int n, int *fetch, Sink &sink, int32_
               h.back = 0;
               tlim = tmax;
               slack = 0.0f;
-              if (!SL.wide || !wide_usable(o, d, SL.wide_reach) || !(0.0f <= tmin && tmin <= tmax)) {
+              if (!SL.wide || !wide_usable(sub3(o, SL.wide_mid), d, SL.wide_reach) || !(0.0f <= tmin && tmin <= tmax)) {
                 retry = i;
               } else {
                 ray = i;

@@ -49,10 +49,12 @@ constexpr int kWideTriVec = 4;       // float4 per triangle record
 // from all over such a ground at the object's triangles, 10^4 to 10^5 times as long
 // as these, are close calls to the last one: 5,455 / 7,388 / 13,718 and 2,101 /
 // 2,965 / 5,588 (the kd loop 2,470 to 2,540, which is faster from 1,000 on).
-// Rays whose origin has a coordinate beyond kWideReach * S do not use the tree.
+// Rays from beyond kWideReach * S of the scene, or kWideFar times the median
+// triangle's extent (WideTri::e), do not use the tree (wide_reach).
 constexpr float kWideSlack = 1.0f / 524288.0f;
 constexpr float kWidePad = 1.0f / 8388608.0f;  // of S: for boxes whose corners are rounded to nearest
 constexpr float kWideReach = 65536.0f;
+constexpr float kWideFar = 16384.0f;
 
 // Triangle sets of the kd-tree's (breadth-first) nodes while the tree is built.
 struct WideSets {
@@ -178,6 +180,28 @@ struct WideTri {
   float lo[3], hi[3];
   float e, n;  // |e1| + |e2| and |n| + |e1||e2| (1-norms)
 };
+
+// Triangles by extent, four ranges to the octave: bucket of an extent, and the
+// least extent of a bucket.
+constexpr int kWideExtents = 1024;
+XYZ_HD int wide_extent_bucket(float e) { return static_cast<int>(wide_bits(e) >> 21) & (kWideExtents - 1); }
+inline float wide_extent_of(int bucket) { return wide_float(static_cast<uint32_t>(bucket) << 21); }
+
+// How far from the middle of a scene (half extent `half`, largest coordinate S, n
+// triangles counted by extent) rays may start to use the tree.  From further the
+// slack of wide_test, a share of the distance, reaches the size of the triangles:
+// nearly every hit is then a close call, and the triangle test's own error at a
+// slope below the 0.17 that the slack allows for exceeds it.  2^21 rays at the
+// triangles of a 1M-triangle mesh / an 80,000-triangle terrain / 6,000 triangles of
+// boxes from 2^12, 2^14, 2^16, 2^18 extents, us: 1,117 / 1,157 / 1,008, 1,405 / 1,429
+// / 1,338, 1,971 / 2,099 / 2,013, 4,971 / 6,266 / 4,804 by the wide tree, 1,730 / 1,320
+// / 905 by the kd-tree at any distance.
+inline float wide_reach_of(float half, float S, const uint32_t *extents, uint32_t n) {
+  uint32_t below = 0;
+  int b = 0;
+  while (b < kWideExtents - 1 && (below += extents[b]) <= n / 2) ++b;
+  return half + std::fmin(kWideReach * S, kWideFar * wide_extent_of(b));
+}
 
 constexpr float kWideGrow = 12.0f / 16777216.0f;
 
@@ -360,7 +384,7 @@ XYZ_HD WideRay wide_ray(f3 o, f3 d) {
   return r;
 }
 
-// Rays the tree answers: within the range of the box arithmetic, no component so
+// Rays the tree answers (o: from the scene's middle): within reach, no component so
 // small that its reciprocal is infinite: such a ray can lie in a split plane of
 // the kd-tree, whose distance is then not a number, and the kd loop's choice of
 // cells is its own.
