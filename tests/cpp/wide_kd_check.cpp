@@ -176,6 +176,8 @@ bool wide_loop(const Trees &B, f3 o, f3 d, float tmin, float tmax, RayHit &h, do
       int const id = B.record[w[7] + __builtin_popcount(valid & ((1u << __builtin_ctz(th)) - 1u))];
       float t, f, g, det, m, dt;
       *tests += 1;
+      if (wide_parallel(dot3(d, mk3(B.tri[3 * id].w, B.tri[3 * id + 1].w, B.tri[3 * id + 2].w)), B.lengths[id].parallel))
+        return false;
       if (!test_triangle(B.tri[3 * id], B.tri[3 * id + 1], B.tri[3 * id + 2], o, d, tmin, tlim, &t, &f, &g, &det))
         continue;
       wide_margin(t, norm1(d), B.lengths[id].e, B.lengths[id].n, reciprocal(det), &m, &dt);
@@ -207,9 +209,10 @@ void terrain(std::vector<f3> &v, int m, float at) {
 }  // namespace
 
 // scenes: sliver:WIDTH (200 long thin triangles), soup:SIZE, terrain:OFFSET, grid:SIDE (a terrain of so many squares
-// a side), ground:HALF (a terrain patch above a ground that wide), boxes
+// a side), ground:HALF (a terrain patch above a ground that wide), boxes, turned (the boxes 30 times as large, about
+// a slanted axis)
 // kinds: edge (rays at a point 1e-7 to 1e-1 of a triangle inside or beyond one of its edges, from near and far),
-// far (the same from 10 to 30,000 scene sizes), local (rays between two points of the scene's finely divided part)
+// plane (rays between two points of a box's face), far (the same as edge, from 10 to 30,000 scene sizes), local (rays between two points of the scene's finely divided part)
 int main(int argc, char **argv) {
   if (argc != 4) return 1;
   std::string const scene = argv[1], kind = argv[3];
@@ -246,6 +249,12 @@ int main(int argc, char **argv) {
         quad(v, P(q[0]), P(q[1]), P(q[2]), P(q[3]));
     }
   }
+  if (scene == "turned")
+    for (f3 &p : v) {
+      f3 const a = unit(mk3(1.0f, 2.0f, 3.0f)), q = scl3(p, 30.0f);  // Rodrigues' rotation by 0.7
+      p = add3(add3(scl3(q, std::cos(0.7f)), scl3(cross3(a, q), std::sin(0.7f))),
+               scl3(a, dot3(a, q) * (1.0f - std::cos(0.7f))));
+    }
   Trees B;
   if (!build(v, B)) return 1;
   int const fine = static_cast<int>(v.size() / 3) - (scene.rfind("ground", 0) == 0 ? 2 : 0);
@@ -266,6 +275,10 @@ int main(int argc, char **argv) {
       f3 const e = add3(a, scl3(sub3(b, a), 0.5f + 0.5f * U(g)));
       d = unit(mk3(N(g), N(g), N(g)));
       o = sub3(add3(e, scl3(sub3(e, c), past)), scl3(d, size * std::pow(10.0f, kind == "far" ? 2.75f + 1.75f * U(g) : -0.5f + U(g))));
+    } else if (kind == "plane") {
+      float const a = 0.5f + 0.5f * U(g), b = (0.5f + 0.5f * U(g)) * (1 - a), c = 0.5f + 0.5f * U(g);
+      o = point(i, a, b);
+      d = unit(sub3(point(i ^ 1, c, (0.5f + 0.5f * U(g)) * (1 - c)), o));
     } else {
       float const a = 0.5f + 0.5f * U(g), b = (0.5f + 0.5f * U(g)) * (1 - a);
       o = add3(point(static_cast<int>(g() % fine), 0.3f, 0.3f), mk3(0, 0.3f + 0.2f * U(g), 0));

@@ -31,6 +31,14 @@ def test_answers_beside_edges(check, scene):
     assert differ == 0
 
 
+def test_answers_in_the_planes_of_triangles(check):
+    """Rays between two points of a face of a box, large enough that rounding keeps
+    the determinant above the triangle test's limit: what the test then accepts
+    are the triangles that the kd loop's cells hold."""
+    rays, hits, _, differ = check("turned", 200000, "plane")[:4]
+    assert hits > rays / 2 and differ == 0
+
+
 def scene_of(pos):
     """A scene of loose triangles, the last of them a light."""
     from xyz_b200 import scenes

@@ -1069,7 +1069,7 @@ __global__ void k_wide_tris(const float4 *__restrict__ tri, int n, WideSets T, c
     out[rec + 1] = b;
     out[rec + 2] = c;
     WideTri const w = wide_triangle(xyz3(a), xyz3(b), xyz3(c), mk3(a.w, b.w, c.w));
-    out[rec + 3] = make_float4(__int_as_float(i), w.e, w.n, 0.0f);
+    out[rec + 3] = make_float4(__int_as_float(i), w.e, w.n, w.parallel);
   }
 }
 
