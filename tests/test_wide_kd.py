@@ -218,3 +218,15 @@ def test_far_rays_hit_as_in_the_kd_tree(side):
     rays[:, 0:3] = (rng.dirichlet([1, 1, 1], n)[..., None] * t).sum(1) - d * 2.0 * 10.0 ** rng.uniform(1, 4, (n, 1))
     rays[:, 3], rays[:, 4:7], rays[:, 7] = 1e-5, d, np.inf
     assert compare(scene_of(pos), rays) > 1 << 19
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("extra", [-1, 0, 1])
+@pytest.mark.parametrize("triangles", [64, 65])
+def test_queues_of_tiny_scenes(triangles, extra):
+    """Queues around the size from which scenes of up to 64 triangles take the
+    kd-tree's kernel, and scenes around that number."""
+    import torch
+    pos = slivers(0.3, n=triangles).astype(np.float32)
+    n = 9 * 128 * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    assert compare(scene_of(pos), edge_rays(pos, n, 10)) > n // 8

@@ -58,6 +58,16 @@ __global__ void __launch_bounds__(kTraceThreads, 9)
   trace_persistent<false>(S, n, fetch, sink, c);
 }
 
+// Scenes of a few triangles in a closed room: the walls' boxes overlap in the
+// corners and a ray tests most of the triangles, where the kd-tree's cells divide
+// them.  Queues that fill the kd kernel's grid go to it: 2^21 rays of a 36-triangle
+// room, wide / kd, us: from the middle 300 / 247, from anywhere inside 226 / 193,
+// between two surface points 401 / 210, from outside 309 / 155; 4 M camera and
+// bounce rays 391 / 377; 262,144 rays 53 / 50, 49 / 47, 73 / 55, 59 / 43.  (Renders,
+// whose rays keep together, are 10 to 25 % faster by the wide tree; shorter queues
+// too.)
+constexpr int kKdTris = 64;
+
 template <bool kCount>
 __global__ void __launch_bounds__(kTraceThreads, kCount ? 9 : 8)
     k_trace_api(DevScene S, const float4 *__restrict__ rays, int n, float4 *__restrict__ hits,
@@ -123,13 +133,19 @@ int trace_api_launch(SceneImpl &s, const float *rays, int n, float *hits, cudaSt
     counters->hits = c[4];
   } else {
     static int wide_grid = 0, kd_grid = 0;
+    int const kd_full = grid_for(k_trace_kd, kd_grid, s.device);
+    if (s.n_tris <= kKdTris && n / kTraceThreads >= kd_full) {
+      k_trace_kd<<<kd_full, kTraceThreads, 0, st>>>(s.dev, r4, n, h4, s.d_fetch);
+      XYZ_CUDA_TRY(cudaGetLastError());
+      return XYZGPU_OK;
+    }
     int const full = grid_for(k_trace_api<false>, wide_grid, s.device);
     int const grid = std::min(full, ceil_div(n, kRaysPerCta));
     bool const kd_follows = n / (2 * kTraceThreads) >= full;
     k_trace_api<false><<<grid, kTraceThreads, 0, st>>>(s.dev, r4, n, h4, s.d_fetch, nullptr, kd_follows);
     XYZ_CUDA_TRY(cudaGetLastError());
     if (kd_follows) {
-      k_trace_kd<<<grid_for(k_trace_kd, kd_grid, s.device), kTraceThreads, 0, st>>>(s.dev, r4, n, h4, s.d_fetch);
+      k_trace_kd<<<kd_full, kTraceThreads, 0, st>>>(s.dev, r4, n, h4, s.d_fetch);
       XYZ_CUDA_TRY(cudaGetLastError());
     }
   }
