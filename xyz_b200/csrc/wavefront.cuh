@@ -583,9 +583,8 @@ struct ShadowSink {
 // counters, which no bounce uses.
 XYZ_DEV int32_t *wave_taken(const WaveArgs &A) { return A.counts + A.kmax * kCountStride; }
 
-// CTAs per SM: 8 (64 registers) for the wide tree, whose kernels spill up to 80
-// bytes a thread there (batched k_trace_both 112) and far more at 10 (+45 % on the
-// 1M-triangle scene); counted renders, on the kd-tree, run at 9 (extension rays, 56
+// CTAs per SM: 8 (64 registers) for the wide tree, whose kernels spill up to 96
+// bytes a thread there and far more at 10 (+45 % on the 1M-triangle scene); counted renders, on the kd-tree, run at 9 (extension rays, 56
 // registers) and 10 (shadow rays, 48 and 124 bytes).  The kernels hold the stacks
 // of both walks, 512 and 480 bytes.
 template <bool kShadow, bool kCount, int kMode = kModePlain>
