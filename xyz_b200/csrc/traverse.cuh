@@ -266,7 +266,7 @@ XYZ_DEV void trace_persistent(const DevScene &S, int n, int *fetch, Sink &sink, 
 // loads and 15 triangle tests, at 8 of 32 lanes and 351 warp instructions a ray (the
 // second bounce of a render); a wide node costs one round of uniform arithmetic on
 // eight boxes for three 32-byte loads, and the ray needs eight of them and five
-// tests, at 17 lanes and 174 instructions.
+// tests, at 17 lanes and 173 instructions.
 constexpr int kWideRetry = 128;  // list entries per warp; 64 + one refill + the lanes under way fit
 constexpr int kWideRetryFull = 64;
 
