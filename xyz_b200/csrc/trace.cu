@@ -1,8 +1,9 @@
 // Closest-hit entry point (xyzgpu_trace_closest): the batch form of
 // Scene::FindIntersection (xyz/core/scene.hpp:277-295).
 //
-// Persistent warps with per-lane refill (trace_wide in traverse.cuh; counting
-// calls and queues of axis-parallel rays walk the kd-tree with trace_persistent):
+// Persistent warps with per-lane refill (trace_wide in traverse.cuh; counting calls
+// and long queues of axis-parallel rays or of tiny scenes walk the kd-tree with
+// trace_persistent):
 // rays are taken from a global counter as lanes free up, so long and short rays
 // balance across lanes and SMs.  Rays are read as two 16-byte vectors and hits
 // written as one.
